@@ -2366,7 +2366,8 @@ struct pbf_ns {
   bool own_stream;
   std::string err;
   DBuf<uint32_t> key, rank, cell_count, cell_start, perm_raw, id_raw, perm, tmp_a, tmp_b, big_list, big_count, err_word;
-  DBuf<uint32_t> nbr_count;
+  DBuf<uint32_t> nbr_count;  // by particle id (pbf_ns_lists)
+  DBuf<float4> sorted;       // pbf_ns_lists: positions in sorted order, the id in w
   void* scan_scratch = nullptr;
   void* radix_scratch = nullptr;  // histograms and look-back words of the radix passes
   // pbf_ns_set_timing: events at the phase boundaries of pbf_ns_run
@@ -2385,9 +2386,6 @@ int nsfail(pbf_ns* s, int code, const char* msg) {
     if (e_ != cudaSuccess) return nsfail((s), PBF_ECUDA, cudaGetErrorString(e_)); \
   } while (0)
 
-// NeighborCount / NeighborList over positions in id order: reuse the fast
-// pass kernels with the stand-alone radius (distance test only, no float
-// arithmetic beyond d.d, identical in both variants).
 }  // namespace
 
 extern "C" {
@@ -2458,6 +2456,7 @@ int pbf_ns_destroy(pbf_ns* s) {
   DBuf<uint32_t>* bufs[] = {&s->key,   &s->rank,  &s->cell_count, &s->cell_start, &s->perm_raw, &s->id_raw, &s->perm,
                             &s->tmp_a, &s->tmp_b, &s->big_list,   &s->big_count,  &s->err_word, &s->nbr_count};
   for (auto* b : bufs) b->release();
+  s->sorted.release();
   if (s->scan_scratch) cudaFree(s->scan_scratch);
   if (s->radix_scratch) cudaFree(s->radix_scratch);
   for (cudaEvent_t& e : s->ev)
@@ -2528,58 +2527,21 @@ int pbf_ns_lists(pbf_ns* s, const float* d_pos4, uint32_t n, float radius, uint3
   if (!s || !d_nbr_offset || (!d_pos4 && n)) return PBF_EINVAL;
   if (n > s->max_n) return nsfail(s, PBF_ECAPACITY, "too many particles for this search context");
   cudaStream_t st = s->stream;
-  // The pass kernels traverse particles in cell-sorted order; gather the
-  // positions into that order (tmp buffers reinterpreted as float4 need 4x
-  // room, so use a temporary allocation).
-  float4* sorted = nullptr;
-  uint32_t* sorted_list = nullptr;
-  uint32_t* ids = nullptr;
-  NSCU(s, cudaMallocAsync((void**)&sorted, ((size_t)n + 1) * sizeof(float4), st));
-  NSCU(s, cudaMallocAsync((void**)&ids, ((size_t)n + 1) * 4, st));
-  SimParams p{};
-  p.h = radius;
-  p.h2 = (float)((double)radius * (double)radius);
-  p.n = n;
-  PassTable tbl;
-  exact::fill_pass_table(&tbl);
-  NSCU(s, launch_gather_state(n, s->perm.p, (const float4*)d_pos4, (const float4*)d_pos4, nullptr, sorted, sorted,
-                              ids, st));
-  tbl.nbr_count<<<nblocks(n + 1, 256), 256, 0, st>>>(p, s->g, sorted, s->cell_start.p, s->nbr_count.p);
-  NSCU(s, cudaGetLastError());
-  // counts are in slot order; the reference's offsets are by particle id
-  uint32_t* cnt_by_id = nullptr;
-  NSCU(s, cudaMallocAsync((void**)&cnt_by_id, ((size_t)n + 1) * 4, st));
-  NSCU(s, cudaMemsetAsync(cnt_by_id, 0, ((size_t)n + 1) * 4, st));
-  NSCU(s, launch_scatter_by_id_u32(n, ids, s->nbr_count.p, cnt_by_id, st));
-  NSCU(s, launch_exclusive_scan(cnt_by_id, d_nbr_offset, (size_t)n + 1, s->scan_scratch, s->err_word.p, st));
-  // slot-order offsets for the list kernel
-  uint32_t* slot_off = nullptr;
-  NSCU(s, cudaMallocAsync((void**)&slot_off, ((size_t)n + 1) * 4, st));
-  NSCU(s, launch_exclusive_scan(s->nbr_count.p, slot_off, (size_t)n + 1, s->scan_scratch, s->err_word.p, st));
+  // the sorted positions' workspace: allocated by the first call, kept with the context
+  if (!s->sorted.p) NSCU(s, s->sorted.alloc(s->max_n));
+  const float h2 = (float)((double)radius * (double)radius);
+  NSCU(s, launch_ns_count(n, s->g, h2, s->perm.p, (const float4*)d_pos4, s->cell_start.p, s->sorted.p, s->nbr_count.p,
+                          st));
+  NSCU(s, launch_exclusive_scan(s->nbr_count.p, d_nbr_offset, (size_t)n + 1, s->scan_scratch, s->err_word.p, st));
   uint32_t tot = 0;
-  NSCU(s, cudaMemcpyAsync(&tot, slot_off + n, 4, cudaMemcpyDeviceToHost, st));
+  NSCU(s, cudaMemcpyAsync(&tot, d_nbr_offset + n, 4, cudaMemcpyDeviceToHost, st));
+  // the kernel itself compares the total with the capacity, so it is queued before the host knows
+  if (d_nbr_list)
+    NSCU(s, launch_ns_list(n, s->g, h2, s->sorted.p, s->cell_start.p, d_nbr_offset, d_nbr_list, capacity, st));
   NSCU(s, cudaStreamSynchronize(st));
   if (total) *total = tot;
-  int rc = PBF_OK;
-  if (tot > capacity) {
-    rc = nsfail(s, PBF_ECAPACITY, "neighbour lists exceed capacity");
-  } else if (tot && d_nbr_list) {
-    NSCU(s, cudaMallocAsync((void**)&sorted_list, (size_t)tot * 4, st));
-    tbl.nbr_list<<<nblocks(n, 256), 256, 0, st>>>(p, s->g, sorted, s->cell_start.p, slot_off, sorted_list, tot,
-                                                   s->err_word.p);
-    NSCU(s, cudaGetLastError());
-    // translate slot ids to particle ids, then move each particle's run to its id-order offset
-    NSCU(s, launch_list_to_ids(tot, sorted_list, ids, sorted_list, st));
-    // move each particle's run from its slot-order offset to its id-order offset
-    NSCU(s, launch_copy_runs(n, slot_off, d_nbr_offset, ids, sorted_list, d_nbr_list, st));
-    NSCU(s, cudaFreeAsync(sorted_list, st));
-  }
-  NSCU(s, cudaFreeAsync(slot_off, st));
-  NSCU(s, cudaFreeAsync(cnt_by_id, st));
-  NSCU(s, cudaFreeAsync(sorted, st));
-  NSCU(s, cudaFreeAsync(ids, st));
-  NSCU(s, cudaStreamSynchronize(st));
-  return rc;
+  if (tot > capacity) return nsfail(s, PBF_ECAPACITY, "neighbour lists exceed capacity");
+  return PBF_OK;
 }
 
 int pbf_ns_sync(pbf_ns* s) {

@@ -199,6 +199,57 @@ __device__ __forceinline__ uint32_t cell_key(int cx, int cy, int cz, const GridP
          (uint32_t)cz;
 }
 
+// |d|^2 with the reference's rounding (x*x + y*y, then + z*z, each product
+// and sum rounded once; no contraction in either compile mode) and the
+// neighbour test |d|^2 <= h^2 on it: every neighbour search of the library
+// and the CPU restatement then agree on the neighbour sets bit for bit.
+__device__ __forceinline__ float dist2_rn(f3 d) {
+  return __fadd_rn(__fadd_rn(__fmul_rn(d.x, d.x), __fmul_rn(d.y, d.y)), __fmul_rn(d.z, d.z));
+}
+
+// Range of slots covering cells (cx+dx, cy+dy, cz-Z .. cz+Z), Z = g.reach_z:
+// the neighbourhood is (2 g.reach + 1)^2 runs of consecutive keys because
+// keys are z-fastest (reach 1, Z = 1: the reference's 27 cells as 9 runs).
+struct Run {
+  uint32_t b, e;
+};
+__device__ __forceinline__ Run run_of(const GridParams& g, const uint32_t* __restrict__ cell_start, int cx, int cy,
+                                      int cz, int dx, int dy) {
+  int x = cx + dx, y = cy + dy;
+  if (x < 0 || y < 0 || x >= g.dim[0] || y >= g.dim[1]) return Run{0, 0};
+  int zlo = max(cz - g.reach_z, 0), zhi = min(cz + g.reach_z, g.dim[2] - 1);
+  uint32_t k0 = cell_key(x, y, zlo, g), k1 = cell_key(x, y, zhi, g) + 1u;
+  return Run{__ldg(cell_start + k0), __ldg(cell_start + k1)};
+}
+
+// Visits the candidates of the slot run [b, e) that lie within sqrt(h2) of
+// xi, in slot order: hit(u).  The run is tested in chunks of 32, four
+// candidates' loads in flight, into a bit mask without branches; only the
+// set bits are then visited, so a warp pays one short loop per chunk over the
+// hits of its fullest lane instead of a divergent branch per candidate.
+template <class Hit>
+__device__ __forceinline__ void visit_run(const float4* __restrict__ xs, uint32_t b, uint32_t e, f3 xi, float h2,
+                                          Hit&& hit) {
+  for (uint32_t u0 = b; u0 < e; u0 += 32u) {
+    const uint32_t cnt = min(e - u0, 32u);
+    unsigned mask = 0u;
+    for (uint32_t k = 0; k < cnt; k += 4u) {
+      float4 c[4];
+#pragma unroll
+      for (uint32_t m = 0; m < 4u; ++m) c[m] = __ldg(xs + min(u0 + k + m, e - 1u));
+#pragma unroll
+      for (uint32_t m = 0; m < 4u; ++m)
+        if (dist2_rn(xyz(c[m]) - xi) <= h2) mask |= 1u << (k + m);
+    }
+    if (cnt < 32u) mask &= (1u << cnt) - 1u;  // the last group repeats candidate e - 1
+    while (mask) {
+      const uint32_t k = (uint32_t)__ffs(mask) - 1u;
+      mask &= mask - 1u;
+      hit(u0 + k);
+    }
+  }
+}
+
 // ---- volume map (src/simulator/boundary/discreteFieldShader.ts:1-192) ---------------
 // 32-node cubic serendipity hexahedron.  Node order per cell: corners
 // (i,j,k),(i+1,j,k),(i,j+1,k),(i+1,j+1,k), then the same at k+1; x-edge nodes

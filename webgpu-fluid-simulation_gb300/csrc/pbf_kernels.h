@@ -65,10 +65,6 @@ struct CbSet {
 };
 
 struct PassTable {
-  // the stand-alone neighbour search (reference list layout)
-  void (*nbr_count)(SimParams, GridParams, const float4*, const uint32_t*, uint32_t*);
-  void (*nbr_list)(SimParams, GridParams, const float4*, const uint32_t*, const uint32_t*, uint32_t*, uint32_t,
-                   uint32_t*);
   PassSet set[2][2];  // [batch][persistent]
   void (*fallback)(FallbackArgs);  // cooperative launch only
   // cell-block passes: the search (masks; with the learned start's features)
@@ -160,11 +156,14 @@ cudaError_t launch_scatter_by_id(uint32_t n, const uint32_t* id, const float4* s
 cudaError_t launch_scatter_w_by_id(uint32_t n, const uint32_t* id, const float4* src, float* dst, cudaStream_t st);
 cudaError_t launch_scatter_by_id_u32(uint32_t n, const uint32_t* id, const uint32_t* src, uint32_t* dst,
                                      cudaStream_t st);
-cudaError_t launch_list_to_ids(uint32_t total, const uint32_t* list, const uint32_t* id, uint32_t* out,
-                               cudaStream_t st);
-// dst[id_off[ids[t]] + q] = src[slot_off[t] + q] for each slot t's run.
-cudaError_t launch_copy_runs(uint32_t n, const uint32_t* slot_off, const uint32_t* id_off, const uint32_t* ids,
-                             const uint32_t* src, uint32_t* dst, cudaStream_t st);
+// Neighbour lists of the stand-alone search (27 cells, |d|^2 <= h2): sorted[t]
+// = (position, id) of order[t] and the neighbour count by particle id (n + 1
+// entries, the last 0); then the lists of neighbour ids at offset[id], the
+// exclusive scan of those counts, written only if offset[n] <= capacity.
+cudaError_t launch_ns_count(uint32_t n, const GridParams& g, float h2, const uint32_t* order, const float4* pos,
+                            const uint32_t* cell_start, float4* sorted, uint32_t* count, cudaStream_t st);
+cudaError_t launch_ns_list(uint32_t n, const GridParams& g, float h2, const float4* sorted, const uint32_t* cell_start,
+                           const uint32_t* offset, uint32_t* list, uint32_t capacity, cudaStream_t st);
 
 // Metrics (max / mean density error, kinetic energy, non-finite and penetration counts).
 struct MetricsAccum {

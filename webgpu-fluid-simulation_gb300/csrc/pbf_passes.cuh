@@ -8,7 +8,7 @@
 // Reference passes restated here (paths relative to the reference root):
 //   predict + key + count  TimeIntegration (src/simulator/PBF/shader/timeIntegration.ts:20-32)
 //                          + ParticleInsert (src/simulator/neighbor/neighborShader.ts:24-32)
-//   nbr_count / nbr_list   NeighborCount / NeighborList (neighborShader.ts:101-246)
+//   nbr_build              NeighborCount / NeighborList (neighborShader.ts:101-246)
 //   lambda                 BoundaryVolume (boundaryVolume.ts:26-57) + LambdaCalculation
 //                          (src/simulator/PBF/shader/pressureConstrain.ts:31-85)
 //   deltap                 ConstrainSolve + ConstrainApply (pressureConstrain.ts:109-179)
@@ -119,54 +119,8 @@ __global__ void __launch_bounds__(256) k_predict(SimParams p0, GridParams g0, Sc
   }
 }
 
-// |d|^2 with the reference's rounding (x*x + y*y, then + z*z, each product
-// and sum rounded once; no contraction in either compile mode) and the
-// neighbour test |d|^2 <= h^2 on it: every neighbour search of the library
-// and the CPU restatement then agree on the neighbour sets bit for bit.
-__device__ __forceinline__ float dist2_rn(f3 d) {
-  return __fadd_rn(__fadd_rn(__fmul_rn(d.x, d.x), __fmul_rn(d.y, d.y)), __fmul_rn(d.z, d.z));
-}
+// The neighbour test |d|^2 <= h^2 (dist2_rn).
 __device__ __forceinline__ bool within_h(const SimParams& p, f3 d) { return dist2_rn(d) <= p.h2; }
-
-// Range of slots covering cells (cx+dx, cy+dy, cz-Z .. cz+Z), Z = g.reach_z:
-// the neighbourhood is (2 g.reach + 1)^2 runs of consecutive keys because
-// keys are z-fastest (reach 1, Z = 1: the reference's 27 cells as 9 runs).
-struct Run {
-  uint32_t b, e;
-};
-__device__ __forceinline__ Run run_of(const GridParams& g, const uint32_t* __restrict__ cell_start, int cx, int cy,
-                                      int cz, int dx, int dy) {
-  int x = cx + dx, y = cy + dy;
-  if (x < 0 || y < 0 || x >= g.dim[0] || y >= g.dim[1]) return Run{0, 0};
-  int zlo = max(cz - g.reach_z, 0), zhi = min(cz + g.reach_z, g.dim[2] - 1);
-  uint32_t k0 = cell_key(x, y, zlo, g), k1 = cell_key(x, y, zhi, g) + 1u;
-  return Run{__ldg(cell_start + k0), __ldg(cell_start + k1)};
-}
-
-// NeighborCount: neighbours within h of x*, self included, 27 cells in key
-// order (stand-alone search; slot n receives 0 so a scan of n + 1 counts
-// ends in the total).
-__global__ void __launch_bounds__(256) k_nbr_count(SimParams p, GridParams g, const float4* __restrict__ xs,
-                                                   const uint32_t* __restrict__ cell_start,
-                                                   uint32_t* __restrict__ nbr_count) {
-  uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t cnt = 0;
-  if (t < p.n) {
-    f3 xi = xyz(xs[t]);
-    int cx = cell_axis(xi.x, g.origin[0], g.inv_cell[0], g.dim[0]);
-    int cy = cell_axis(xi.y, g.origin[1], g.inv_cell[1], g.dim[1]);
-    int cz = cell_axis(xi.z, g.origin[2], g.inv_cell[2], g.dim[2]);
-    for (int dx = -1; dx <= 1; ++dx)
-      for (int dy = -1; dy <= 1; ++dy) {
-        Run r = run_of(g, cell_start, cx, cy, cz, dx, dy);
-        for (uint32_t u = r.b; u < r.e; ++u) {
-          f3 d = xyz(__ldg(xs + u)) - xi;
-          if (within_h(p, d)) ++cnt;
-        }
-      }
-  }
-  if (t <= p.n) nbr_count[t] = cnt;
-}
 
 // Velocity divergence feature of the learned start, -div(v') dt, by the
 // continuity equation: (rho_prev - rho*) / rho* with rho* the fluid density
@@ -480,32 +434,6 @@ __global__ void __launch_bounds__(256) k_nbr_build_warp(SimParams p, GridParams 
       }
     }
   }
-}
-
-// NeighborList: the same traversal writing slot indices at nbr_offset[t].
-__global__ void __launch_bounds__(256) k_nbr_list(SimParams p, GridParams g, const float4* __restrict__ xs,
-                                                  const uint32_t* __restrict__ cell_start,
-                                                  const uint32_t* __restrict__ nbr_offset, uint32_t* __restrict__ nbr_list,
-                                                  uint32_t capacity, uint32_t* err) {
-  uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= p.n) return;
-  if (t == 0 && nbr_offset[p.n] > capacity) atomicOr(err, 0x1u);
-  f3 xi = xyz(xs[t]);
-  int cx = cell_axis(xi.x, g.origin[0], g.inv_cell[0], g.dim[0]);
-  int cy = cell_axis(xi.y, g.origin[1], g.inv_cell[1], g.dim[1]);
-  int cz = cell_axis(xi.z, g.origin[2], g.inv_cell[2], g.dim[2]);
-  uint32_t o = nbr_offset[t];
-  for (int dx = -1; dx <= 1; ++dx)
-    for (int dy = -1; dy <= 1; ++dy) {
-      Run r = run_of(g, cell_start, cx, cy, cz, dx, dy);
-      for (uint32_t u = r.b; u < r.e; ++u) {
-        f3 d = xyz(__ldg(xs + u)) - xi;
-        if (within_h(p, d)) {
-          if (o < capacity) nbr_list[o] = u;
-          ++o;
-        }
-      }
-    }
 }
 
 // Loads of per-particle records.  kC = false: the read-only path (the record
@@ -1275,8 +1203,6 @@ void fill_set(PassSet* ps) {
 
 void fill_pass_table(PassTable* tbl) {
   tbl->fallback = k_fallback_solve;
-  tbl->nbr_count = k_nbr_count;
-  tbl->nbr_list = k_nbr_list;
   fill_set<false, false>(&tbl->set[0][0]);
   fill_set<false, true>(&tbl->set[0][1]);
   fill_set<true, false>(&tbl->set[1][0]);

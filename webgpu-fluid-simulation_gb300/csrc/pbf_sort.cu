@@ -553,19 +553,84 @@ __global__ void k_scatter_u32(uint32_t n, const uint32_t* __restrict__ id, const
   if (t >= n) return;
   dst[id[t]] = src[t];
 }
-__global__ void k_list_to_ids(uint32_t total, const uint32_t* __restrict__ list, const uint32_t* __restrict__ id,
-                              uint32_t* __restrict__ out) {
-  uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= total) return;
-  out[q] = id[list[q]];
-}
-__global__ void k_copy_runs(uint32_t n, const uint32_t* __restrict__ slot_off, const uint32_t* __restrict__ id_off,
-                            const uint32_t* __restrict__ ids, const uint32_t* __restrict__ src, uint32_t* __restrict__ dst) {
-  uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+// ---- neighbour lists in the reference layout (stand-alone search) -------------------
+// NeighborCount + NeighborList (neighborShader.ts:101-246) in two traversals
+// of the 27 cells.  The positions go into sorted order once, each with its
+// particle id in w, so the traversals read coalesced candidates and the list
+// kernel has a neighbour's id at hand.
+__global__ void __launch_bounds__(256) k_ns_sorted(uint32_t n, const uint32_t* __restrict__ order,
+                                                   const float4* __restrict__ pos, float4* __restrict__ sorted) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
-  uint32_t b = slot_off[t], e = slot_off[t + 1], o = id_off[ids[t]];
-  for (uint32_t q = b; q < e; ++q) dst[o + (q - b)] = src[q];
+  const uint32_t o = order[t];
+  float4 x = __ldg(pos + o);
+  x.w = __uint_as_float(o);
+  sorted[t] = x;
 }
+
+template <class Hit>
+__device__ __forceinline__ void visit_cells27(const GridParams& g, const uint32_t* __restrict__ cell_start,
+                                              const float4* __restrict__ sorted, f3 xi, float h2, Hit&& hit) {
+  const int cx = cell_axis(xi.x, g.origin[0], g.inv_cell[0], g.dim[0]);
+  const int cy = cell_axis(xi.y, g.origin[1], g.inv_cell[1], g.dim[1]);
+  const int cz = cell_axis(xi.z, g.origin[2], g.inv_cell[2], g.dim[2]);
+  for (int dx = -1; dx <= 1; ++dx)
+    for (int dy = -1; dy <= 1; ++dy) {
+      const Run r = run_of(g, cell_start, cx, cy, cz, dx, dy);
+      visit_run(sorted, r.b, r.e, xi, h2, hit);
+    }
+}
+
+// Counts by particle id; entry n receives 0, so a scan of n + 1 ends in the total.
+__global__ void __launch_bounds__(128) k_ns_count(uint32_t n, GridParams g, float h2,
+                                                  const float4* __restrict__ sorted,
+                                                  const uint32_t* __restrict__ cell_start,
+                                                  uint32_t* __restrict__ count) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == n) count[n] = 0u;
+  if (t >= n) return;
+  const float4 x = sorted[t];
+  uint32_t c = 0;
+  visit_cells27(g, cell_start, sorted, xyz(x), h2, [&](uint32_t) { ++c; });
+  count[__float_as_uint(x.w)] = c;
+}
+
+// The lists, written only if they all fit (offset[n] <= capacity).  A thread
+// finds one particle's neighbours; its warp keeps the first kListRows of each
+// lane in shared memory (row q, lane l at 33 q + l: both sides free of bank
+// conflicts) and then writes each particle's run with all lanes, coalesced.
+// Neighbours past kListRows go straight to global memory.
+constexpr uint32_t kListRows = 48;
+constexpr uint32_t kListWarps = 4;
+__global__ void __launch_bounds__(32 * kListWarps) k_ns_list(uint32_t n, GridParams g, float h2,
+                                                             const float4* __restrict__ sorted,
+                                                             const uint32_t* __restrict__ cell_start,
+                                                             const uint32_t* __restrict__ offset,
+                                                             uint32_t* __restrict__ list, uint32_t capacity) {
+  __shared__ uint32_t s_rows[kListWarps][kListRows * 33u];
+  if (__ldg(offset + n) > capacity) return;
+  const uint32_t lane = threadIdx.x & 31u, t = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t* rows = s_rows[threadIdx.x >> 5];
+  uint32_t q = 0, at = 0;
+  if (t < n) {
+    const float4 x = sorted[t];
+    at = __ldg(offset + __float_as_uint(x.w));
+    visit_cells27(g, cell_start, sorted, xyz(x), h2, [&](uint32_t u) {
+      const uint32_t id = __float_as_uint(__ldg(&sorted[u].w));
+      if (q < kListRows)
+        rows[33u * q + lane] = id;
+      else
+        list[at + q] = id;
+      ++q;
+    });
+  }
+  __syncwarp();
+  for (int p = 0; p < 32; ++p) {
+    const uint32_t cnt = min(__shfl_sync(kFull, q, p), kListRows), to = __shfl_sync(kFull, at, p);
+    for (uint32_t r = lane; r < cnt; r += 32u) list[to + r] = rows[33u * r + (uint32_t)p];
+  }
+}
+
 // ---- metrics --------------------------------------------------------------------------
 __device__ __forceinline__ void atomic_max_pos_float(float* addr, float v) {
   // v >= 0: the int ordering of non-negative floats matches their value ordering
@@ -822,16 +887,17 @@ cudaError_t launch_scatter_by_id_u32(uint32_t n, const uint32_t* id, const uint3
   k_scatter_u32<<<blocks_for(n, 256), 256, 0, st>>>(n, id, src, dst);
   return cudaGetLastError();
 }
-cudaError_t launch_list_to_ids(uint32_t total, const uint32_t* list, const uint32_t* id, uint32_t* out,
-                               cudaStream_t st) {
-  if (total == 0) return cudaSuccess;
-  k_list_to_ids<<<blocks_for(total, 256), 256, 0, st>>>(total, list, id, out);
+cudaError_t launch_ns_count(uint32_t n, const GridParams& g, float h2, const uint32_t* order, const float4* pos,
+                            const uint32_t* cell_start, float4* sorted, uint32_t* count, cudaStream_t st) {
+  if (n) k_ns_sorted<<<blocks_for(n, 256), 256, 0, st>>>(n, order, pos, sorted);
+  k_ns_count<<<blocks_for((size_t)n + 1, 128), 128, 0, st>>>(n, g, h2, sorted, cell_start, count);
   return cudaGetLastError();
 }
-cudaError_t launch_copy_runs(uint32_t n, const uint32_t* slot_off, const uint32_t* id_off, const uint32_t* ids,
-                             const uint32_t* src, uint32_t* dst, cudaStream_t st) {
+cudaError_t launch_ns_list(uint32_t n, const GridParams& g, float h2, const float4* sorted, const uint32_t* cell_start,
+                           const uint32_t* offset, uint32_t* list, uint32_t capacity, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_copy_runs<<<blocks_for(n, 256), 256, 0, st>>>(n, slot_off, id_off, ids, src, dst);
+  k_ns_list<<<blocks_for(n, 32 * kListWarps), 32 * kListWarps, 0, st>>>(n, g, h2, sorted, cell_start, offset, list,
+                                                                       capacity);
   return cudaGetLastError();
 }
 cudaError_t launch_metrics(SimParams p, FieldParams f, const float* sdf, const float4* pos, const float4* vel,
