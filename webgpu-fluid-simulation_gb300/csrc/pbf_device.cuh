@@ -222,31 +222,57 @@ __device__ __forceinline__ Run run_of(const GridParams& g, const uint32_t* __res
   return Run{__ldg(cell_start + k0), __ldg(cell_start + k1)};
 }
 
-// Visits the candidates of the slot run [b, e) that lie within sqrt(h2) of
-// xi, in slot order: hit(u).  The run is tested in chunks of 32, four
-// candidates' loads in flight, into a bit mask without branches; only the
-// set bits are then visited, so a warp pays one short loop per chunk over the
-// hits of its fullest lane instead of a divergent branch per candidate.
-template <class Hit>
-__device__ __forceinline__ void visit_run(const float4* __restrict__ xs, uint32_t b, uint32_t e, f3 xi, float h2,
-                                          Hit&& hit) {
+// Tests the candidates of the slot run [b, e) against |x_j - xi|^2 <= h2 in
+// chunks of 32, in slot order: hits(u0, mask) gets each chunk's first slot and
+// its hit bits.  The loop holds nothing but the test: eight loads in flight at
+// constant offsets, the x and y terms as packed f32x2 operations (each lane
+// rounds like the scalar one: the squared distance is dist2_rn's bit for bit)
+// and no branch; a warp then visits the set bits, a few per chunk, instead of
+// taking a divergent branch at most candidates.  Groups of eight read up to
+// seven records past e (their bits are cleared), so the searched arrays carry
+// kRunPad records of padding.
+// each(r2, in): every candidate's squared distance and whether it is a hit,
+// for a caller that sums over the hits in order (kEach).
+constexpr uint32_t kRunGroup = 8;
+constexpr uint32_t kRunPad = kRunGroup - 1;
+template <bool kEach = false, class Hits, class Each>
+__device__ __forceinline__ void test_run(const float4* __restrict__ xs, uint32_t b, uint32_t e, f3 xi, float h2,
+                                         Hits&& hits, Each&& each) {
+  const float2 nxy = make_float2(-xi.x, -xi.y);
   for (uint32_t u0 = b; u0 < e; u0 += 32u) {
     const uint32_t cnt = min(e - u0, 32u);
     unsigned mask = 0u;
-    for (uint32_t k = 0; k < cnt; k += 4u) {
-      float4 c[4];
+    const float4* c = xs + u0;
+    for (uint32_t k = 0; k < cnt; k += kRunGroup, c += kRunGroup) {
+      float4 v[kRunGroup];
 #pragma unroll
-      for (uint32_t m = 0; m < 4u; ++m) c[m] = __ldg(xs + min(u0 + k + m, e - 1u));
+      for (int m = 0; m < (int)kRunGroup; ++m) v[m] = __ldg(c + m);
+      unsigned group = 0u;
 #pragma unroll
-      for (uint32_t m = 0; m < 4u; ++m)
-        if (dist2_rn(xyz(c[m]) - xi) <= h2) mask |= 1u << (k + m);
+      for (int m = 0; m < (int)kRunGroup; ++m) {
+        const float2 d = __fadd2_rn(make_float2(v[m].x, v[m].y), nxy), s = __fmul2_rn(d, d);
+        const float dz = __fsub_rn(v[m].z, xi.z);
+        const float r2 = __fadd_rn(__fadd_rn(s.x, s.y), __fmul_rn(dz, dz));
+        if (r2 <= h2) group |= 1u << m;
+        if constexpr (kEach) each(r2, r2 <= h2 && k + (uint32_t)m < cnt);
+      }
+      mask |= group << k;
     }
-    if (cnt < 32u) mask &= (1u << cnt) - 1u;  // the last group repeats candidate e - 1
-    while (mask) {
-      const uint32_t k = (uint32_t)__ffs(mask) - 1u;
-      mask &= mask - 1u;
-      hit(u0 + k);
-    }
+    hits(u0, mask & (0xffffffffu >> (32u - cnt)));
+  }
+}
+template <class Hits>
+__device__ __forceinline__ void test_run(const float4* __restrict__ xs, uint32_t b, uint32_t e, f3 xi, float h2,
+                                         Hits&& hits) {
+  test_run<false>(xs, b, e, xi, h2, hits, [](float, bool) {});
+}
+// hit(u) for each set bit of a chunk's mask, in slot order.
+template <class Hit>
+__device__ __forceinline__ void for_each_hit(uint32_t u0, unsigned mask, Hit&& hit) {
+  while (mask) {
+    const uint32_t k = (uint32_t)__ffs(mask) - 1u;
+    mask &= mask - 1u;
+    hit(u0 + k);
   }
 }
 

@@ -139,6 +139,7 @@ __device__ __forceinline__ float divergence_feature(const SimParams& p, float4 x
 // the true count; a count above max_nbr flags an overflow (the entries past
 // the slice are dropped and max_seen records the largest count for growing).
 // Runs are visited in key order, so entries come in increasing slot order.
+// One thread per slot; candidates are tested in masked chunks (test_run).
 template <bool kBatch, bool kLoop>
 __global__ void __launch_bounds__(256) k_nbr_build(SimParams p, GridParams g0, SceneTab tab,
                                                    const float4* __restrict__ xs,
@@ -158,14 +159,13 @@ __global__ void __launch_bounds__(256) k_nbr_build(SimParams p, GridParams g0, S
       uint32_t q = 0;
       for (int dx = -g.reach; dx <= g.reach; ++dx)
         for (int dy = -g.reach; dy <= g.reach; ++dy) {
-          Run r = run_of(g, cell_start, cx, cy, cz, dx, dy);
-          for (uint32_t u = r.b; u < r.e; ++u) {
-            f3 d = xyz(__ldg(xs + u)) - xi;
-            if (within_h(p, d)) {
+          const Run r = run_of(g, cell_start, cx, cy, cz, dx, dy);
+          test_run(xs, r.b, r.e, xi, p.h2, [&](uint32_t u0, unsigned mask) {
+            for_each_hit(u0, mask, [&](uint32_t u) {
               if (q < max_nbr) out[32u * q] = u;
               ++q;
-            }
-          }
+            });
+          });
         }
       nbr_count[t] = q;
       const unsigned m = __activemask();
@@ -206,17 +206,21 @@ __global__ void __launch_bounds__(256) k_nbr_build_feat(SimParams p, GridParams 
       float w = 0.0f;  // sum of (h^2 - r^2)^3 over the neighbours
       for (int dx = -g.reach; dx <= g.reach; ++dx)
         for (int dy = -g.reach; dy <= g.reach; ++dy) {
-          Run r = run_of(g, cell_start, cx, cy, cz, dx, dy);
-          for (uint32_t u = r.b; u < r.e; ++u) {
-            f3 d = xyz(__ldg(xs + u)) - xi;
-            const float r2 = dist2_rn(d);
-            if (r2 <= p.h2) {
-              if (q < max_nbr) out[32u * q] = u;
-              ++q;
-              const float c = p.h2 - r2;
-              w = w + c * c * c;
-            }
-          }
+          const Run r = run_of(g, cell_start, cx, cy, cz, dx, dy);
+          test_run<true>(
+              xs, r.b, r.e, xi, p.h2,
+              [&](uint32_t u0, unsigned mask) {
+                for_each_hit(u0, mask, [&](uint32_t u) {
+                  if (q < max_nbr) out[32u * q] = u;
+                  ++q;
+                });
+              },
+              [&](float r2, bool in) {
+                if (in) {
+                  const float c = p.h2 - r2;
+                  w = w + c * c * c;
+                }
+              });
         }
       nbr_count[t] = q;
       const unsigned m = __activemask();

@@ -568,16 +568,16 @@ __global__ void __launch_bounds__(256) k_ns_sorted(uint32_t n, const uint32_t* _
   sorted[t] = x;
 }
 
-template <class Hit>
-__device__ __forceinline__ void visit_cells27(const GridParams& g, const uint32_t* __restrict__ cell_start,
-                                              const float4* __restrict__ sorted, f3 xi, float h2, Hit&& hit) {
+template <class Hits>
+__device__ __forceinline__ void test_cells27(const GridParams& g, const uint32_t* __restrict__ cell_start,
+                                             const float4* __restrict__ sorted, f3 xi, float h2, Hits&& hits) {
   const int cx = cell_axis(xi.x, g.origin[0], g.inv_cell[0], g.dim[0]);
   const int cy = cell_axis(xi.y, g.origin[1], g.inv_cell[1], g.dim[1]);
   const int cz = cell_axis(xi.z, g.origin[2], g.inv_cell[2], g.dim[2]);
   for (int dx = -1; dx <= 1; ++dx)
     for (int dy = -1; dy <= 1; ++dy) {
       const Run r = run_of(g, cell_start, cx, cy, cz, dx, dy);
-      visit_run(sorted, r.b, r.e, xi, h2, hit);
+      test_run(sorted, r.b, r.e, xi, h2, hits);
     }
 }
 
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(128) k_ns_count(uint32_t n, GridParams g, floa
   if (t >= n) return;
   const float4 x = sorted[t];
   uint32_t c = 0;
-  visit_cells27(g, cell_start, sorted, xyz(x), h2, [&](uint32_t) { ++c; });
+  test_cells27(g, cell_start, sorted, xyz(x), h2, [&](uint32_t, unsigned mask) { c += (uint32_t)__popc(mask); });
   count[__float_as_uint(x.w)] = c;
 }
 
@@ -615,13 +615,15 @@ __global__ void __launch_bounds__(32 * kListWarps) k_ns_list(uint32_t n, GridPar
   if (t < n) {
     const float4 x = sorted[t];
     at = __ldg(offset + __float_as_uint(x.w));
-    visit_cells27(g, cell_start, sorted, xyz(x), h2, [&](uint32_t u) {
-      const uint32_t id = __float_as_uint(__ldg(&sorted[u].w));
-      if (q < kListRows)
-        rows[33u * q + lane] = id;
-      else
-        list[at + q] = id;
-      ++q;
+    test_cells27(g, cell_start, sorted, xyz(x), h2, [&](uint32_t u0, unsigned mask) {
+      for_each_hit(u0, mask, [&](uint32_t u) {
+        const uint32_t id = __float_as_uint(__ldg(&sorted[u].w));
+        if (q < kListRows)
+          rows[33u * q + lane] = id;
+        else
+          list[at + q] = id;
+        ++q;
+      });
     });
   }
   __syncwarp();
