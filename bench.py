@@ -51,8 +51,7 @@ FALLBACK_HBM_GBS = 6800.0
 # each field read or written once; neighbour gathers are cache-served.
 ALG_BYTES = {
     "predict": 68,            # read x, v, a; write x*, key (+ rank)
-    "sort": 32,               # key, rank, id -> perm_raw, id_raw; cell fix -> perm
-    "gather": 76,             # perm -> pos, x*, id in the new order
+    "sort": 104,              # key, rank, id -> perm_raw, id_raw; cell fix -> perm, with pos, x*, id in the new order
     "nbr_build": 20,          # read x*, write count; + 4 B per list entry written (added per run)
     "nbr_build_feat": 92,     # the build + read x, bData, previous lambda, SDF; write 2 feature float4
     "mlp": 68,                # read 8 features (32), x* (16); write (x*, lambda_hat) (16), lambda sum (4)
@@ -493,17 +492,17 @@ def gpu_arm(args, dist):
                 "passes": {k: {"launches": v[0], "ms": round(v[1], 4),
                                "share": round(v[1] / total_ms, 4) if total_ms else None} for k, v in kt.items()}}
     if chosen["learned_iters"] is None:
-        # per substep: predict, scan + scatter + cell fix + big cells, gather,
+        # per substep: predict, scan + scatter + cell fix + big cells,
         # neighbour build, band pass, 3 per iteration (band sampling, lambda,
-        # delta-p), density/velocity, vorticity, XSPH
-        per_sub = 11 + 3 * iters
+        # delta-p), density/velocity, vorticity, XSPH (the last one also
+        # writes the by-id positions)
+        per_sub = 10 + 3 * iters
     else:
-        # predict, 4 sort, gather, lam_prev gather, band pass + sampling at
-        # x*_0, build with features, network, first projection, 3 per
-        # iteration, density/velocity, fallback decision, fallback kernel,
-        # vorticity, XSPH
-        per_sub = 17 + 3 * chosen["learned_iters"]
-    launches_per_frame = sub * per_sub + 1  # + export
+        # predict, 4 sort, band pass + sampling at x*_0, build with features,
+        # network, first projection, 3 per iteration, density/velocity,
+        # fallback decision, fallback kernel, vorticity, XSPH
+        per_sub = 15 + 3 * chosen["learned_iters"]
+    launches_per_frame = sub * per_sub
     m = plain["metrics"]
     line = {
         "metric": METRIC, "value": chosen["value"], "unit": UNIT, "n_gpus": dist.world, "steps": args.steps,

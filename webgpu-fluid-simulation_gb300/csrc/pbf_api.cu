@@ -70,7 +70,11 @@ struct pbf_handle {
   DBuf<float4> pos[2], xs[2], xl, vel, acc, bdata, omega, normal, dp, out_pos, out_tmp;
   DBuf<float4> visc, coh;  // fast mode: XSPH's viscosity and cohesion sums from the vorticity pass
   DBuf<uint32_t> ids[2], key, rank, perm_raw, id_raw, perm, tmp_a, tmp_b;
-  DBuf<uint32_t> cell_count, cell_start, big_list, big_count;
+  // counts of this substep's cells and, cleared by its scan, of the next one's
+  DBuf<uint32_t> cell_count[2], cell_start, big_list, big_count;
+  int count_buf = 0;         // the buffer that the next substep counts into
+  bool count_clear = false;  // ... and whether it is known to be all zero
+  int xs_final = 0;          // the xs buffer holding the last substep's x*
   DBuf<uint32_t> nbr_count, nbr_max, nbr_list;
   DBuf<uint32_t> band_list[2], band_count;  // boundary band lists (ping-pong) and their lengths
   // cell-block passes (PBF_BUILD_CELLBLOCK_*): cell key and x*_0 per sorted
@@ -95,6 +99,7 @@ struct pbf_handle {
   cudaGraphExec_t graph_exec = nullptr;
   bool graph_enabled = false;
   bool graph_valid = false;
+  int graph_cur = 0, graph_count_buf = 0;  // the buffers that the graph starts from
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   uint32_t last_nbr_total = 0;
   // learned start and trace capture
@@ -148,11 +153,11 @@ struct pbf_handle {
 namespace {
 
 enum PassId {
-  K_PREDICT, K_SORT, K_GATHER, K_NBR_BUILD, K_BOUNDARY, K_LAMBDA, K_DELTAP, K_DENSITY, K_VORTICITY, K_XSPH,
+  K_PREDICT, K_SORT, K_NBR_BUILD, K_BOUNDARY, K_LAMBDA, K_DELTAP, K_DENSITY, K_VORTICITY, K_XSPH,
   K_EXPORT, K_FEATURES, K_MLP, K_FALLBACK, K_NUM
 };
-const char* kPassNames[K_NUM] = {"predict",   "sort", "gather", "nbr_build", "boundary",     "lambda", "deltap_apply",
-                                 "density_velocity", "vorticity", "xsph", "export", "nbr_build_feat", "mlp",
+const char* kPassNames[K_NUM] = {"predict", "sort", "nbr_build", "boundary", "lambda", "deltap_apply", "density_velocity",
+                                 "vorticity", "xsph", "export", "nbr_build_feat", "mlp",
                                  "fallback_guarded"};
 
 // Brackets one launch (or one group of launches) with events when timing is on.
@@ -380,8 +385,9 @@ int check_device_errors(pbf_handle* h) {
 
 // One substep: the dispatch sequence of PBF.run (PBF.ts:398-448).  When
 // `ev` is given, events are recorded at the reference's four interval
-// boundaries (PBF.runTimestamp, PBF.ts:450-510).
-int substep(pbf_handle* h, cudaEvent_t* ev) {
+// boundaries (PBF.runTimestamp, PBF.ts:450-510).  With exported given, the
+// last pass also writes the by-id positions where it can (*exported).
+int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   const uint32_t n = h->n;
   cudaStream_t st = h->stream;
   SimParams p = h->sp;
@@ -397,35 +403,37 @@ int substep(pbf_handle* h, cudaEvent_t* ev) {
   const unsigned cbg = cb_grid(n);
   if (ev) CU(h, cudaEventRecord(ev[0], st));
   // neighborSearch.clearBuffer + TimeIntegration (+ ParticleInsert counts)
-  CU(h, cudaMemsetAsync(h->cell_count.p, 0, ((size_t)g.cells + 1) * sizeof(uint32_t), st));
+  uint32_t* const counts = h->cell_count[h->count_buf].p;
+  if (!h->count_clear) CU(h, cudaMemsetAsync(counts, 0, ((size_t)g.cells + 1) * sizeof(uint32_t), st));
+  h->count_clear = false;
   {
-  KScope ks(h, K_PREDICT);
-  ps.predict<<<grid_of(h, n), h->blk, 0, st>>>(p, g, h->tab, h->pos[c].p, h->vel.p, h->acc.p, h->xs[1].p,
-                                                       h->key.p, h->rank.p, h->cell_count.p);
+    KScope ks(h, K_PREDICT);
+    const ClearArgs clear{(uint32_t*)h->scan_scratch,
+                          (uint32_t)(scan_scratch_bytes((size_t)g.cells + 1) / sizeof(uint32_t)), h->big_count.p,
+                          h->band_count.p};
+    ps.predict<<<grid_of(h, n), h->blk, 0, st>>>(p, g, h->tab, h->pos[c].p, h->vel.p, h->acc.p, h->xs[1].p, h->key.p,
+                                                 h->rank.p, counts, clear);
   }
   CU(h, cudaGetLastError());
   if (ev) CU(h, cudaEventRecord(ev[1], st));
   // cell scan + counting sort (stable by id) + reorder of the state
-  SortBuffers sb{h->key.p,     h->rank.p,  h->cell_count.p, h->cell_start.p, h->perm_raw.p, h->id_raw.p,
-                 h->perm.p,    h->tmp_a.p, h->tmp_b.p,      h->big_list.p,   h->big_count.p, h->scan_scratch,
-                 h->err_word.p};
-  {
-    KScope ks(h, K_SORT);
-    CU(h, launch_sort_by_cell(g, n, h->ids[c].p, sb, h->id_bits, st));
-  }
+  SortBuffers sb{h->key.p,    h->rank.p,  counts,    h->cell_count[1 - h->count_buf].p, h->cell_start.p, h->perm_raw.p,
+                 h->id_raw.p, h->perm.p,  h->tmp_a.p, h->tmp_b.p,                       h->big_list.p,   h->big_count.p,
+                 h->scan_scratch, h->err_word.p};
   // the learned start's and trace capture's features: the previous multiplier
-  // sum is gathered with the state
+  // sum moves with the state
   const bool need_feat = h->learned || h->trace_cap > 0;
   {
-    KScope ks(h, K_GATHER);
-    if (cb)
-      CU(h, launch_gather_state_cb(n, h->perm.p, h->pos[c].p, h->xs[1].p, h->ids[c].p, h->key.p, h->pos[nx].p,
-                                   h->xs[0].p, h->ids[nx].p, h->skey.p, h->xs0.p, st,
-                                   need_feat ? h->lam_sum.p : nullptr, need_feat ? h->lam_prev.p : nullptr));
-    else
-      CU(h, launch_gather_state(n, h->perm.p, h->pos[c].p, h->xs[1].p, h->ids[c].p, h->pos[nx].p, h->xs[0].p,
-                                h->ids[nx].p, st, need_feat ? h->lam_sum.p : nullptr,
-                                need_feat ? h->lam_prev.p : nullptr));
+    KScope ks(h, K_SORT);
+    GatherArgs G{h->pos[c].p, h->xs[1].p, h->key.p, need_feat ? h->lam_sum.p : nullptr, h->pos[nx].p, h->xs[0].p,
+                 h->ids[nx].p, need_feat ? h->lam_prev.p : nullptr, nullptr, nullptr};
+    if (cb) {
+      G.skey_out = h->skey.p;
+      G.xs0_out = h->xs0.p;
+    }
+    CU(h, launch_sort_by_cell(g, n, h->ids[c].p, sb, h->id_bits, G, st));
+    h->count_buf = 1 - h->count_buf;
+    h->count_clear = true;
   }
   h->cur = nx;
   const int cc = nx;
@@ -436,7 +444,6 @@ int substep(pbf_handle* h, cudaEvent_t* ev) {
   // band pass builds it at x*_0, each delta-p pass marks the band of the next
   // iteration at the positions it writes, and the sampling kernel interpolates
   // the volume map for the listed slots only.
-  CU(h, cudaMemsetAsync(h->band_count.p, 0, 2 * sizeof(uint32_t), st));
   int band = -1;  // band list holding the current iteration's band (-1: not built)
   const unsigned band_grid = std::min(nblocks(n, 256), (unsigned)h->sms * 2u);  // one resident wave
   auto band_args = [&](int list, float* bsdf) {
@@ -737,7 +744,11 @@ int substep(pbf_handle* h, cudaEvent_t* ev) {
                                         dim3(256), args, 0, st));
     }
   }
-  if (a != 0) CU(h, cudaMemcpyAsync(h->xs[0].p, h->xs[1].p, (size_t)n * sizeof(float4), cudaMemcpyDeviceToDevice, st));
+  h->xs_final = a;
+  // per-kernel timing keeps the export a launch of its own
+  const bool ex_here = exported && !cb && !h->ktiming;
+  const ExportArgs ex = ex_here ? ExportArgs{h->ids[cc].p, h->out_pos.p} : ExportArgs{nullptr, nullptr};
+  if (ex_here) *exported = true;
   if (cb && cs.xsph_split) {  // fast mode: XSPH's sum split over the two passes
     {
       KScope ks(h, K_VORTICITY);
@@ -773,7 +784,7 @@ int substep(pbf_handle* h, cudaEvent_t* ev) {
     {
       KScope ks(h, K_XSPH);
       ps.xsph_split<<<grid_of(h, n), h->blk, 0, st>>>(p, h->pos[cc].p, h->omega.p, h->normal.p, h->visc.p, h->coh.p,
-                                                       ms, h->nbr_count.p, h->nbr_list.p, h->acc.p);
+                                                       ms, h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
     }
     CU(h, cudaGetLastError());
   } else {
@@ -786,7 +797,7 @@ int substep(pbf_handle* h, cudaEvent_t* ev) {
     {
       KScope ks(h, K_XSPH);
       ps.xsph<<<grid_of(h, n), h->blk, 0, st>>>(p, h->pos[cc].p, h->vel.p, h->omega.p, h->normal.p, ms,
-                                                 h->nbr_count.p, h->nbr_list.p, h->acc.p);
+                                                 h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
     }
     CU(h, cudaGetLastError());
   }
@@ -800,12 +811,13 @@ int export_positions(pbf_handle* h) {
   return PBF_OK;
 }
 
-int frame(pbf_handle* h) {
-  for (uint32_t s = 0; s < h->cfg.substeps; ++s) {
-    int rc = substep(h, nullptr);
+int frame(pbf_handle* h, uint32_t substeps) {
+  bool exported = false;
+  for (uint32_t s = 0; s < substeps; ++s) {
+    int rc = substep(h, nullptr, s + 1 == substeps ? &exported : nullptr);
     if (rc) return rc;
   }
-  return export_positions(h);
+  return exported ? PBF_OK : export_positions(h);
 }
 
 // The state after an upload of n particles whose positions (w = 0) and ids
@@ -859,7 +871,7 @@ void release_all(pbf_handle* h) {
                          &h->omega,  &h->normal, &h->dp,    &h->out_pos, &h->out_tmp, &h->xs0};
   for (auto* b : f4s) b->release();
   DBuf<uint32_t>* u32s[] = {&h->ids[0],   &h->ids[1],      &h->key,      &h->rank,      &h->perm_raw,
-                            &h->id_raw,   &h->perm,        &h->tmp_a,    &h->tmp_b,     &h->cell_count,
+                            &h->id_raw,   &h->perm,        &h->tmp_a,    &h->tmp_b,     &h->cell_count[0], &h->cell_count[1],
                             &h->cell_start, &h->big_list,  &h->big_count, &h->nbr_count, &h->nbr_max,
                             &h->nbr_list, &h->err_word,    &h->m_u,      &h->skey,      &h->cb_mask};
   for (auto* b : u32s) b->release();
@@ -963,11 +975,16 @@ void pack_field_blocks(const uint32_t res[3], const float* sdf, const float* vol
 // (Re)allocates the cell arrays for h->gp.cells cells.
 cudaError_t alloc_cells(pbf_handle* h) {
   const size_t cells = h->gp.cells;
-  if (h->cell_count.p && h->cell_count.n == cells + 1) return cudaSuccess;
-  h->cell_count.release();
+  if (h->cell_count[0].p && h->cell_count[1].p && h->cell_start.p && h->big_list.p && h->scan_scratch &&
+      h->cell_count[0].n == cells + 1)
+    return cudaSuccess;
+  h->cell_count[0].release();
+  h->cell_count[1].release();
   h->cell_start.release();
   h->big_list.release();
-  cudaError_t e = h->cell_count.alloc(cells + 1);
+  h->count_clear = false;
+  cudaError_t e = h->cell_count[0].alloc(cells + 1);
+  if (e == cudaSuccess) e = h->cell_count[1].alloc(cells + 1);
   if (e == cudaSuccess) e = h->cell_start.alloc(cells + 1);
   if (e == cudaSuccess) e = h->big_list.alloc(cells);
   if (h->scan_scratch) {
@@ -1212,7 +1229,8 @@ int pbf_create(const pbf_config* cfg, pbf_handle** out) {
   A(h->perm.alloc(cap));
   A(h->tmp_a.alloc(cap));
   A(h->tmp_b.alloc(cap));
-  A(h->cell_count.alloc(cells + 1));
+  A(h->cell_count[0].alloc(cells + 1));
+  A(h->cell_count[1].alloc(cells + 1));
   A(h->cell_start.alloc(cells + 1));
   A(h->big_list.alloc(cells));
   A(h->big_count.alloc(1));
@@ -1612,9 +1630,7 @@ int pbf_set_capture(pbf_handle* h, int enable) {
 int pbf_run(pbf_handle* h) {
   if (!h) return PBF_EINVAL;
   if (h->paused || h->n == 0) return PBF_OK;
-  int rc = substep(h, nullptr);
-  if (rc) return rc;
-  return export_positions(h);
+  return frame(h, 1);
 }
 
 int pbf_enable_graph(pbf_handle* h, int enable) {
@@ -1632,7 +1648,7 @@ int pbf_step(pbf_handle* h, uint32_t frames) {
   // runs eagerly, as per-kernel timing does.
   if (!h->graph_enabled || h->ktiming || h->trace_cap > 0) {
     for (uint32_t f = 0; f < frames; ++f) {
-      int rc = frame(h);
+      int rc = frame(h, h->cfg.substeps);
       if (rc) return rc;
     }
     return PBF_OK;
@@ -1641,14 +1657,22 @@ int pbf_step(pbf_handle* h, uint32_t frames) {
   // number of substeps (one frame, or two frames when substeps is odd) and
   // every replay starts from the same buffers.
   const uint32_t per_graph = (h->cfg.substeps % 2 == 0) ? 1u : 2u;
+  if (h->graph_valid && (h->graph_cur != h->cur || h->graph_count_buf != h->count_buf || !h->count_clear))
+    invalidate_graph(h);  // single substeps since the capture left the other buffers current
   if (!h->graph_valid) {
-    const int start_cur = h->cur;
+    if (!h->count_clear) {  // the graph relies on its counts being clear
+      CU(h, cudaMemsetAsync(h->cell_count[h->count_buf].p, 0, ((size_t)h->gp.cells + 1) * sizeof(uint32_t), h->stream));
+      h->count_clear = true;
+    }
+    const int start_cur = h->cur, start_buf = h->count_buf;
     cudaGraph_t g = nullptr;
     CU(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int rc = PBF_OK;
-    for (uint32_t f = 0; f < per_graph && rc == PBF_OK; ++f) rc = frame(h);
+    for (uint32_t f = 0; f < per_graph && rc == PBF_OK; ++f) rc = frame(h, h->cfg.substeps);
     cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
     h->cur = start_cur;  // capture only recorded the work
+    h->count_buf = start_buf;
+    h->count_clear = true;
     if (rc) {
       if (g) cudaGraphDestroy(g);
       return rc;
@@ -1658,6 +1682,8 @@ int pbf_step(pbf_handle* h, uint32_t frames) {
     cudaGraphDestroy(g);
     if (ce != cudaSuccess) return fail(h, PBF_ECUDA, "graph instantiate: %s", cudaGetErrorString(ce));
     h->graph_valid = true;
+    h->graph_cur = start_cur;
+    h->graph_count_buf = start_buf;
   }
   uint32_t full = frames / per_graph, rest = frames % per_graph;
   for (uint32_t f = 0; f < full; ++f) CU(h, cudaGraphLaunch(h->graph_exec, h->stream));
@@ -1665,7 +1691,7 @@ int pbf_step(pbf_handle* h, uint32_t frames) {
     // an odd remainder runs eagerly and leaves the buffers swapped: the graph
     // no longer matches them
     invalidate_graph(h);
-    int rc = frame(h);
+    int rc = frame(h, h->cfg.substeps);
     if (rc) return rc;
   }
   return PBF_OK;
@@ -1943,7 +1969,7 @@ int pbf_copy_field(pbf_handle* h, int field, void* host, size_t bytes) {
     case PBF_FIELD_POSITION: src4 = h->pos[h->cur].p; break;
     case PBF_FIELD_VELOCITY: src4 = h->vel.p; break;
     case PBF_FIELD_ACCELERATION: src4 = h->acc.p; break;
-    case PBF_FIELD_PREDICTED: src4 = h->xs[0].p; break;
+    case PBF_FIELD_PREDICTED: src4 = h->xs[h->xs_final].p; break;
     case PBF_FIELD_BOUNDARY: src4 = h->bdata.p; break;
     case PBF_FIELD_OMEGA: src4 = h->omega.p; break;
     case PBF_FIELD_NORMAL: src4 = h->normal.p; break;  // w (|omega|, internal) is cleared below
@@ -2001,7 +2027,7 @@ int pbf_copy_search_state(pbf_handle* h, int which, uint32_t* host, size_t count
     for (uint32_t s = 0; s < n; ++s) host[old_ids[s]] = key[s];
   } else {
     const uint32_t* src = which == PBF_SEARCH_ORDER        ? h->ids[h->cur].p
-                          : which == PBF_SEARCH_CELL_COUNT ? h->cell_count.p
+                          : which == PBF_SEARCH_CELL_COUNT ? h->cell_count[1 - h->count_buf].p
                                                            : h->cell_start.p;
     CU(h, cudaMemcpyAsync(host, src, need * 4, cudaMemcpyDeviceToHost, st));
     CU(h, cudaStreamSynchronize(st));

@@ -16,7 +16,7 @@ namespace pbf {
 // one tile per CTA or persistent (grid-stride).
 struct PassSet {
   void (*predict)(SimParams, GridParams, SceneTab, const float4*, const float4*, const float4*, float4*, uint32_t*,
-                  uint32_t*, uint32_t*);
+                  uint32_t*, uint32_t*, ClearArgs);
   void (*nbr_build)(SimParams, GridParams, SceneTab, const float4*, const uint32_t*, uint32_t, uint32_t*, uint32_t*,
                     uint32_t*, uint32_t*);
   void (*nbr_build2)(SimParams, GridParams, SceneTab, const float4*, const uint32_t*, uint32_t, uint32_t*,
@@ -41,12 +41,12 @@ struct PassSet {
   void (*vorticity)(SimParams, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*, float4*,
                     float4*);
   void (*xsph)(SimParams, const float4*, const float4*, const float4*, const float4*, uint32_t, const uint32_t*,
-               const uint32_t*, float4*);
+               const uint32_t*, float4*, ExportArgs);
   // fast mode: XSPH's neighbour sum split over the vorticity and XSPH passes (null in exact mode)
   void (*vorticity_split)(SimParams, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*,
                           float4*, float4*, float4*, float4*);
   void (*xsph_split)(SimParams, const float4*, const float4*, const float4*, const float4*, const float4*, uint32_t,
-                     const uint32_t*, const uint32_t*, float4*);
+                     const uint32_t*, const uint32_t*, float4*, ExportArgs);
 };
 
 // The cell-block passes of one membership variant (pbf_cellblock.cuh).
@@ -92,15 +92,21 @@ size_t scan_scratch_bytes(size_t n);
 // bounded look-back wait gives up.
 cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* scratch, uint32_t* err,
                                   cudaStream_t st);
+// The same with the scratch already cleared by the caller's own kernel; zero
+// (optional): another array of n entries that the scan clears.
+cudaError_t launch_exclusive_scan_cleared(const uint32_t* in, uint32_t* out, size_t n, void* scratch, uint32_t* err,
+                                          cudaStream_t st, uint32_t* zero);
 // Self-test of the scan's bounded look-back wait (a predecessor status that
 // nothing writes): *err receives PBF_DEVERR_SCAN_TIMEOUT.
 cudaError_t launch_scan_timeout_selftest(uint32_t* err, cudaStream_t st);
 
-// Counting-sort pipeline shared by the step and the stand-alone search.
+// The step's counting sort.  The caller has cleared cell_count, the scan's
+// scratch and big_count (k_predict clears the last two).
 struct SortBuffers {
   uint32_t* key;        // [n] cell key per input slot
   uint32_t* rank;       // [n] warp-aggregated (unordered) rank per input slot
   uint32_t* cell_count; // [cells + 1]
+  uint32_t* count_next; // [cells + 1] cleared by the scan: the next substep's counts
   uint32_t* cell_start; // [cells + 1] exclusive scan of cell_count
   uint32_t* perm_raw;   // [n] scattered slots (unordered within a cell)
   uint32_t* id_raw;     // [n] particle id of perm_raw entries
@@ -111,6 +117,23 @@ struct SortBuffers {
   uint32_t* big_count;  // [1]
   void* scan_scratch;
   uint32_t* err;
+};
+// The particle state moved into the new order with the sort: positions,
+// predicted positions and ids, f (optional): one scalar per particle (the
+// learned start's previous multiplier sum); skey_out / xs0_out (optional, for
+// the cell-block passes): the cell key of each sorted slot and a second copy
+// of x*_0 that the solve leaves untouched.
+struct GatherArgs {
+  const float4* pos_in;
+  const float4* xs_in;
+  const uint32_t* key;
+  const float* f_in;
+  float4* pos_out;
+  float4* xs_out;
+  uint32_t* id_out;
+  float* f_out;
+  uint32_t* skey_out;
+  float4* xs0_out;
 };
 
 // Stable LSD radix sort of points in particle-id order by cell key (the
@@ -136,21 +159,9 @@ cudaError_t launch_cell_offsets(uint32_t cells, const uint32_t* cell_count, uint
 // rank_out[order[q]] = q - cell_start[skeys[q]].
 cudaError_t launch_rank_sorted(uint32_t n, const uint32_t* skeys, const uint32_t* order, const uint32_t* cell_start,
                                uint32_t* rank_out, cudaStream_t st);
-// scatter + stable within-cell order + (optionally) gather of the particle state.
+// Scan of the counts, scatter, stable within-cell order with the state moved along.
 cudaError_t launch_sort_by_cell(GridParams g, uint32_t n, const uint32_t* ids, SortBuffers& b, uint32_t id_bits,
-                                cudaStream_t st);
-// f_in / f_out (optional): one scalar per particle gathered along (the
-// learned start's previous multiplier sum).
-cudaError_t launch_gather_state(uint32_t n, const uint32_t* perm, const float4* pos_in, const float4* xs_in,
-                                const uint32_t* id_in, float4* pos_out, float4* xs_out, uint32_t* id_out,
-                                cudaStream_t st, const float* f_in = nullptr, float* f_out = nullptr);
-// The same gather that also writes, for the cell-block passes, the cell key
-// of each sorted slot (skey_out[t] = key_in[perm[t]]) and a second copy of
-// the predicted positions x*_0 (xs0_out) that the solve leaves untouched.
-cudaError_t launch_gather_state_cb(uint32_t n, const uint32_t* perm, const float4* pos_in, const float4* xs_in,
-                                   const uint32_t* id_in, const uint32_t* key_in, float4* pos_out, float4* xs_out,
-                                   uint32_t* id_out, uint32_t* skey_out, float4* xs0_out, cudaStream_t st,
-                                   const float* f_in = nullptr, float* f_out = nullptr);
+                                const GatherArgs& G, cudaStream_t st);
 cudaError_t launch_scatter_by_id(uint32_t n, const uint32_t* id, const float4* src, float4* dst, cudaStream_t st);
 // dst[id[t]] = src[t].w (a scalar kept in the w lane of a packed float4 array)
 cudaError_t launch_scatter_w_by_id(uint32_t n, const uint32_t* id, const float4* src, float* dst, cudaStream_t st);

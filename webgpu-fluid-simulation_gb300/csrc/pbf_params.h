@@ -62,6 +62,22 @@ struct SceneDesc {
   uint32_t first, n;
 };
 
+// Scratch words that k_predict clears for the passes after it: the scan's
+// (counter and tile status), the list length of very full cells and the two
+// band counts.
+struct ClearArgs {
+  uint32_t* scan;
+  uint32_t scan_words;
+  uint32_t* big_count;
+  uint32_t* band_count;
+};
+
+// The by-id positions written by the last pass of a frame (id null: none).
+struct ExportArgs {
+  const uint32_t* id;  // [n] particle id of each slot
+  float4* out;         // [n] (x, rho) by id
+};
+
 // Boundary band of the next boundary sampling: the particles whose field
 // cell can produce a sample.  Whoever computes a new x* (the band pass, or
 // delta-p for the next iteration) tests the cell flag: outside the band it

@@ -92,7 +92,15 @@ __global__ void __launch_bounds__(256) k_predict(SimParams p0, GridParams g0, Sc
                                                  const float4* __restrict__ pos, const float4* __restrict__ vel,
                                                  const float4* __restrict__ acc, float4* __restrict__ xs_out,
                                                  uint32_t* __restrict__ key_out, uint32_t* __restrict__ rank_out,
-                                                 uint32_t* cell_count) {
+                                                 uint32_t* cell_count, ClearArgs clear) {
+  // scratch of the passes that follow (four memset launches otherwise)
+  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  for (uint32_t i = i0; i < clear.scan_words; i += gridDim.x * blockDim.x) clear.scan[i] = 0u;
+  if (i0 == 0u) {
+    *clear.big_count = 0u;
+    clear.band_count[0] = 0u;
+    clear.band_count[1] = 0u;
+  }
   PBF_TILES(p0.n) {
     const uint32_t s = tile0 + threadIdx.x;
     uint32_t key = kNoKey;
@@ -1123,12 +1131,14 @@ __global__ void __launch_bounds__(256, 4) k_xsph(SimParams p, const float4* __re
                                                  uint32_t max_nbr,
                                                  const uint32_t* __restrict__ nbr_cnt,
                                                  const uint32_t* __restrict__ nbr_list,
-                                                 float4* __restrict__ acc) {
+                                                 float4* __restrict__ acc, ExportArgs ex) {
   PBF_SLOTS(t, p.n) {
     uint32_t b, e;
     list_slice(max_nbr, nbr_cnt, t, b, e);
     XsphSum s;
-    s.init(pos[t], xyz(vel[t]), xyz(normal[t]));
+    const float4 pi = pos[t];
+    if (ex.id) ex.out[ex.id[t]] = pi;
+    s.init(pi, xyz(vel[t]), xyz(normal[t]));
     for_each_neighbor(nbr_list, b, e, pos,
                       [&](uint32_t j, float4 pj) { s.add(p, pj, __ldg(vel + j), __ldg(normal + j)); });
     xsph_finish(p, acc, t, s, xyz(omega[t]));
@@ -1166,12 +1176,15 @@ __global__ void __launch_bounds__(256) k_xsph_split(SimParams p, const float4* _
                                                     const float4* __restrict__ visc,
                                                     const float4* __restrict__ coh_sum, uint32_t max_nbr,
                                                     const uint32_t* __restrict__ nbr_cnt,
-                                                    const uint32_t* __restrict__ nbr_list, float4* __restrict__ acc) {
+                                                    const uint32_t* __restrict__ nbr_list, float4* __restrict__ acc,
+                                                    ExportArgs ex) {
   PBF_SLOTS(t, p.n) {
     uint32_t b, e;
     list_slice(max_nbr, nbr_cnt, t, b, e);
     XsphSplitSum s;
-    s.init(pos[t], xyz(normal[t]));
+    const float4 pi = pos[t];
+    if (ex.id) ex.out[ex.id[t]] = pi;
+    s.init(pi, xyz(normal[t]));
     for_each_neighbor2(nbr_list, b, e, pos, normal, [&](uint32_t, float4 pj, float4 nj) { s.add(p, pj, nj); });
     xsph_split_finish(p, acc, t, s, xyz(omega[t]), visc[t], coh_sum[t]);
   }

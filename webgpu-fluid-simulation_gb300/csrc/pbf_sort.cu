@@ -71,10 +71,11 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total,
 
 // Single-pass scan: tiles take ids from a counter in launch order, publish
 // their aggregate, look back over predecessors (bounded waits) and publish
-// the inclusive prefix.  Status words pack (flag << 32 | value).
+// the inclusive prefix.  Status words pack (flag << 32 | value).  zero
+// (optional, n entries) is cleared along the way.
 __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                        size_t n, unsigned long long* status, uint32_t* counter,
-                                                       uint32_t* err) {
+                                                       uint32_t* err, uint32_t* __restrict__ zero) {
   __shared__ uint32_t s_items[kScanTile + kScanTile / 32];
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_tile;
@@ -89,6 +90,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t* __restric
     int li = k * kScanThreads + threadIdx.x;
     size_t gi = base + li;
     s_items[li + (li >> 5)] = (gi < n) ? __ldg(in + gi) : 0u;
+    if (zero && gi < n) zero[gi] = 0u;
   }
   __syncthreads();
   uint32_t items[kScanItems];
@@ -172,51 +174,65 @@ __global__ void __launch_bounds__(256) k_scatter(uint32_t n, const uint32_t* __r
   id_raw[dst] = ids ? __ldg(ids + s) : s;
 }
 
-// ---- stable within-cell order ------------------------------------------------------
+// ---- stable within-cell order and the state in the new order ------------------------
+// Moves the state of input slot s (particle id) to sorted slot d.
+template <bool kCb>
+__device__ __forceinline__ void place_state(const GatherArgs& G, uint32_t d, uint32_t s, uint32_t id) {
+  G.pos_out[d] = __ldg(G.pos_in + s);
+  const float4 x = __ldg(G.xs_in + s);
+  G.xs_out[d] = x;
+  G.id_out[d] = id;
+  if constexpr (kCb) {
+    G.xs0_out[d] = x;
+    G.skey_out[d] = __ldg(G.key + s);
+  }
+  if (G.f_in) G.f_out[d] = __ldg(G.f_in + s);
+}
+
 // One thread per sorted position q: the entry scattered there ranks itself
-// by particle id among its cell's entries and moves to cell_start + rank.
-// The work follows the particles (sum over cells of count^2), not the cell
-// count, so empty cells cost nothing.  Cells above kRankMax entries go to
-// the block radix path (the thread at the cell's first position lists it).
+// by particle id among its cell's entries and moves to cell_start + rank,
+// with its state (the cell is a few consecutive slots, so the stores of a warp
+// stay together; a gather of its own would read the order back).  The work
+// follows the particles (sum over cells of count^2), not the cell count, so
+// empty cells cost nothing.  Cells above kRankMax entries go to the block
+// radix path (the thread at the cell's first position lists it).
 constexpr uint32_t kRankMax = 1024;
 
+template <bool kCb>
 __global__ void __launch_bounds__(256) k_cellfix(uint32_t n, const uint32_t* __restrict__ key,
                                                  const uint32_t* __restrict__ cell_count,
                                                  const uint32_t* __restrict__ cell_start,
                                                  const uint32_t* __restrict__ perm_raw,
                                                  const uint32_t* __restrict__ id_raw, uint32_t* __restrict__ perm,
-                                                 uint32_t* big_list, uint32_t* big_count) {
+                                                 uint32_t* big_list, uint32_t* big_count, GatherArgs G) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
-  const uint32_t s = perm_raw[q];
+  const uint32_t s = perm_raw[q], my = id_raw[q];
   const uint32_t c = __ldg(key + s);
-  const uint32_t cnt = __ldg(cell_count + c);
-  if (cnt == 1) {
-    perm[q] = s;
-    return;
-  }
-  const uint32_t st = __ldg(cell_start + c);
+  const uint32_t cnt = __ldg(cell_count + c), st = __ldg(cell_start + c);
   if (cnt > kRankMax) {
     if (q == st) big_list[atomicAdd(big_count, 1u)] = c;
     return;
   }
-  const uint32_t my = id_raw[q];
   uint32_t r = 0;
-  for (uint32_t m = 0; m < cnt; ++m) r += (__ldg(id_raw + st + m) < my) ? 1u : 0u;
+  if (cnt > 1)
+    for (uint32_t m = 0; m < cnt; ++m) r += (__ldg(id_raw + st + m) < my) ? 1u : 0u;
   perm[st + r] = s;
+  place_state<kCb>(G, st + r, s, my);
 }
 
 // Block LSD radix sort (8-bit digits) of one very full cell by particle id;
 // stable because tiles are processed in order and ranks within a tile follow
 // thread order.
 constexpr int kRadixThreads = 256;
+template <bool kCb>
 __global__ void __launch_bounds__(kRadixThreads) k_bigcell(const uint32_t* __restrict__ big_list,
                                                            const uint32_t* __restrict__ big_count,
                                                            const uint32_t* __restrict__ cell_count,
                                                            const uint32_t* __restrict__ cell_start,
                                                            uint32_t* __restrict__ perm_raw, uint32_t* __restrict__ id_raw,
                                                            uint32_t* __restrict__ perm, uint32_t* __restrict__ tmp_slot,
-                                                           uint32_t* __restrict__ tmp_id, int passes) {
+                                                           uint32_t* __restrict__ tmp_id, int passes, GatherArgs G) {
   __shared__ uint32_t s_base[256];
   __shared__ uint32_t s_wcount[kRadixThreads / 32][256];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -276,6 +292,8 @@ __global__ void __launch_bounds__(kRadixThreads) k_bigcell(const uint32_t* __res
       src_id = dst_id;
       __syncthreads();
     }
+    for (uint32_t e = tid; e < cnt; e += kRadixThreads) place_state<kCb>(G, st + e, src_slot[e], src_id[e]);
+    __syncthreads();
   }
 }
 
@@ -498,41 +516,6 @@ __global__ void __launch_bounds__(256) k_rank_sorted(uint32_t n, const uint32_t*
   } else {
     for (uint32_t q = q0; q < n; ++q) rank_out[order[q]] = q - __ldg(cell_start + skey[q]);
   }
-}
-
-// ---- gather of the particle state into the new order -------------------------------
-__global__ void __launch_bounds__(256) k_gather(uint32_t n, const uint32_t* __restrict__ perm,
-                                                const float4* __restrict__ pos_in, const float4* __restrict__ xs_in,
-                                                const uint32_t* __restrict__ id_in, float4* __restrict__ pos_out,
-                                                float4* __restrict__ xs_out, uint32_t* __restrict__ id_out,
-                                                const float* __restrict__ f_in, float* __restrict__ f_out) {
-  uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  uint32_t o = perm[t];
-  pos_out[t] = __ldg(pos_in + o);
-  xs_out[t] = __ldg(xs_in + o);
-  id_out[t] = id_in ? __ldg(id_in + o) : o;  // no id array: the input order is the id order
-  if (f_in) f_out[t] = __ldg(f_in + o);
-}
-
-__global__ void __launch_bounds__(256) k_gather_cb(uint32_t n, const uint32_t* __restrict__ perm,
-                                                   const float4* __restrict__ pos_in,
-                                                   const float4* __restrict__ xs_in,
-                                                   const uint32_t* __restrict__ id_in,
-                                                   const uint32_t* __restrict__ key_in, float4* __restrict__ pos_out,
-                                                   float4* __restrict__ xs_out, uint32_t* __restrict__ id_out,
-                                                   uint32_t* __restrict__ skey_out, float4* __restrict__ xs0_out,
-                                                   const float* __restrict__ f_in, float* __restrict__ f_out) {
-  uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  uint32_t o = perm[t];
-  pos_out[t] = __ldg(pos_in + o);
-  const float4 x = __ldg(xs_in + o);
-  xs_out[t] = x;
-  xs0_out[t] = x;
-  skey_out[t] = __ldg(key_in + o);
-  id_out[t] = id_in ? __ldg(id_in + o) : o;
-  if (f_in) f_out[t] = __ldg(f_in + o);
 }
 
 __global__ void k_scatter_f4(uint32_t n, const uint32_t* __restrict__ id, const float4* __restrict__ src,
@@ -797,12 +780,17 @@ size_t scan_scratch_bytes(size_t n) {
 cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* scratch, uint32_t* err,
                                   cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  size_t tiles = (n + kScanTile - 1) / kScanTile;
-  cudaError_t e = cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), st);
-  if (e != cudaSuccess) return e;
+  const cudaError_t e = cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), st);
+  return e != cudaSuccess ? e : launch_exclusive_scan_cleared(in, out, n, scratch, err, st, nullptr);
+}
+
+cudaError_t launch_exclusive_scan_cleared(const uint32_t* in, uint32_t* out, size_t n, void* scratch, uint32_t* err,
+                                          cudaStream_t st, uint32_t* zero) {
+  if (n == 0) return cudaSuccess;
+  const size_t tiles = (n + kScanTile - 1) / kScanTile;
   uint32_t* counter = reinterpret_cast<uint32_t*>(scratch);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(scratch) + 256);
-  k_scan<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, status, counter, err);
+  k_scan<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, status, counter, err, zero);
   return cudaGetLastError();
 }
 
@@ -825,7 +813,7 @@ cudaError_t launch_scan_timeout_selftest(uint32_t* err, cudaStream_t st) {
   if (e == cudaSuccess) e = cudaMemcpyAsync(counter, &one, sizeof(one), cudaMemcpyHostToDevice, st);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(scratch) + 256);
   if (e == cudaSuccess) {
-    k_scan<<<1, kScanThreads, 0, st>>>(in, out, n, status, counter, err);
+    k_scan<<<1, kScanThreads, 0, st>>>(in, out, n, status, counter, err, nullptr);
     e = cudaGetLastError();
   }
   // the host value copied above must outlive the copy
@@ -839,37 +827,20 @@ cudaError_t launch_scan_timeout_selftest(uint32_t* err, cudaStream_t st) {
 }
 
 cudaError_t launch_sort_by_cell(GridParams g, uint32_t n, const uint32_t* ids, SortBuffers& b, uint32_t id_bits,
-                                cudaStream_t st) {
-  cudaError_t e = launch_exclusive_scan(b.cell_count, b.cell_start, (size_t)g.cells + 1, b.scan_scratch, b.err, st);
+                                const GatherArgs& G, cudaStream_t st) {
+  const cudaError_t e = launch_exclusive_scan_cleared(b.cell_count, b.cell_start, (size_t)g.cells + 1, b.scan_scratch,
+                                                      b.err, st, b.count_next);
   if (e != cudaSuccess) return e;
   if (n == 0) return cudaSuccess;
   k_scatter<<<blocks_for(n, 256), 256, 0, st>>>(n, b.key, b.rank, b.cell_start, ids, b.perm_raw, b.id_raw);
-  e = cudaMemsetAsync(b.big_count, 0, sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
-  k_cellfix<<<blocks_for(n, 256), 256, 0, st>>>(n, b.key, b.cell_count, b.cell_start, b.perm_raw, b.id_raw, b.perm,
-                                                 b.big_list, b.big_count);
   int passes = (int)((id_bits + 7) / 8);
   if (passes < 1) passes = 1;
-  k_bigcell<<<152, kRadixThreads, 0, st>>>(b.big_list, b.big_count, b.cell_count, b.cell_start, b.perm_raw, b.id_raw,
-                                           b.perm, b.tmp_a, b.tmp_b, passes);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gather_state(uint32_t n, const uint32_t* perm, const float4* pos_in, const float4* xs_in,
-                                const uint32_t* id_in, float4* pos_out, float4* xs_out, uint32_t* id_out,
-                                cudaStream_t st, const float* f_in, float* f_out) {
-  if (n == 0) return cudaSuccess;
-  k_gather<<<blocks_for(n, 256), 256, 0, st>>>(n, perm, pos_in, xs_in, id_in, pos_out, xs_out, id_out, f_in, f_out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gather_state_cb(uint32_t n, const uint32_t* perm, const float4* pos_in, const float4* xs_in,
-                                   const uint32_t* id_in, const uint32_t* key_in, float4* pos_out, float4* xs_out,
-                                   uint32_t* id_out, uint32_t* skey_out, float4* xs0_out, cudaStream_t st,
-                                   const float* f_in, float* f_out) {
-  if (n == 0) return cudaSuccess;
-  k_gather_cb<<<blocks_for(n, 256), 256, 0, st>>>(n, perm, pos_in, xs_in, id_in, key_in, pos_out, xs_out, id_out,
-                                                  skey_out, xs0_out, f_in, f_out);
+  auto fix = G.skey_out ? k_cellfix<true> : k_cellfix<false>;
+  fix<<<blocks_for(n, 256), 256, 0, st>>>(n, b.key, b.cell_count, b.cell_start, b.perm_raw, b.id_raw, b.perm,
+                                          b.big_list, b.big_count, G);
+  auto big = G.skey_out ? k_bigcell<true> : k_bigcell<false>;
+  big<<<152, kRadixThreads, 0, st>>>(b.big_list, b.big_count, b.cell_count, b.cell_start, b.perm_raw, b.id_raw, b.perm,
+                                     b.tmp_a, b.tmp_b, passes, G);
   return cudaGetLastError();
 }
 
