@@ -340,6 +340,25 @@ CbArgs cb_args(const pbf_handle* h) {
   return A;
 }
 
+// The passes that gather neighbours are bound by the L1 and use no shared
+// memory, so by default they run with whatever split of an SM's 256 KB they
+// find.  Beside a kernel with a large stage on another stream (the network
+// pass of another handle: 179 KB) that left them 28 KB of L1 until the SM ran
+// empty: three learned-start handles of 2^20 particles stepped side by side
+// took 2436 us per frame, 1527 us with the small split asked for (14 %: 32 KB;
+// 0, 7 and 28 % measure the same, 44 % is 6 % slower), one handle alone 1663
+// us either way.  The density pass keeps the default: it has a little shared
+// memory of its own and any request slows it down (73 -> 160 us).
+void prefer_l1(const PassSet& ps) {
+  for (const void* k :
+       {(const void*)ps.predict, (const void*)ps.nbr_build, (const void*)ps.nbr_build2, (const void*)ps.nbr_build_warp,
+        (const void*)ps.nbr_build_feat, (const void*)ps.band, (const void*)ps.boundary_band, (const void*)ps.lambda,
+        (const void*)ps.deltap, (const void*)ps.vorticity, (const void*)ps.xsph, (const void*)ps.vorticity_split,
+        (const void*)ps.xsph_split})
+    if (k && cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 14) != cudaSuccess)
+      cudaGetLastError();  // a hint only
+}
+
 void invalidate_graph(pbf_handle* h) {
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
   h->graph_exec = nullptr;
@@ -1085,6 +1104,7 @@ int apply_launch(pbf_handle* h, const pbf_launch& l) {
   h->blk = (int)l.block;
   h->per_sm = l.ctas_per_sm;
   h->grid_cap = l.ctas_per_sm * (uint32_t)h->sms;
+  if (h->grid_cap) prefer_l1(h->passes.set[h->batch ? 1 : 0][1]);
   return PBF_OK;
 }
 
@@ -1183,6 +1203,7 @@ int pbf_create(const pbf_config* cfg, pbf_handle** out) {
     exact::fill_pass_table(&h->passes);
   else
     fast::fill_pass_table(&h->passes);
+  prefer_l1(h->passes.set[0][0]);
   h->fp = FieldParams{};
   h->fp.loaded = 0;
   cudaError_t e = cudaSuccess;
@@ -2261,6 +2282,7 @@ int pbf_batch_create(const pbf_config* shared, const pbf_scene* scenes, uint32_t
     return code;
   };
   h->batch = true;
+  prefer_l1(h->passes.set[1][0]);
   h->scenes.resize(count);
   h->scene_info.resize(count);
   uint64_t nodes = 0, flags = 0;
