@@ -96,10 +96,14 @@ struct pbf_handle {
   uint32_t nbr_slice = 0;  // list entries per particle (fixed slice)
   uint32_t id_bits = 1;
 
-  cudaGraphExec_t graph_exec = nullptr;
+  // One captured frame per set of buffers it starts from: with an odd number
+  // of substeps a frame ends in the other buffers and two graphs alternate.
+  struct FrameGraph {
+    cudaGraphExec_t exec = nullptr;
+    int cur = 0, count_buf = 0;
+  };
+  FrameGraph graphs[2];
   bool graph_enabled = false;
-  bool graph_valid = false;
-  int graph_cur = 0, graph_count_buf = 0;  // the buffers that the graph starts from
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   uint32_t last_nbr_total = 0;
   // learned start and trace capture
@@ -360,9 +364,10 @@ void prefer_l1(const PassSet& ps) {
 }
 
 void invalidate_graph(pbf_handle* h) {
-  if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
-  h->graph_exec = nullptr;
-  h->graph_valid = false;
+  for (auto& g : h->graphs) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+  }
 }
 
 // Reads and clears the device error word.  A neighbour-list overflow (a
@@ -837,6 +842,32 @@ int frame(pbf_handle* h, uint32_t substeps) {
     if (rc) return rc;
   }
   return exported ? PBF_OK : export_positions(h);
+}
+
+// Records a frame that starts from the current buffers; nothing runs.
+int capture_frame(pbf_handle* h, pbf_handle::FrameGraph* g) {
+  if (!h->count_clear) {  // the frame relies on its counts being clear
+    CU(h, cudaMemsetAsync(h->cell_count[h->count_buf].p, 0, ((size_t)h->gp.cells + 1) * sizeof(uint32_t), h->stream));
+    h->count_clear = true;
+  }
+  const int cur = h->cur, buf = h->count_buf;
+  cudaGraph_t graph = nullptr;
+  CU(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+  const int rc = frame(h, h->cfg.substeps);
+  cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
+  h->cur = cur;
+  h->count_buf = buf;
+  h->count_clear = true;
+  if (rc == PBF_OK && e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, graph, 0);
+  if (graph) cudaGraphDestroy(graph);
+  if (rc) return rc;
+  if (e != cudaSuccess) {
+    g->exec = nullptr;
+    return fail(h, PBF_ECUDA, "graph capture: %s", cudaGetErrorString(e));
+  }
+  g->cur = cur;
+  g->count_buf = buf;
+  return PBF_OK;
 }
 
 // The state after an upload of n particles whose positions (w = 0) and ids
@@ -1674,46 +1705,25 @@ int pbf_step(pbf_handle* h, uint32_t frames) {
     }
     return PBF_OK;
   }
-  // Each substep swaps the state buffers once, so a graph covers an even
-  // number of substeps (one frame, or two frames when substeps is odd) and
-  // every replay starts from the same buffers.
-  const uint32_t per_graph = (h->cfg.substeps % 2 == 0) ? 1u : 2u;
-  if (h->graph_valid && (h->graph_cur != h->cur || h->graph_count_buf != h->count_buf || !h->count_clear))
-    invalidate_graph(h);  // single substeps since the capture left the other buffers current
-  if (!h->graph_valid) {
-    if (!h->count_clear) {  // the graph relies on its counts being clear
-      CU(h, cudaMemsetAsync(h->cell_count[h->count_buf].p, 0, ((size_t)h->gp.cells + 1) * sizeof(uint32_t), h->stream));
-      h->count_clear = true;
+  // Each substep swaps the state and count buffers, so a frame's graph fits
+  // the buffers it was captured from.
+  for (uint32_t f = 0; f < frames; ++f) {
+    pbf_handle::FrameGraph* g = nullptr;
+    for (auto& q : h->graphs)
+      if (q.exec && q.cur == h->cur && q.count_buf == h->count_buf && h->count_clear) g = &q;
+    if (!g) {
+      // single substeps since the last capture may have left other buffers
+      // current than either graph starts from
+      if (h->graphs[0].exec && h->graphs[1].exec) invalidate_graph(h);
+      g = h->graphs[0].exec ? &h->graphs[1] : &h->graphs[0];
+      const int rc = capture_frame(h, g);
+      if (rc) return rc;
     }
-    const int start_cur = h->cur, start_buf = h->count_buf;
-    cudaGraph_t g = nullptr;
-    CU(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = PBF_OK;
-    for (uint32_t f = 0; f < per_graph && rc == PBF_OK; ++f) rc = frame(h, h->cfg.substeps);
-    cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
-    h->cur = start_cur;  // capture only recorded the work
-    h->count_buf = start_buf;
-    h->count_clear = true;
-    if (rc) {
-      if (g) cudaGraphDestroy(g);
-      return rc;
+    CU(h, cudaGraphLaunch(g->exec, h->stream));
+    if (h->cfg.substeps % 2 != 0) {
+      h->cur = 1 - h->cur;
+      h->count_buf = 1 - h->count_buf;
     }
-    if (ce != cudaSuccess) return fail(h, PBF_ECUDA, "graph capture: %s", cudaGetErrorString(ce));
-    ce = cudaGraphInstantiate(&h->graph_exec, g, 0);
-    cudaGraphDestroy(g);
-    if (ce != cudaSuccess) return fail(h, PBF_ECUDA, "graph instantiate: %s", cudaGetErrorString(ce));
-    h->graph_valid = true;
-    h->graph_cur = start_cur;
-    h->graph_count_buf = start_buf;
-  }
-  uint32_t full = frames / per_graph, rest = frames % per_graph;
-  for (uint32_t f = 0; f < full; ++f) CU(h, cudaGraphLaunch(h->graph_exec, h->stream));
-  for (uint32_t f = 0; f < rest; ++f) {
-    // an odd remainder runs eagerly and leaves the buffers swapped: the graph
-    // no longer matches them
-    invalidate_graph(h);
-    int rc = frame(h, h->cfg.substeps);
-    if (rc) return rc;
   }
   return PBF_OK;
 }
