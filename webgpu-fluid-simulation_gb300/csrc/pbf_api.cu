@@ -425,6 +425,7 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   const CbSet& cs = h->passes.cb[cb_memb(h)];
   CbArgs A = cb ? cb_args(h) : CbArgs{};
   const unsigned cbg = cb_grid(n);
+  const bool early = n <= kEarlyMax;
   if (ev) CU(h, cudaEventRecord(ev[0], st));
   // neighborSearch.clearBuffer + TimeIntegration (+ ParticleInsert counts)
   uint32_t* const counts = h->cell_count[h->count_buf].p;
@@ -435,8 +436,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
     const ClearArgs clear{(uint32_t*)h->scan_scratch,
                           (uint32_t)(scan_scratch_bytes((size_t)g.cells + 1) / sizeof(uint32_t)), h->big_count.p,
                           h->band_count.p};
-    ps.predict<<<grid_of(h, n), h->blk, 0, st>>>(p, g, h->tab, h->pos[c].p, h->vel.p, h->acc.p, h->xs[1].p, h->key.p,
-                                                 h->rank.p, counts, clear);
+    launch_chain(early, ps.predict, grid_of(h, n), h->blk, 0, st, p, g, h->tab, h->pos[c].p, h->vel.p, h->acc.p, h->xs[1].p,
+                 h->key.p, h->rank.p, counts, clear);
   }
   CU(h, cudaGetLastError());
   if (ev) CU(h, cudaEventRecord(ev[1], st));
@@ -487,13 +488,12 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
     KScope ks(h, K_BOUNDARY);
     cudaStream_t sst = on ? on : st;
     if (band < 0) {
-      ps.band<<<grid_of(h, n), h->blk, 0, sst>>>(p, h->tab, h->xs[a].p, band_args(0, bsdf));
+      launch_chain(early, ps.band, grid_of(h, n), h->blk, 0, sst, p, h->tab, h->xs[a].p, band_args(0, bsdf));
       band = 0;
     }
-    ps.boundary_band<<<band_grid, 256, 0, sst>>>(p, f, h->sdf.p, h->vol.p, FieldBlocks{h->bcell.p, h->bnodes.p},
-                                                 h->tab, h->xs[a].p, h->bdata.p, bsdf,
-                                                 h->band_list[band].p, h->band_count.p + band,
-                                                 h->band_count.p + (1 - band), guard);
+    launch_chain(early, ps.boundary_band, band_grid, 256, 0, sst, p, f, h->sdf.p, h->vol.p, FieldBlocks{h->bcell.p,
+                 h->bnodes.p}, h->tab, h->xs[a].p, h->bdata.p, bsdf, h->band_list[band].p, h->band_count.p + band,
+                 h->band_count.p + (1 - band), guard);
     return cudaGetLastError();
   };
   // NeighborCount + NeighborList in one pass (fixed per-particle slices: no
@@ -534,9 +534,9 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
       h->passes.cb_build_feat<<<cbg, 128, (size_t)h->cb_cap * sizeof(float4), st>>>(
           p, A, h->cb_mask.p, h->cb_ovf.p, h->nbr_count.p, f.loaded, h->bdata.p, al);
     else
-      ps.nbr_build_feat<<<grid_of(h, n), h->blk, 0, st>>>(p, g, h->xs[0].p, h->cell_start.p, ms, h->nbr_list.p,
-                                                           h->nbr_count.p, h->nbr_max.p, h->err_word.p,
-                                                           (f.loaded && !late) ? 1 : 0, h->bdata.p, al);
+      launch_chain(early, ps.nbr_build_feat, grid_of(h, n), h->blk, 0, st, p, g, h->xs[0].p, h->cell_start.p, ms,
+                   h->nbr_list.p, h->nbr_count.p, h->nbr_max.p, h->err_word.p, (f.loaded && !late) ? 1 : 0,
+                   h->bdata.p, al);
   } else if (cb) {
     // the mask variant's search; the list-free variant has none (the
     // density pass counts the neighbours)
@@ -548,16 +548,14 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   } else {
     KScope ks(h, K_NBR_BUILD);
     if (h->build == PBF_BUILD_PAIR)
-      ps.nbr_build2<<<grid_of(h, (n + 1) / 2), h->blk, 0, st>>>(p, g, h->tab, h->xs[0].p, h->cell_start.p, ms,
-                                                                  h->nbr_list.p, h->nbr_count.p, h->nbr_max.p,
-                                                                  h->err_word.p);
+      launch_chain(early, ps.nbr_build2, grid_of(h, (n + 1) / 2), h->blk, 0, st, p, g, h->tab, h->xs[0].p, h->cell_start.p,
+                   ms, h->nbr_list.p, h->nbr_count.p, h->nbr_max.p, h->err_word.p);
     else if (h->build == PBF_BUILD_WARP)
-      ps.nbr_build_warp<<<grid_of(h, n), h->blk, 0, st>>>(p, g, h->tab, h->xs[0].p, h->cell_start.p, ms,
-                                                           h->nbr_list.p, h->nbr_count.p, h->nbr_max.p,
-                                                           h->err_word.p);
+      launch_chain(early, ps.nbr_build_warp, grid_of(h, n), h->blk, 0, st, p, g, h->tab, h->xs[0].p, h->cell_start.p, ms,
+                   h->nbr_list.p, h->nbr_count.p, h->nbr_max.p, h->err_word.p);
     else
-      ps.nbr_build<<<grid_of(h, n), h->blk, 0, st>>>(p, g, h->tab, h->xs[0].p, h->cell_start.p, ms, h->nbr_list.p,
-                                                      h->nbr_count.p, h->nbr_max.p, h->err_word.p);
+      launch_chain(early, ps.nbr_build, grid_of(h, n), h->blk, 0, st, p, g, h->tab, h->xs[0].p, h->cell_start.p, ms,
+                   h->nbr_list.p, h->nbr_count.p, h->nbr_max.p, h->err_word.p);
   }
   CU(h, cudaGetLastError());
   if (ev) CU(h, cudaEventRecord(ev[2], st));
@@ -615,8 +613,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
           kl<<<cbg, 128, cb_smem(h, 1), st>>>(p, A, f.loaded, h->bdata.p, h->xs[a].p, h->xl.p, al);
         } else {
           auto kl = fe ? ps.lambda_feat : (al.stats && adaptive ? ps.lambda_stats : ps.lambda);
-          kl<<<grid_of(h, n), h->blk, 0, st>>>(p, f.loaded, h->bdata.p, h->xs[a].p, ms, h->nbr_count.p,
-                                               h->nbr_list.p, h->xl.p, al);
+          launch_chain(early, kl, grid_of(h, n), h->blk, 0, st, p, f.loaded, h->bdata.p, h->xs[a].p, ms, h->nbr_count.p,
+                       h->nbr_list.p, h->xl.p, al);
         }
       }
       if (cudaGetLastError() != cudaSuccess) { *rc = PBF_ECUDA; return a; }
@@ -644,8 +642,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
           cs.deltap<<<cbg, 128, cb_smem(h, 1), st>>>(p, A, ad, f.loaded, h->xl.p, h->bdata.p, h->xs[1 - a].p,
                                                      h->capture ? h->dp.p : nullptr);
         else
-          ps.deltap<<<grid_of(h, n), h->blk, 0, st>>>(p, ad, f.loaded, h->xl.p, h->bdata.p, ms, h->nbr_count.p,
-                                                       h->nbr_list.p, h->xs[1 - a].p, h->capture ? h->dp.p : nullptr);
+          launch_chain(early, ps.deltap, grid_of(h, n), h->blk, 0, st, p, ad, f.loaded, h->xl.p, h->bdata.p, ms,
+                       h->nbr_count.p, h->nbr_list.p, h->xs[1 - a].p, h->capture ? h->dp.p : nullptr);
       }
       if (cudaGetLastError() != cudaSuccess) { *rc = PBF_ECUDA; return a; }
       a = 1 - a;
@@ -685,8 +683,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
         cs.deltap<<<cbg, 128, cb_smem(h, 1), st>>>(p, A, ad, f.loaded, h->xs_save.p, h->bdata.p, h->xs[1].p,
                                                    nullptr);
       else
-        ps.deltap<<<grid_of(h, n), h->blk, 0, st>>>(p, ad, f.loaded, h->xs_save.p, h->bdata.p, ms, h->nbr_count.p,
-                                                     h->nbr_list.p, h->xs[1].p, nullptr);
+        launch_chain(early, ps.deltap, grid_of(h, n), h->blk, 0, st, p, ad, f.loaded, h->xs_save.p, h->bdata.p, ms,
+                     h->nbr_count.p, h->nbr_list.p, h->xs[1].p, nullptr);
     }
     CU(h, cudaGetLastError());
     a = iterate(1, h->learned_iters, false, true, false, nullptr, &rc, h->adaptive, h->lagged_fraction > 0.0f);
@@ -714,8 +712,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
       cs.density_velocity<<<cbg, 128, cb_smem(h, 1), st>>>(p, A, ad, h->xs[a].p, h->pos[cc].p, h->vel.p,
                                                             cb_memb(h) == kMemMaskHost ? nullptr : h->nbr_count.p);
     else
-      ps.density_velocity<<<grid_of(h, n), h->blk, 0, st>>>(p, ad, h->xs[a].p, ms, h->nbr_count.p,
-                                                             h->nbr_list.p, h->pos[cc].p, h->vel.p);
+      launch_chain(early, ps.density_velocity, grid_of(h, n), h->blk, 0, st, p, ad, h->xs[a].p, ms, h->nbr_count.p,
+                   h->nbr_list.p, h->pos[cc].p, h->vel.p);
   }
   CU(h, cudaGetLastError());
   if (rec) CU(h, launch_stats_record(h->stats.p, h->trace_err.p, st));
@@ -800,28 +798,27 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   } else if (ps.xsph_split) {  // fast mode: XSPH's sum split over the two passes
     {
       KScope ks(h, K_VORTICITY);
-      ps.vorticity_split<<<grid_of(h, n), h->blk, 0, st>>>(p, h->pos[cc].p, h->vel.p, ms, h->nbr_count.p,
-                                                            h->nbr_list.p, h->omega.p, h->normal.p, h->visc.p,
-                                                            h->coh.p);
+      launch_chain(early, ps.vorticity_split, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->vel.p, ms, h->nbr_count.p,
+                   h->nbr_list.p, h->omega.p, h->normal.p, h->visc.p, h->coh.p);
     }
     CU(h, cudaGetLastError());
     {
       KScope ks(h, K_XSPH);
-      ps.xsph_split<<<grid_of(h, n), h->blk, 0, st>>>(p, h->pos[cc].p, h->omega.p, h->normal.p, h->visc.p, h->coh.p,
-                                                       ms, h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
+      launch_chain(early, ps.xsph_split, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->omega.p, h->normal.p, h->visc.p,
+                   h->coh.p, ms, h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
     }
     CU(h, cudaGetLastError());
   } else {
     {
       KScope ks(h, K_VORTICITY);
-      ps.vorticity<<<grid_of(h, n), h->blk, 0, st>>>(p, h->pos[cc].p, h->vel.p, ms, h->nbr_count.p, h->nbr_list.p,
-                                                      h->omega.p, h->normal.p);
+      launch_chain(early, ps.vorticity, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->vel.p, ms, h->nbr_count.p,
+                   h->nbr_list.p, h->omega.p, h->normal.p);
     }
     CU(h, cudaGetLastError());
     {
       KScope ks(h, K_XSPH);
-      ps.xsph<<<grid_of(h, n), h->blk, 0, st>>>(p, h->pos[cc].p, h->vel.p, h->omega.p, h->normal.p, ms,
-                                                 h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
+      launch_chain(early, ps.xsph, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->vel.p, h->omega.p, h->normal.p, ms,
+                   h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
     }
     CU(h, cudaGetLastError());
   }

@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(256) k_predict(SimParams p0, GridParams g0, Sc
                                                  const float4* __restrict__ acc, float4* __restrict__ xs_out,
                                                  uint32_t* __restrict__ key_out, uint32_t* __restrict__ rank_out,
                                                  uint32_t* cell_count, ClearArgs clear) {
+  chain_begin(pos, vel, acc);
   // scratch of the passes that follow (four memset launches otherwise)
   const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
   for (uint32_t i = i0; i < clear.scan_words; i += gridDim.x * blockDim.x) clear.scan[i] = 0u;
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(256) k_nbr_build(SimParams p, GridParams g0, S
                                                    const uint32_t* __restrict__ cell_start, uint32_t max_nbr,
                                                    uint32_t* __restrict__ nbr_list, uint32_t* __restrict__ nbr_count,
                                                    uint32_t* max_seen, uint32_t* err) {
+  chain_begin(xs, cell_start);
   PBF_TILES(p.n) {
     const uint32_t t = tile0 + threadIdx.x;
     if (t < p.n) {
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(256) k_nbr_build_feat(SimParams p, GridParams 
                                                         uint32_t* __restrict__ nbr_count, uint32_t* max_seen,
                                                         uint32_t* err, int have_field,
                                                         const float4* __restrict__ bdata, SolverAux a) {
+  chain_begin(xs, cell_start, bdata, a.pos, a.lam_prev, a.bsdf);
   PBF_TILES(p.n) {
     const uint32_t t = tile0 + threadIdx.x;
     if (t < p.n) {
@@ -274,6 +277,7 @@ __global__ void __launch_bounds__(256) k_nbr_build2(SimParams p, GridParams g0, 
                                                     const uint32_t* __restrict__ cell_start, uint32_t max_nbr,
                                                     uint32_t* __restrict__ nbr_list, uint32_t* __restrict__ nbr_count,
                                                     uint32_t* max_seen, uint32_t* err) {
+  chain_begin(xs, cell_start);
   const uint32_t npair = (p.n + 1u) >> 1;
   PBF_TILES(npair) {
     const uint32_t k = tile0 + threadIdx.x;
@@ -374,6 +378,7 @@ __global__ void __launch_bounds__(256) k_nbr_build_warp(SimParams p, GridParams 
                                                         uint32_t* __restrict__ nbr_list,
                                                         uint32_t* __restrict__ nbr_count, uint32_t* max_seen,
                                                         uint32_t* err) {
+  chain_begin(xs, cell_start);
   const uint32_t lane = threadIdx.x & 31u;
   PBF_TILES(p.n) {
     const uint32_t t = tile0 + threadIdx.x;
@@ -467,39 +472,63 @@ __device__ __forceinline__ float4 ldo(const float4* p) {  // the slot's own reco
 // entry q at base + 32 q).  Neighbours go in batches of four: the batch's
 // records are gathered, the next batch's indices are requested, then the
 // batch is consumed, so the list read (from DRAM) of one batch overlaps the
-// gathers and arithmetic of the previous one.  List entries are streamed
+// gathers and arithmetic of the previous one.  The last, partial batch's
+// indices are requested the same way and its records gathered together: taken
+// one by one, its up to three entries cost a list read and a gather in turn
+// each, and in most warps some lane has three (16,384 slots, two substeps: 299
+// -> 247 us; at 2^20 the density pass 73 -> 68 us, the others unchanged).
+// kTail = false takes them one by one: the passes whose fn loads a second
+// record itself are faster that way (vorticity at 2^20: 117 against 124 us).
+// List entries are streamed
 // (evict-first): each pass reads the list once, and the records it gathers
 // stay cached.  fn(j, xj) keeps the sequential accumulation order of the
 // reference loop.
-template <bool kC = false, class Fn>
+struct WalkIndex {
+  uint32_t j[4];
+};
+// Indices of the entries [q, q + 4) of a column of cnt entries; slot 0 past the end.
+template <bool kTail>
+__device__ __forceinline__ WalkIndex walk_index(const uint32_t* __restrict__ l, uint32_t q, uint32_t cnt) {
+  WalkIndex w{};
+  if (q + 4u <= cnt) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) w.j[m] = __ldcs(l + 32u * (q + m));
+  } else if constexpr (kTail) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) w.j[m] = q + m < cnt ? __ldcs(l + 32u * (q + m)) : 0u;
+  }
+  return w;
+}
+template <bool kC = false, bool kTail = true, class Fn>
 __device__ __forceinline__ void for_each_neighbor(const uint32_t* __restrict__ list, uint32_t base, uint32_t cnt,
                                                   const float4* xs, Fn&& fn) {
   const uint32_t* l = list + base;
-  const uint32_t full = cnt & ~3u;
+  WalkIndex w = walk_index<kTail>(l, 0u, cnt);
   uint32_t q = 0;
-  if (full) {
-    uint32_t j0 = __ldcs(l), j1 = __ldcs(l + 32), j2 = __ldcs(l + 64), j3 = __ldcs(l + 96);
-    while (true) {
-      const float4 x0 = ldr<kC>(xs + j0), x1 = ldr<kC>(xs + j1), x2 = ldr<kC>(xs + j2), x3 = ldr<kC>(xs + j3);
-      const uint32_t c0 = j0, c1 = j1, c2 = j2, c3 = j3;
-      q += 4;
-      const bool more = q < full;
-      if (more) {
-        j0 = __ldcs(l + 32 * q);
-        j1 = __ldcs(l + 32 * q + 32);
-        j2 = __ldcs(l + 32 * q + 64);
-        j3 = __ldcs(l + 32 * q + 96);
-      }
-      fn(c0, x0);
-      fn(c1, x1);
-      fn(c2, x2);
-      fn(c3, x3);
-      if (!more) break;
-    }
+  while (q + 4u <= cnt) {
+    const WalkIndex c = w;
+    float4 x[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) x[m] = ldr<kC>(xs + c.j[m]);
+    q += 4u;
+    w = walk_index<kTail>(l, q, cnt);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) fn(c.j[m], x[m]);
   }
-  for (; q < cnt; ++q) {
-    uint32_t j = __ldcs(l + 32 * q);
-    fn(j, ldr<kC>(xs + j));
+  if constexpr (kTail) {
+    if (q < cnt) {
+      float4 x[3];
+#pragma unroll
+      for (int m = 0; m < 3; ++m) x[m] = ldr<kC>(xs + w.j[m]);
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+        if (q + m < cnt) fn(w.j[m], x[m]);
+    }
+  } else {
+    for (; q < cnt; ++q) {
+      const uint32_t j = __ldcs(l + 32u * q);
+      fn(j, ldr<kC>(xs + j));
+    }
   }
 }
 
@@ -512,32 +541,31 @@ template <class Fn>
 __device__ __forceinline__ void for_each_neighbor2(const uint32_t* __restrict__ list, uint32_t base, uint32_t cnt,
                                                    const float4* xs, const float4* ys, Fn&& fn) {
   const uint32_t* l = list + base;
-  const uint32_t full = cnt & ~3u;
+  WalkIndex w = walk_index<true>(l, 0u, cnt);
   uint32_t q = 0;
-  if (full) {
-    uint32_t j0 = __ldcs(l), j1 = __ldcs(l + 32), j2 = __ldcs(l + 64), j3 = __ldcs(l + 96);
-    while (true) {
-      const float4 x0 = __ldg(xs + j0), x1 = __ldg(xs + j1), x2 = __ldg(xs + j2), x3 = __ldg(xs + j3);
-      const float4 y0 = __ldg(ys + j0), y1 = __ldg(ys + j1), y2 = __ldg(ys + j2), y3 = __ldg(ys + j3);
-      const uint32_t c0 = j0, c1 = j1, c2 = j2, c3 = j3;
-      q += 4;
-      const bool more = q < full;
-      if (more) {
-        j0 = __ldcs(l + 32 * q);
-        j1 = __ldcs(l + 32 * q + 32);
-        j2 = __ldcs(l + 32 * q + 64);
-        j3 = __ldcs(l + 32 * q + 96);
-      }
-      fn(c0, x0, y0);
-      fn(c1, x1, y1);
-      fn(c2, x2, y2);
-      fn(c3, x3, y3);
-      if (!more) break;
+  while (q + 4u <= cnt) {
+    const WalkIndex c = w;
+    float4 x[4], y[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      x[m] = __ldg(xs + c.j[m]);
+      y[m] = __ldg(ys + c.j[m]);
     }
+    q += 4u;
+    w = walk_index<true>(l, q, cnt);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) fn(c.j[m], x[m], y[m]);
   }
-  for (; q < cnt; ++q) {
-    const uint32_t j = __ldcs(l + 32 * q);
-    fn(j, __ldg(xs + j), __ldg(ys + j));
+  if (q < cnt) {
+    float4 x[3], y[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      x[m] = __ldg(xs + w.j[m]);
+      y[m] = __ldg(ys + w.j[m]);
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+      if (q + m < cnt) fn(w.j[m], x[m], y[m]);
   }
 }
 
@@ -618,6 +646,7 @@ __device__ __forceinline__ void band_mark(const SimParams& p, const BandArgs& B,
 // substep; later ones are marked by delta-p).
 template <bool kBatch, bool kLoop>
 __global__ void __launch_bounds__(256) k_band(SimParams p, SceneTab tab, const float4* __restrict__ xs, BandArgs B) {
+  chain_begin(xs);
   PBF_SLOTS(t, p.n) band_mark<kBatch>(p, B, tab, t, xyz(xs[t]));
 }
 
@@ -633,6 +662,7 @@ __global__ void __launch_bounds__(256, 2) k_boundary_band(SimParams p, FieldPara
                                                           float* __restrict__ bsdf, const uint32_t* __restrict__ list,
                                                           const uint32_t* count, uint32_t* other_count,
                                                           const int* guard) {
+  chain_begin(xs, list, count, guard);
   if (other_count && blockIdx.x == 0 && threadIdx.x == 0) *other_count = 0u;
   if (guard && *guard == 0) return;  // the iteration is skipped (lagged iteration control)
   const uint32_t nb = *count;
@@ -893,6 +923,7 @@ __global__ void __launch_bounds__(256) k_lambda(SimParams p, int have_field, con
                                                 const uint32_t* __restrict__ nbr_cnt,
                                                 const uint32_t* __restrict__ nbr_list,
                                                 float4* __restrict__ xl, SolverAux a) {
+  chain_begin(bdata, xs, nbr_cnt, nbr_list, a.guard, a.pos, a.lam_prev, a.bsdf, a.lam_sum);
   if (a.guard && *a.guard == 0) return;
   // kMode 2: also the density error at these positions into a.stats (the
   // adaptive iteration's test; the same quantity AttributeUpdate reports)
@@ -950,6 +981,7 @@ __global__ void __launch_bounds__(256) k_deltap(SimParams p, SolverAux a, int ha
                                                 uint32_t max_nbr, const uint32_t* __restrict__ nbr_cnt,
                                                 const uint32_t* __restrict__ nbr_list,
                                                 float4* __restrict__ xs_out, float4* __restrict__ dp_out) {
+  chain_begin(xl, bdata, nbr_cnt, nbr_list, a.guard, a.need, a.xs_in);
   if (a.guard && *a.guard == 0) return;
   const bool skip = a.need && *a.need == 0;  // the adaptive test found this iteration unneeded
   PBF_SLOTS(t, p.n) {
@@ -1010,6 +1042,7 @@ __global__ void __launch_bounds__(256) k_density_velocity(SimParams p, SolverAux
                                                           const uint32_t* __restrict__ nbr_cnt,
                                                           const uint32_t* __restrict__ nbr_list,
                                                           float4* __restrict__ pos, float4* __restrict__ vel) {
+  chain_begin(xs, nbr_cnt, nbr_list, a.guard);
   if (a.guard && *a.guard == 0) return;
   unsigned cmax = 0u, csum = 0u, ccnt = 0u;
   PBF_SLOTS(t, p.n) {
@@ -1113,12 +1146,14 @@ __global__ void __launch_bounds__(256) k_vorticity(SimParams p, const float4* __
                                                    const uint32_t* __restrict__ nbr_cnt,
                                                    const uint32_t* __restrict__ nbr_list,
                                                    float4* __restrict__ omega, float4* __restrict__ normal) {
+  chain_begin(pos, vel, nbr_cnt, nbr_list);
   PBF_SLOTS(t, p.n) {
     uint32_t b, e;
     list_slice(max_nbr, nbr_cnt, t, b, e);
     VortSum acc;
     acc.init(xyz(pos[t]), xyz(vel[t]));
-    for_each_neighbor(nbr_list, b, e, pos, [&](uint32_t j, float4 pj) { acc.add(p, pj, __ldg(vel + j)); });
+    for_each_neighbor<false, false>(nbr_list, b, e, pos,
+                                    [&](uint32_t j, float4 pj) { acc.add(p, pj, __ldg(vel + j)); });
     vorticity_finish(p, omega, normal, t, acc);
   }
 }
@@ -1132,6 +1167,7 @@ __global__ void __launch_bounds__(256, 4) k_xsph(SimParams p, const float4* __re
                                                  const uint32_t* __restrict__ nbr_cnt,
                                                  const uint32_t* __restrict__ nbr_list,
                                                  float4* __restrict__ acc, ExportArgs ex) {
+  chain_begin(pos, vel, omega, normal, nbr_cnt, nbr_list, ex.id);
   PBF_SLOTS(t, p.n) {
     uint32_t b, e;
     list_slice(max_nbr, nbr_cnt, t, b, e);
@@ -1139,8 +1175,8 @@ __global__ void __launch_bounds__(256, 4) k_xsph(SimParams p, const float4* __re
     const float4 pi = pos[t];
     if (ex.id) ex.out[ex.id[t]] = pi;
     s.init(pi, xyz(vel[t]), xyz(normal[t]));
-    for_each_neighbor(nbr_list, b, e, pos,
-                      [&](uint32_t j, float4 pj) { s.add(p, pj, __ldg(vel + j), __ldg(normal + j)); });
+    for_each_neighbor<false, false>(
+        nbr_list, b, e, pos, [&](uint32_t j, float4 pj) { s.add(p, pj, __ldg(vel + j), __ldg(normal + j)); });
     xsph_finish(p, acc, t, s, xyz(omega[t]));
   }
 }
@@ -1159,12 +1195,14 @@ __global__ void __launch_bounds__(256, 4) k_vorticity_split(SimParams p, const f
                                                             const uint32_t* __restrict__ nbr_list,
                                                             float4* __restrict__ omega, float4* __restrict__ normal,
                                                             float4* __restrict__ visc, float4* __restrict__ coh_sum) {
+  chain_begin(pos, vel, nbr_cnt, nbr_list);
   PBF_SLOTS(t, p.n) {
     uint32_t b, e;
     list_slice(max_nbr, nbr_cnt, t, b, e);
     VortSplitSum s;
     s.init(pos[t], xyz(vel[t]));
-    for_each_neighbor(nbr_list, b, e, pos, [&](uint32_t j, float4 pj) { s.add(p, pj, __ldg(vel + j)); });
+    for_each_neighbor<false, false>(nbr_list, b, e, pos,
+                                    [&](uint32_t j, float4 pj) { s.add(p, pj, __ldg(vel + j)); });
     vorticity_split_finish(p, omega, normal, visc, coh_sum, t, s);
   }
 }
@@ -1178,6 +1216,7 @@ __global__ void __launch_bounds__(256) k_xsph_split(SimParams p, const float4* _
                                                     const uint32_t* __restrict__ nbr_cnt,
                                                     const uint32_t* __restrict__ nbr_list, float4* __restrict__ acc,
                                                     ExportArgs ex) {
+  chain_begin(pos, omega, normal, visc, coh_sum, nbr_cnt, nbr_list, ex.id);
   PBF_SLOTS(t, p.n) {
     uint32_t b, e;
     list_slice(max_nbr, nbr_cnt, t, b, e);

@@ -76,6 +76,7 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total,
 __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                        size_t n, unsigned long long* status, uint32_t* counter,
                                                        uint32_t* err, uint32_t* __restrict__ zero) {
+  chain_begin(in);
   __shared__ uint32_t s_items[kScanTile + kScanTile / 32];
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_tile;
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(256) k_scatter(uint32_t n, const uint32_t* __r
                                                  const uint32_t* __restrict__ rank, const uint32_t* __restrict__ cell_start,
                                                  const uint32_t* __restrict__ ids, uint32_t* __restrict__ perm_raw,
                                                  uint32_t* __restrict__ id_raw) {
+  chain_begin(key, rank, cell_start, ids);
   uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   uint32_t k = key[s];
@@ -205,6 +207,7 @@ __global__ void __launch_bounds__(256) k_cellfix(uint32_t n, const uint32_t* __r
                                                  const uint32_t* __restrict__ perm_raw,
                                                  const uint32_t* __restrict__ id_raw, uint32_t* __restrict__ perm,
                                                  uint32_t* big_list, uint32_t* big_count, GatherArgs G) {
+  chain_begin(key, cell_count, cell_start, perm_raw, id_raw, G.pos_in, G.xs_in, G.key, G.f_in);
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const uint32_t s = perm_raw[q], my = id_raw[q];
@@ -233,6 +236,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_bigcell(const uint32_t* __res
                                                            uint32_t* __restrict__ perm_raw, uint32_t* __restrict__ id_raw,
                                                            uint32_t* __restrict__ perm, uint32_t* __restrict__ tmp_slot,
                                                            uint32_t* __restrict__ tmp_id, int passes, GatherArgs G) {
+  chain_begin(big_list, big_count, cell_count, cell_start, G.pos_in, G.xs_in, G.key, G.f_in);
   __shared__ uint32_t s_base[256];
   __shared__ uint32_t s_wcount[kRadixThreads / 32][256];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -781,17 +785,16 @@ cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, v
                                   cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const cudaError_t e = cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), st);
-  return e != cudaSuccess ? e : launch_exclusive_scan_cleared(in, out, n, scratch, err, st, nullptr);
+  return e != cudaSuccess ? e : launch_exclusive_scan_cleared(in, out, n, scratch, err, st, nullptr, false);
 }
 
 cudaError_t launch_exclusive_scan_cleared(const uint32_t* in, uint32_t* out, size_t n, void* scratch, uint32_t* err,
-                                          cudaStream_t st, uint32_t* zero) {
+                                          cudaStream_t st, uint32_t* zero, bool early) {
   if (n == 0) return cudaSuccess;
   const size_t tiles = (n + kScanTile - 1) / kScanTile;
   uint32_t* counter = reinterpret_cast<uint32_t*>(scratch);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(scratch) + 256);
-  k_scan<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, status, counter, err, zero);
-  return cudaGetLastError();
+  return launch_chain(early, k_scan, (unsigned)tiles, kScanThreads, 0, st, in, out, n, status, counter, err, zero);
 }
 
 // Self-test of the look-back's bounded wait: one CTA of a two-tile scan,
@@ -828,20 +831,21 @@ cudaError_t launch_scan_timeout_selftest(uint32_t* err, cudaStream_t st) {
 
 cudaError_t launch_sort_by_cell(GridParams g, uint32_t n, const uint32_t* ids, SortBuffers& b, uint32_t id_bits,
                                 const GatherArgs& G, cudaStream_t st) {
-  const cudaError_t e = launch_exclusive_scan_cleared(b.cell_count, b.cell_start, (size_t)g.cells + 1, b.scan_scratch,
-                                                      b.err, st, b.count_next);
+  const bool early = n <= kEarlyMax;
+  cudaError_t e = launch_exclusive_scan_cleared(b.cell_count, b.cell_start, (size_t)g.cells + 1, b.scan_scratch,
+                                                      b.err, st, b.count_next, early);
   if (e != cudaSuccess) return e;
   if (n == 0) return cudaSuccess;
-  k_scatter<<<blocks_for(n, 256), 256, 0, st>>>(n, b.key, b.rank, b.cell_start, ids, b.perm_raw, b.id_raw);
+  e = launch_chain(early, k_scatter, blocks_for(n, 256), 256, 0, st, n, b.key, b.rank, b.cell_start, ids, b.perm_raw, b.id_raw);
+  if (e != cudaSuccess) return e;
   int passes = (int)((id_bits + 7) / 8);
   if (passes < 1) passes = 1;
-  auto fix = G.skey_out ? k_cellfix<true> : k_cellfix<false>;
-  fix<<<blocks_for(n, 256), 256, 0, st>>>(n, b.key, b.cell_count, b.cell_start, b.perm_raw, b.id_raw, b.perm,
-                                          b.big_list, b.big_count, G);
-  auto big = G.skey_out ? k_bigcell<true> : k_bigcell<false>;
-  big<<<152, kRadixThreads, 0, st>>>(b.big_list, b.big_count, b.cell_count, b.cell_start, b.perm_raw, b.id_raw, b.perm,
-                                     b.tmp_a, b.tmp_b, passes, G);
-  return cudaGetLastError();
+  e = launch_chain(early, G.skey_out ? k_cellfix<true> : k_cellfix<false>, blocks_for(n, 256), 256, 0, st, n, b.key,
+                   b.cell_count, b.cell_start, b.perm_raw, b.id_raw, b.perm, b.big_list, b.big_count, G);
+  if (e != cudaSuccess) return e;
+  return launch_chain(early, G.skey_out ? k_bigcell<true> : k_bigcell<false>, 152, kRadixThreads, 0, st, b.big_list,
+                      b.big_count, b.cell_count, b.cell_start, b.perm_raw, b.id_raw, b.perm, b.tmp_a, b.tmp_b, passes,
+                      G);
 }
 
 cudaError_t launch_scatter_by_id(uint32_t n, const uint32_t* id, const float4* src, float4* dst, cudaStream_t st) {
