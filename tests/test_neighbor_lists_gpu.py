@@ -43,3 +43,29 @@ def test_lists_at_the_edges(n, spread):
     assert rc == L.PBF_ECAPACITY and total == want
     assert np.array_equal(off, ref["nbr_offset"])
     assert (lst == 0xffffffff).all()
+
+
+@pytest.mark.parametrize("n", [1, 3072, 3073, 32 * 3072, 32 * 3072 + 1])
+@pytest.mark.parametrize("dims", [(5, 4, 3), (40, 40, 40), (100, 70, 120)])
+def test_search_at_the_tile_edges(n, dims):
+    """One to four radix passes at the edges of a tile and of the range that
+    sorts from the tiles' counts directly; a second search on the same context
+    finds its scratch cleared."""
+    rng = np.random.default_rng(n)
+    cfg = scenes.base_config(kernel_radius=1.0 / max(dims), grid_dim=dims, max_particles=n)
+    ns = None
+    for _ in range(2):
+        pts = np.zeros((n, 4), np.float32)
+        pts[:, :3] = rng.random((n, 3)) ** 2
+        ref = O.neighbor_search(cfg, pts)
+        cells = int(np.prod(dims))
+        if ns is None:
+            ns = NeighborSearch((0.0, 0.0, 0.0), [float(np.float32(d)) for d in dims], dims, n)
+        pos = torch.from_numpy(pts).cuda()
+        out = {k: torch.full((m,), -1, dtype=torch.int32, device="cuda")
+               for k, m in (("keys", n), ("cell_count", cells), ("cell_offset", cells + 1), ("order", n), ("rank", n))}
+        ns.run(pos.data_ptr(), n, *(out[k].data_ptr() for k in ("keys", "cell_count", "cell_offset", "order", "rank")))
+        ns.sync()
+        for k, v in out.items():
+            assert np.array_equal(v.cpu().numpy().view(np.uint32), ref[k]), k
+    ns.close()

@@ -2532,26 +2532,30 @@ int pbf_ns_run(pbf_ns* s, const float* d_pos4, uint32_t n, uint32_t* d_keys, uin
   const bool tm = s->timing;
   s->timed = false;
   if (tm) NSCU(s, cudaEventRecord(s->ev[0], st));
-  NSCU(s, cudaMemsetAsync(s->cell_count.p, 0, ((size_t)g.cells + 1) * 4, st));
   // The points come in particle-id order, so a stable radix sort of the ids
   // by cell key is the counting sort with each cell in id order.  Keys go
-  // straight to the caller's array when it wants them.
+  // straight to the caller's array when it wants them; counts, offsets and
+  // order stay in the context too (pbf_ns_lists), so the kernels that make
+  // them write both.
   uint32_t* key = d_keys ? d_keys : s->key.p;
   uint32_t* const tk[2] = {s->tmp_a.p, s->perm_raw.p};
   uint32_t* const tv[2] = {s->tmp_b.p, s->id_raw.p};
-  NSCU(s, launch_radix_sort_idorder(g, (const float4*)d_pos4, n, key, s->rank.p, s->perm.p, tk, tv, s->radix_scratch,
-                                    s->err_word.p, st, tm ? s->ev[1] : nullptr, s->cell_count.p));
+  if (n) {
+    NSCU(s, launch_radix_sort_idorder(g, (const float4*)d_pos4, n, key, s->rank.p, s->perm.p, d_order, tk, tv,
+                                      s->radix_scratch, s->err_word.p, st, tm ? s->ev[1] : nullptr, s->cell_count.p,
+                                      s->scan_scratch));
+  } else {
+    NSCU(s, cudaMemsetAsync(s->cell_count.p, 0, ((size_t)g.cells + 1) * 4, st));
+    NSCU(s, cudaMemsetAsync(s->scan_scratch, 0, scan_scratch_bytes((size_t)g.cells + 1), st));
+    if (tm) NSCU(s, cudaEventRecord(s->ev[1], st));
+  }
   if (tm) NSCU(s, cudaEventRecord(s->ev[2], st));
-  // offsets from the counts the last pass made (s->rank holds the sorted
-  // keys); the order and offsets stay in the context for pbf_ns_lists
-  NSCU(s, launch_cell_offsets(g.cells, s->cell_count.p, s->cell_start.p, s->scan_scratch, s->err_word.p, st));
+  // offsets from the counts the last pass made (s->rank holds the sorted keys)
+  NSCU(s, launch_exclusive_scan_cleared(s->cell_count.p, s->cell_start.p, (size_t)g.cells + 1, s->scan_scratch,
+                                        s->err_word.p, st, ScanExtra{nullptr, d_cell_count, g.cells, d_cell_offset},
+                                        n <= kEarlyMax));
   if (tm) NSCU(s, cudaEventRecord(s->ev[3], st));
   if (d_rank) NSCU(s, launch_rank_sorted(n, s->rank.p, s->perm.p, s->cell_start.p, d_rank, st));
-  if (d_cell_count)
-    NSCU(s, cudaMemcpyAsync(d_cell_count, s->cell_count.p, (size_t)g.cells * 4, cudaMemcpyDeviceToDevice, st));
-  if (d_cell_offset)
-    NSCU(s, cudaMemcpyAsync(d_cell_offset, s->cell_start.p, ((size_t)g.cells + 1) * 4, cudaMemcpyDeviceToDevice, st));
-  if (d_order && n) NSCU(s, cudaMemcpyAsync(d_order, s->perm.p, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
   if (tm) {
     NSCU(s, cudaEventRecord(s->ev[4], st));
     s->timed = true;
@@ -2586,8 +2590,7 @@ int pbf_ns_lists(pbf_ns* s, const float* d_pos4, uint32_t n, float radius, uint3
   if (!s->sorted.p) NSCU(s, s->sorted.alloc((size_t)s->max_n + kRunPad));
   const float h2 = (float)((double)radius * (double)radius);
   NSCU(s, launch_ns_count(n, s->g, h2, s->perm.p, (const float4*)d_pos4, s->cell_start.p, s->sorted.p, s->nbr_count.p,
-                          st));
-  NSCU(s, launch_exclusive_scan(s->nbr_count.p, d_nbr_offset, (size_t)n + 1, s->scan_scratch, s->err_word.p, st));
+                          d_nbr_offset, s->scan_scratch, s->err_word.p, st));
   uint32_t tot = 0;
   NSCU(s, cudaMemcpyAsync(&tot, d_nbr_offset + n, 4, cudaMemcpyDeviceToHost, st));
   // the kernel itself compares the total with the capacity, so it is queued before the host knows

@@ -116,10 +116,9 @@ size_t scan_scratch_bytes(size_t n);
 // bounded look-back wait gives up.
 cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* scratch, uint32_t* err,
                                   cudaStream_t st);
-// The same with the scratch already cleared by the caller's own kernel; zero
-// (optional): another array of n entries that the scan clears.
+// The same with the scratch already cleared by the caller's own kernel.
 cudaError_t launch_exclusive_scan_cleared(const uint32_t* in, uint32_t* out, size_t n, void* scratch, uint32_t* err,
-                                          cudaStream_t st, uint32_t* zero, bool early);
+                                          cudaStream_t st, const ScanExtra& X, bool early);
 // Self-test of the scan's bounded look-back wait (a predecessor status that
 // nothing writes): *err receives PBF_DEVERR_SCAN_TIMEOUT.
 cudaError_t launch_scan_timeout_selftest(uint32_t* err, cudaStream_t st);
@@ -161,12 +160,12 @@ struct GatherArgs {
 };
 
 // Stable LSD radix sort of points in particle-id order by cell key (the
-// stand-alone search): keys[n] (by id) receive the cell keys, skeys[n] the
-// sorted keys and order[n] the ids in sorted order, stable by id.  tmp_k /
-// tmp_v: two pairs of n-entry scratch arrays; scratch: radix_scratch_bytes(n)
-// bytes.  after_keys (optional) is recorded after the keys.  cell_count
-// (cells + 1 entries, zeroed by the caller) receives the cell counts from the
-// last pass.
+// stand-alone search), n > 0: keys[n] (by id) receive the cell keys, skeys[n]
+// the sorted keys and order[n] (and order2, optional) the ids in sorted order,
+// stable by id.  tmp_k / tmp_v: two pairs of n-entry scratch arrays; scratch:
+// radix_scratch_bytes(n) bytes.  after_keys (optional) is recorded after the
+// keys.  cell_count (cells + 1 entries) receives the cell counts from the last
+// pass and scan_scratch (for a scan of cells + 1) is cleared.
 struct RadixPlan {
   int passes, width;
   size_t tiles;
@@ -174,12 +173,9 @@ struct RadixPlan {
 RadixPlan radix_plan(uint32_t cells, size_t n);
 size_t radix_scratch_bytes(size_t n);
 cudaError_t launch_radix_sort_idorder(GridParams g, const float4* pos, uint32_t n, uint32_t* keys, uint32_t* skeys,
-                                      uint32_t* order, uint32_t* const tmp_k[2], uint32_t* const tmp_v[2],
-                                      void* scratch, uint32_t* err, cudaStream_t st, cudaEvent_t after_keys,
-                                      uint32_t* cell_count);
-// Exclusive offsets (cells + 1 entries) of the cell counts.
-cudaError_t launch_cell_offsets(uint32_t cells, const uint32_t* cell_count, uint32_t* cell_start, void* scan_scratch,
-                                uint32_t* err, cudaStream_t st);
+                                      uint32_t* order, uint32_t* order2, uint32_t* const tmp_k[2],
+                                      uint32_t* const tmp_v[2], void* scratch, uint32_t* err, cudaStream_t st,
+                                      cudaEvent_t after_keys, uint32_t* cell_count, void* scan_scratch);
 // rank_out[order[q]] = q - cell_start[skeys[q]].
 cudaError_t launch_rank_sorted(uint32_t n, const uint32_t* skeys, const uint32_t* order, const uint32_t* cell_start,
                                uint32_t* rank_out, cudaStream_t st);
@@ -192,11 +188,13 @@ cudaError_t launch_scatter_w_by_id(uint32_t n, const uint32_t* id, const float4*
 cudaError_t launch_scatter_by_id_u32(uint32_t n, const uint32_t* id, const uint32_t* src, uint32_t* dst,
                                      cudaStream_t st);
 // Neighbour lists of the stand-alone search (27 cells, |d|^2 <= h2): sorted[t]
-// = (position, id) of order[t] and the neighbour count by particle id (n + 1
-// entries, the last 0); then the lists of neighbour ids at offset[id], the
-// exclusive scan of those counts, written only if offset[n] <= capacity.
+// = (position, id) of order[t], the neighbour count by particle id (n + 1
+// entries, the last 0) and its exclusive scan offset; then the lists of
+// neighbour ids at offset[id], written only if offset[n] <= capacity.  scan:
+// scan_scratch_bytes(n + 1) bytes.
 cudaError_t launch_ns_count(uint32_t n, const GridParams& g, float h2, const uint32_t* order, const float4* pos,
-                            const uint32_t* cell_start, float4* sorted, uint32_t* count, cudaStream_t st);
+                            const uint32_t* cell_start, float4* sorted, uint32_t* count, uint32_t* offset, void* scan,
+                            uint32_t* err, cudaStream_t st);
 cudaError_t launch_ns_list(uint32_t n, const GridParams& g, float h2, const float4* sorted, const uint32_t* cell_start,
                            const uint32_t* offset, uint32_t* list, uint32_t capacity, cudaStream_t st);
 

@@ -2,6 +2,7 @@
 // Host code (pbf_api.cu) fills them from pbf_config; every derived constant
 // is computed in double from the float configuration and rounded once.
 #pragma once
+#include <cstddef>
 #include <cstdint>
 
 namespace pbf {
@@ -70,6 +71,22 @@ struct ClearArgs {
   uint32_t scan_words;
   uint32_t* big_count;
   uint32_t* band_count;
+};
+
+// Scratch cleared by the first kernel of the stand-alone search (words 0: none).
+struct ClearRanges {
+  static constexpr int kRanges = 3;
+  uint32_t* p[kRanges];
+  size_t words[kRanges];
+};
+
+// What the exclusive scan does on the way, each where given: clears zero (as
+// long as its input), copies its first in_copy_n inputs and its result.
+struct ScanExtra {
+  uint32_t* zero;
+  uint32_t* in_copy;
+  size_t in_copy_n;
+  uint32_t* out_copy;
 };
 
 // The by-id positions written by the last pass of a frame (id null: none).

@@ -12,6 +12,7 @@
 // to return; here it is defined as particle-id order (the sequential
 // semantics), which the sort below reproduces exactly whatever order the
 // warp-aggregated atomics ran in.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -71,11 +72,12 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total,
 
 // Single-pass scan: tiles take ids from a counter in launch order, publish
 // their aggregate, look back over predecessors (bounded waits) and publish
-// the inclusive prefix.  Status words pack (flag << 32 | value).  zero
-// (optional, n entries) is cleared along the way.
+// the inclusive prefix.  Status words pack (flag << 32 | value).  Along the
+// way X.zero (n entries) is cleared, X.in_copy receives the first in_copy_n
+// inputs and X.out_copy the result, each where given.
 __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                        size_t n, unsigned long long* status, uint32_t* counter,
-                                                       uint32_t* err, uint32_t* __restrict__ zero) {
+                                                       uint32_t* err, ScanExtra X) {
   chain_begin(in);
   __shared__ uint32_t s_items[kScanTile + kScanTile / 32];
   __shared__ uint32_t s_warp[32];
@@ -90,8 +92,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t* __restric
   for (int k = 0; k < kScanItems; ++k) {
     int li = k * kScanThreads + threadIdx.x;
     size_t gi = base + li;
-    s_items[li + (li >> 5)] = (gi < n) ? __ldg(in + gi) : 0u;
-    if (zero && gi < n) zero[gi] = 0u;
+    const uint32_t v = (gi < n) ? __ldg(in + gi) : 0u;
+    s_items[li + (li >> 5)] = v;
+    if (X.zero && gi < n) X.zero[gi] = 0u;
+    if (X.in_copy && gi < X.in_copy_n) X.in_copy[gi] = v;
   }
   __syncthreads();
   uint32_t items[kScanItems];
@@ -158,7 +162,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t* __restric
   for (int k = 0; k < kScanItems; ++k) {
     int li = k * kScanThreads + threadIdx.x;
     size_t gi = base + li;
-    if (gi < n) out[gi] = s_items[li + (li >> 5)];
+    if (gi < n) {
+      out[gi] = s_items[li + (li >> 5)];
+      if (X.out_copy) X.out_copy[gi] = s_items[li + (li >> 5)];
+    }
   }
 }
 
@@ -310,7 +317,11 @@ __global__ void __launch_bounds__(kRadixThreads) k_bigcell(const uint32_t* __res
 // exclusive scan of that matrix gives each (digit, tile) run its global
 // place; then every tile ranks its records by digit in shared memory (stable
 // in input order) and writes each digit's run there.  Reads and writes are
-// coalesced, and no tile waits on another.
+// coalesced, and no tile waits on another.  The first pass's counts come from
+// the kernel that computes the keys.  Up to kFewTiles tiles the scan is a
+// launch for a few thousand words: every tile then adds up the counts it needs
+// itself, and the previous pass counts the next one's digits where it writes
+// its records (their place says their tile), so a pass is one kernel.
 constexpr int kOsThreads = 256;
 constexpr int kOsItems = 12;
 constexpr int kOsTile = kOsThreads * kOsItems;  // 3072 records per tile
@@ -330,15 +341,55 @@ __device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid) {
   return peers;
 }
 
-// Cell key of every point (ParticleInsert).
-__global__ void __launch_bounds__(256) k_cell_keys(GridParams g, const float4* __restrict__ pos, uint32_t n,
-                                                   uint32_t* __restrict__ key) {
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-    const float4 x = __ldg(pos + s);
-    const int cx = cell_axis(x.x, g.origin[0], g.inv_cell[0], g.dim[0]);
-    const int cy = cell_axis(x.y, g.origin[1], g.inv_cell[1], g.dim[1]);
-    const int cz = cell_axis(x.z, g.origin[2], g.inv_cell[2], g.dim[2]);
-    key[s] = cell_key(cx, cy, cz, g);
+// Up to this many tiles (98,304 points) the passes work from the counts
+// themselves.  A tile reads tiles x 2^width words for it; at 32 tiles that is
+// less than a launch of the scan, at 64 about the same.
+constexpr uint32_t kFewTiles = 32;
+
+// Cell key of every point (ParticleInsert) and the first pass's digit counts
+// of each tile (per-warp counters in shared memory, summed at the end).  The
+// grid may be larger than the tiles: every CTA clears its share of the
+// scratch of the kernels that follow.
+template <int kWidth>
+__global__ void __launch_bounds__(kOsThreads) k_keys_digits(GridParams g, const float4* __restrict__ pos, uint32_t n,
+                                                            uint32_t* __restrict__ key, uint32_t* __restrict__ count,
+                                                            uint32_t tiles, ClearRanges clear) {
+  constexpr uint32_t kRadix = 1u << kWidth, kMask = kRadix - 1u;
+  __shared__ uint32_t s_cnt[kOsWarps][kRadix];
+  chain_begin(pos);
+  const uint32_t tid = threadIdx.x, warp = tid >> 5;
+  for (uint32_t d = tid; d < kOsWarps * kRadix; d += kOsThreads) (&s_cnt[0][0])[d] = 0u;
+#pragma unroll
+  for (int r = 0; r < ClearRanges::kRanges; ++r)
+    for (size_t i = (size_t)blockIdx.x * kOsThreads + tid; i < clear.words[r]; i += (size_t)gridDim.x * kOsThreads)
+      clear.p[r][i] = 0u;
+  if (blockIdx.x >= tiles) return;
+  const uint32_t t0 = blockIdx.x * (uint32_t)kOsTile;
+  uint32_t d[kOsItems];
+#pragma unroll
+  for (int i = 0; i < kOsItems; ++i) {
+    const uint32_t idx = t0 + (uint32_t)i * kOsThreads + tid;
+    d[i] = kRadix;
+    if (idx < n) {
+      const float4 x = __ldg(pos + idx);
+      const int cx = cell_axis(x.x, g.origin[0], g.inv_cell[0], g.dim[0]);
+      const int cy = cell_axis(x.y, g.origin[1], g.inv_cell[1], g.dim[1]);
+      const int cz = cell_axis(x.z, g.origin[2], g.inv_cell[2], g.dim[2]);
+      const uint32_t k = cell_key(cx, cy, cz, g);
+      key[idx] = k;
+      d[i] = k & kMask;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kOsItems; ++i)
+    if (d[i] < kRadix) atomicAdd(&s_cnt[warp][d[i]], 1u);
+  __syncthreads();
+  for (uint32_t dd = tid; dd < kRadix; dd += kOsThreads) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int w = 0; w < kOsWarps; ++w) c += s_cnt[w][dd];
+    count[(size_t)dd * tiles + blockIdx.x] = c;
   }
 }
 
@@ -347,6 +398,7 @@ __global__ void __launch_bounds__(256) k_cell_keys(GridParams g, const float4* _
 template <int kWidth>
 __global__ void __launch_bounds__(kOsThreads) k_tile_digits(uint32_t n, const uint32_t* __restrict__ kin,
                                                             uint32_t* __restrict__ count, uint32_t tiles, int shift) {
+  chain_begin(kin);
   constexpr uint32_t kRadix = 1u << kWidth, kMask = kRadix - 1u;
   __shared__ uint32_t s_cnt[kOsWarps][kRadix];
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
@@ -375,23 +427,42 @@ __global__ void __launch_bounds__(kOsThreads) k_tile_digits(uint32_t n, const ui
 // tile] is where the tile's run of digit d starts.  vin == nullptr: the values
 // are the input positions (particle ids).  cell_count (the last pass only):
 // the written keys are in final order, so each run of equal keys a warp
-// writes is added to its cell's count once.
-template <int kWidth>
+// writes is added to its cell's count once; vout2 (optional) receives the
+// values too.  kFew: place holds the tiles' digit counts instead (at most
+// kFewTiles tiles), and next_count (optional, cleared) receives those of the
+// next pass.
+template <int kWidth, bool kFew>
 __global__ void __launch_bounds__(kOsThreads, 4) k_radix_pass(uint32_t n, const uint32_t* __restrict__ kin,
                                                               const uint32_t* __restrict__ vin,
                                                               uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
                                                               const uint32_t* __restrict__ place, uint32_t tiles,
-                                                              int shift, uint32_t* cell_count) {
+                                                              int shift, uint32_t* cell_count,
+                                                              uint32_t* __restrict__ vout2, uint32_t* next_count) {
   constexpr uint32_t kRadix = 1u << kWidth, kMask = kRadix - 1u;
   __shared__ uint32_t s_key[kOsTile];
   __shared__ uint32_t s_val[kOsTile];
   __shared__ uint32_t s_wcnt[kOsWarps][kRadix];  // per-warp digit counts, then offsets over warps
   __shared__ uint32_t s_loc[kRadix];             // digit counts of the tile, then their exclusive scan
   __shared__ uint32_t s_glob[kRadix];            // global place of the tile's first record of each digit
+  chain_begin(kin, vin, place);
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t tile = blockIdx.x;
   for (uint32_t i = tid; i < kOsWarps * kRadix; i += kOsThreads) (&s_wcnt[0][0])[i] = 0u;
-  for (uint32_t d = tid; d < kRadix; d += kOsThreads) s_glob[d] = __ldg(place + (size_t)d * tiles + tile);
+  if constexpr (kFew) {
+    // the digit's records in all tiles, and in the tiles before this one
+    __shared__ uint32_t s_warp[32];
+    uint32_t all = 0u, before = 0u, total;
+    if (tid < kRadix)
+      for (uint32_t t = 0; t < tiles; ++t) {
+        const uint32_t c = __ldg(place + (size_t)tid * tiles + t);
+        all += c;
+        before += t < tile ? c : 0u;
+      }
+    const uint32_t base = block_exclusive(all, &total, s_warp);
+    if (tid < kRadix) s_glob[tid] = base + before;
+  } else {
+    for (uint32_t d = tid; d < kRadix; d += kOsThreads) s_glob[d] = __ldg(place + (size_t)d * tiles + tile);
+  }
   const uint32_t t0 = tile * (uint32_t)kOsTile;
   // warp w holds records t0 + 512 w .. + 511; round i is records 32 i .. 32 i + 31 of it
   const uint32_t w0 = t0 + warp * (32u * kOsItems) + lane;
@@ -481,8 +552,12 @@ __global__ void __launch_bounds__(kOsThreads, 4) k_radix_pass(uint32_t n, const 
       const uint32_t d = (kk >> shift) & kMask;
       const uint32_t p = s_glob[d] + (j - s_loc[d]);
       if (p < n) {
+        const uint32_t v = s_val[j];
         kout[p] = kk;
-        vout[p] = s_val[j];
+        vout[p] = v;
+        if (vout2) vout2[p] = v;
+        if constexpr (kFew)
+          if (next_count) atomicAdd(next_count + (size_t)((kk >> (shift + kWidth)) & kMask) * tiles + p / kOsTile, 1u);
       }
     }
     if (cell_count) {  // a warp's 32 consecutive records: one add per run of equal keys
@@ -506,6 +581,7 @@ __global__ void __launch_bounds__(256) k_rank_sorted(uint32_t n, const uint32_t*
                                                      const uint32_t* __restrict__ order,
                                                      const uint32_t* __restrict__ cell_start,
                                                      uint32_t* __restrict__ rank_out) {
+  chain_begin(skey, order, cell_start);
   const uint32_t q0 = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
   if (q0 >= n) return;
   if (q0 + 4u <= n) {
@@ -546,8 +622,11 @@ __global__ void k_scatter_u32(uint32_t n, const uint32_t* __restrict__ id, const
 // particle id in w, so the traversals read coalesced candidates and the list
 // kernel has a neighbour's id at hand.
 __global__ void __launch_bounds__(256) k_ns_sorted(uint32_t n, const uint32_t* __restrict__ order,
-                                                   const float4* __restrict__ pos, float4* __restrict__ sorted) {
+                                                   const float4* __restrict__ pos, float4* __restrict__ sorted,
+                                                   uint32_t* __restrict__ scan, uint32_t scan_words) {
+  chain_begin(order, pos);
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  for (uint32_t i = t; i < scan_words; i += gridDim.x * blockDim.x) scan[i] = 0u;  // of the scan between the traversals
   if (t >= n) return;
   const uint32_t o = order[t];
   float4 x = __ldg(pos + o);
@@ -573,6 +652,7 @@ __global__ void __launch_bounds__(128) k_ns_count(uint32_t n, GridParams g, floa
                                                   const float4* __restrict__ sorted,
                                                   const uint32_t* __restrict__ cell_start,
                                                   uint32_t* __restrict__ count) {
+  chain_begin(sorted, cell_start);
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t == n) count[n] = 0u;
   if (t >= n) return;
@@ -595,6 +675,7 @@ __global__ void __launch_bounds__(32 * kListWarps) k_ns_list(uint32_t n, GridPar
                                                              const uint32_t* __restrict__ offset,
                                                              uint32_t* __restrict__ list, uint32_t capacity) {
   __shared__ uint32_t s_rows[kListWarps][kListRows * 33u];
+  chain_begin(sorted, cell_start, offset);
   if (__ldg(offset + n) > capacity) return;
   const uint32_t lane = threadIdx.x & 31u, t = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t* rows = s_rows[threadIdx.x >> 5];
@@ -701,31 +782,45 @@ namespace {
 size_t round256(size_t b) { return (b + 255) / 256 * 256; }
 }  // namespace
 
-// Scratch: the digit-major count matrix, its scan and the scan's own scratch.
+// Scratch: the digit-major count matrix, its scan and one scan scratch per
+// pass; or, with few tiles, one count matrix per pass.
+constexpr int kMaxPasses = 4;
 size_t radix_scratch_bytes(size_t n) {
   size_t tiles = (n + kOsTile - 1) / kOsTile;
   if (tiles == 0) tiles = 1;
   const size_t m = tiles * kOsMaxRadix;
-  return 2 * round256(m * sizeof(uint32_t)) + scan_scratch_bytes(m);
+  const size_t many = 2 * round256(m * sizeof(uint32_t)) + kMaxPasses * round256(scan_scratch_bytes(m));
+  const size_t few = kMaxPasses * (size_t)kFewTiles * kOsMaxRadix * sizeof(uint32_t);
+  return many > few ? many : few;
 }
 
-cudaError_t launch_radix_sort_idorder(GridParams g, const float4* pos, uint32_t n, uint32_t* keys, uint32_t* skeys,
-                                      uint32_t* order, uint32_t* const tmp_k[2], uint32_t* const tmp_v[2],
-                                      void* scratch, uint32_t* err, cudaStream_t st, cudaEvent_t after_keys,
-                                      uint32_t* cell_count) {
-  cudaError_t e = cudaSuccess;
-  if (n == 0) return after_keys ? cudaEventRecord(after_keys, st) : cudaSuccess;
-  const RadixPlan plan = radix_plan(g.cells, n);
-  const uint32_t radix = 1u << plan.width;
-  const size_t m = plan.tiles * radix;
-  char* sc = reinterpret_cast<char*>(scratch);
+namespace {
+template <int W>
+cudaError_t radix_sort(const GridParams& g, const float4* pos, uint32_t n, const RadixPlan& plan, uint32_t* keys,
+                       uint32_t* skeys, uint32_t* order, uint32_t* order2, uint32_t* const tmp_k[2],
+                       uint32_t* const tmp_v[2], char* sc, uint32_t* err, cudaStream_t st, cudaEvent_t after_keys,
+                       uint32_t* cell_count, uint32_t* scan_scratch) {
+  constexpr uint32_t kRadix = 1u << W;
+  const uint32_t tiles = (uint32_t)plan.tiles;
+  const bool few = tiles <= kFewTiles, early = n <= kEarlyMax;
+  const size_t m = plan.tiles * kRadix;
   uint32_t* count = reinterpret_cast<uint32_t*>(sc);
-  uint32_t* place = reinterpret_cast<uint32_t*>(sc + round256(plan.tiles * kOsMaxRadix * sizeof(uint32_t)));
-  void* scan_scr = sc + 2 * round256(plan.tiles * kOsMaxRadix * sizeof(uint32_t));
-  unsigned blocks = (unsigned)((n + 255) / 256);
-  if (blocks > 152u * 8u) blocks = 152u * 8u;
-  k_cell_keys<<<blocks, 256, 0, st>>>(g, pos, n, keys);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  uint32_t* place = reinterpret_cast<uint32_t*>(sc + round256(m * sizeof(uint32_t)));
+  char* scans = sc + 2 * round256(m * sizeof(uint32_t));
+  const size_t scan_bytes = round256(scan_scratch_bytes(m));
+  ClearRanges clear{};
+  clear.p[0] = cell_count;
+  clear.words[0] = (size_t)g.cells + 1;
+  clear.p[1] = scan_scratch;
+  clear.words[1] = scan_scratch_bytes((size_t)g.cells + 1) / sizeof(uint32_t);
+  // few: the later passes' counts are added up in place; else the scans' scratch
+  clear.p[2] = few ? count + m : reinterpret_cast<uint32_t*>(scans);
+  clear.words[2] = few ? (size_t)(plan.passes - 1) * m : (size_t)plan.passes * scan_bytes / sizeof(uint32_t);
+  // enough CTAs that clearing the cells does not hang on a few of them
+  const size_t clearing = std::min<size_t>((clear.words[0] + 4095) / 4096, 152u * 8u);
+  cudaError_t e = launch_chain(early, k_keys_digits<W>, (unsigned)std::max<size_t>(tiles, clearing), kOsThreads, 0, st, g,
+                               pos, n, keys, count, tiles, clear);
+  if (e != cudaSuccess) return e;
   if (after_keys && (e = cudaEventRecord(after_keys, st)) != cudaSuccess) return e;
   for (int p = 0; p < plan.passes; ++p) {
     const bool last = p == plan.passes - 1;
@@ -733,46 +828,59 @@ cudaError_t launch_radix_sort_idorder(GridParams g, const float4* pos, uint32_t 
     const uint32_t* vin = p == 0 ? nullptr : tmp_v[(p - 1) & 1];
     uint32_t* kout = last ? skeys : tmp_k[p & 1];
     uint32_t* vout = last ? order : tmp_v[p & 1];
-    const int shift = p * plan.width;
-    const unsigned grid = (unsigned)plan.tiles;
-    const uint32_t tl = (uint32_t)plan.tiles;
-    switch (plan.width) {
-#define PBF_RADIX_WIDTH(W)                                                              \
-  case W:                                                                               \
-    k_tile_digits<W><<<grid, kOsThreads, 0, st>>>(n, kin, count, tl, shift);            \
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;                              \
-    if ((e = launch_exclusive_scan(count, place, m, scan_scr, err, st)) != cudaSuccess) \
-      return e;                                                                         \
-    k_radix_pass<W><<<grid, kOsThreads, 0, st>>>(n, kin, vin, kout, vout, place, tl, shift, last ? cell_count : nullptr); \
-    break;
-      PBF_RADIX_WIDTH(1)
-      PBF_RADIX_WIDTH(2)
-      PBF_RADIX_WIDTH(3)
-      PBF_RADIX_WIDTH(4)
-      PBF_RADIX_WIDTH(5)
-      PBF_RADIX_WIDTH(6)
-      PBF_RADIX_WIDTH(7)
-      PBF_RADIX_WIDTH(8)
-#undef PBF_RADIX_WIDTH
-      default:
-        return cudaErrorInvalidValue;
+    uint32_t* cc = last ? cell_count : nullptr;
+    uint32_t* v2 = last ? order2 : nullptr;
+    const int shift = p * W;
+    if (few) {
+      uint32_t* c = count + (size_t)p * m;
+      e = launch_chain(early, k_radix_pass<W, true>, tiles, kOsThreads, 0, st, n, kin, vin, kout, vout, c, tiles, shift,
+                       cc, v2, last ? nullptr : c + m);
+    } else {
+      if (p > 0) {
+        e = launch_chain(early, k_tile_digits<W>, tiles, kOsThreads, 0, st, n, kin, count, tiles, shift);
+        if (e != cudaSuccess) return e;
+      }
+      e = launch_exclusive_scan_cleared(count, place, m, scans + (size_t)p * scan_bytes, err, st, ScanExtra{}, early);
+      if (e != cudaSuccess) return e;
+      e = launch_chain(early, k_radix_pass<W, false>, tiles, kOsThreads, 0, st, n, kin, vin, kout, vout, place, tiles,
+                       shift, cc, v2, nullptr);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
+}  // namespace
 
-cudaError_t launch_cell_offsets(uint32_t cells, const uint32_t* cell_count, uint32_t* cell_start, void* scan_scratch,
-                                uint32_t* err, cudaStream_t st) {
-  return launch_exclusive_scan(cell_count, cell_start, (size_t)cells + 1, scan_scratch, err, st);
+cudaError_t launch_radix_sort_idorder(GridParams g, const float4* pos, uint32_t n, uint32_t* keys, uint32_t* skeys,
+                                      uint32_t* order, uint32_t* order2, uint32_t* const tmp_k[2],
+                                      uint32_t* const tmp_v[2], void* scratch, uint32_t* err, cudaStream_t st,
+                                      cudaEvent_t after_keys, uint32_t* cell_count, void* scan_scratch) {
+  const RadixPlan plan = radix_plan(g.cells, n);
+  switch (plan.width) {
+#define PBF_RADIX_WIDTH(W)                                                                                        \
+  case W:                                                                                                         \
+    return radix_sort<W>(g, pos, n, plan, keys, skeys, order, order2, tmp_k, tmp_v, reinterpret_cast<char*>(scratch), \
+                         err, st, after_keys, cell_count, reinterpret_cast<uint32_t*>(scan_scratch));
+    PBF_RADIX_WIDTH(1)
+    PBF_RADIX_WIDTH(2)
+    PBF_RADIX_WIDTH(3)
+    PBF_RADIX_WIDTH(4)
+    PBF_RADIX_WIDTH(5)
+    PBF_RADIX_WIDTH(6)
+    PBF_RADIX_WIDTH(7)
+    PBF_RADIX_WIDTH(8)
+#undef PBF_RADIX_WIDTH
+    default:
+      return cudaErrorInvalidValue;
+  }
 }
 
 cudaError_t launch_rank_sorted(uint32_t n, const uint32_t* skeys, const uint32_t* order, const uint32_t* cell_start,
                                uint32_t* rank_out, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const uint32_t threads = (n + 3u) / 4u;
-  k_rank_sorted<<<(threads + 255u) / 256u, 256, 0, st>>>(n, skeys, order, cell_start, rank_out);
-  return cudaGetLastError();
+  return launch_chain(n <= kEarlyMax, k_rank_sorted, (threads + 255u) / 256u, 256, 0, st, n, skeys, order, cell_start,
+                      rank_out);
 }
 
 size_t scan_scratch_bytes(size_t n) {
@@ -785,16 +893,16 @@ cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, v
                                   cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const cudaError_t e = cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), st);
-  return e != cudaSuccess ? e : launch_exclusive_scan_cleared(in, out, n, scratch, err, st, nullptr, false);
+  return e != cudaSuccess ? e : launch_exclusive_scan_cleared(in, out, n, scratch, err, st, ScanExtra{}, false);
 }
 
 cudaError_t launch_exclusive_scan_cleared(const uint32_t* in, uint32_t* out, size_t n, void* scratch, uint32_t* err,
-                                          cudaStream_t st, uint32_t* zero, bool early) {
+                                          cudaStream_t st, const ScanExtra& X, bool early) {
   if (n == 0) return cudaSuccess;
   const size_t tiles = (n + kScanTile - 1) / kScanTile;
   uint32_t* counter = reinterpret_cast<uint32_t*>(scratch);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(scratch) + 256);
-  return launch_chain(early, k_scan, (unsigned)tiles, kScanThreads, 0, st, in, out, n, status, counter, err, zero);
+  return launch_chain(early, k_scan, (unsigned)tiles, kScanThreads, 0, st, in, out, n, status, counter, err, X);
 }
 
 // Self-test of the look-back's bounded wait: one CTA of a two-tile scan,
@@ -816,7 +924,7 @@ cudaError_t launch_scan_timeout_selftest(uint32_t* err, cudaStream_t st) {
   if (e == cudaSuccess) e = cudaMemcpyAsync(counter, &one, sizeof(one), cudaMemcpyHostToDevice, st);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(scratch) + 256);
   if (e == cudaSuccess) {
-    k_scan<<<1, kScanThreads, 0, st>>>(in, out, n, status, counter, err, nullptr);
+    k_scan<<<1, kScanThreads, 0, st>>>(in, out, n, status, counter, err, ScanExtra{});
     e = cudaGetLastError();
   }
   // the host value copied above must outlive the copy
@@ -833,7 +941,7 @@ cudaError_t launch_sort_by_cell(GridParams g, uint32_t n, const uint32_t* ids, S
                                 const GatherArgs& G, cudaStream_t st) {
   const bool early = n <= kEarlyMax;
   cudaError_t e = launch_exclusive_scan_cleared(b.cell_count, b.cell_start, (size_t)g.cells + 1, b.scan_scratch,
-                                                      b.err, st, b.count_next, early);
+                                                      b.err, st, ScanExtra{b.count_next}, early);
   if (e != cudaSuccess) return e;
   if (n == 0) return cudaSuccess;
   e = launch_chain(early, k_scatter, blocks_for(n, 256), 256, 0, st, n, b.key, b.rank, b.cell_start, ids, b.perm_raw, b.id_raw);
@@ -865,17 +973,23 @@ cudaError_t launch_scatter_by_id_u32(uint32_t n, const uint32_t* id, const uint3
   return cudaGetLastError();
 }
 cudaError_t launch_ns_count(uint32_t n, const GridParams& g, float h2, const uint32_t* order, const float4* pos,
-                            const uint32_t* cell_start, float4* sorted, uint32_t* count, cudaStream_t st) {
-  if (n) k_ns_sorted<<<blocks_for(n, 256), 256, 0, st>>>(n, order, pos, sorted);
-  k_ns_count<<<blocks_for((size_t)n + 1, 128), 128, 0, st>>>(n, g, h2, sorted, cell_start, count);
-  return cudaGetLastError();
+                            const uint32_t* cell_start, float4* sorted, uint32_t* count, uint32_t* offset, void* scan,
+                            uint32_t* err, cudaStream_t st) {
+  const bool early = n <= kEarlyMax;
+  const size_t m = (size_t)n + 1;
+  cudaError_t e = launch_chain(early, k_ns_sorted, blocks_for(m, 256), 256, 0, st, n, order, pos, sorted,
+                               reinterpret_cast<uint32_t*>(scan), (uint32_t)(scan_scratch_bytes(m) / sizeof(uint32_t)));
+  if (e != cudaSuccess) return e;
+  e = launch_chain(early, k_ns_count, blocks_for(m, 128), 128, 0, st, n, g, h2, sorted, cell_start, count);
+  if (e != cudaSuccess) return e;
+  return launch_exclusive_scan_cleared(count, offset, m, scan, err, st, ScanExtra{}, early);
 }
 cudaError_t launch_ns_list(uint32_t n, const GridParams& g, float h2, const float4* sorted, const uint32_t* cell_start,
                            const uint32_t* offset, uint32_t* list, uint32_t capacity, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_ns_list<<<blocks_for(n, 32 * kListWarps), 32 * kListWarps, 0, st>>>(n, g, h2, sorted, cell_start, offset, list,
-                                                                       capacity);
-  return cudaGetLastError();
+  // an ordinary launch: the total is read back between the scan and this kernel
+  return launch_chain(false, k_ns_list, blocks_for(n, 32 * kListWarps), 32 * kListWarps, 0, st, n, g, h2, sorted,
+                      cell_start, offset, list, capacity);
 }
 cudaError_t launch_metrics(SimParams p, FieldParams f, const float* sdf, const float4* pos, const float4* vel,
                            const uint32_t* nbr_count, uint32_t n, float* accum_f, double* accum_d, uint32_t* accum_u,
