@@ -2587,7 +2587,7 @@ int pbf_ns_lists(pbf_ns* s, const float* d_pos4, uint32_t n, float radius, uint3
   if (n > s->max_n) return nsfail(s, PBF_ECAPACITY, "too many particles for this search context");
   cudaStream_t st = s->stream;
   // the sorted positions' workspace: allocated by the first call, kept with the context
-  if (!s->sorted.p) NSCU(s, s->sorted.alloc((size_t)s->max_n + kRunPad));
+  if (!s->sorted.p) NSCU(s, s->sorted.alloc(s->max_n));
   const float h2 = (float)((double)radius * (double)radius);
   NSCU(s, launch_ns_count(n, s->g, h2, s->perm.p, (const float4*)d_pos4, s->cell_start.p, s->sorted.p, s->nbr_count.p,
                           d_nbr_offset, s->scan_scratch, s->err_word.p, st));

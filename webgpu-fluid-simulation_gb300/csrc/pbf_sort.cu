@@ -619,8 +619,8 @@ __global__ void k_scatter_u32(uint32_t n, const uint32_t* __restrict__ id, const
 // ---- neighbour lists in the reference layout (stand-alone search) -------------------
 // NeighborCount + NeighborList (neighborShader.ts:101-246) in two traversals
 // of the 27 cells.  The positions go into sorted order once, each with its
-// particle id in w, so the traversals read coalesced candidates and the list
-// kernel has a neighbour's id at hand.
+// particle id in w, so the traversals read neighbouring candidates and the
+// list kernel has a neighbour's id at hand.
 __global__ void __launch_bounds__(256) k_ns_sorted(uint32_t n, const uint32_t* __restrict__ order,
                                                    const float4* __restrict__ pos, float4* __restrict__ sorted,
                                                    uint32_t* __restrict__ scan, uint32_t scan_words) {
@@ -634,16 +634,29 @@ __global__ void __launch_bounds__(256) k_ns_sorted(uint32_t n, const uint32_t* _
   sorted[t] = x;
 }
 
-template <class Hits>
+// each(in, id): every candidate in order, in: whether it is a neighbour.  Four
+// loads in flight; the last group of a run repeats its last candidate.
+template <class Each>
 __device__ __forceinline__ void test_cells27(const GridParams& g, const uint32_t* __restrict__ cell_start,
-                                             const float4* __restrict__ sorted, f3 xi, float h2, Hits&& hits) {
+                                             const float4* __restrict__ sorted, f3 xi, float h2, Each&& each) {
   const int cx = cell_axis(xi.x, g.origin[0], g.inv_cell[0], g.dim[0]);
   const int cy = cell_axis(xi.y, g.origin[1], g.inv_cell[1], g.dim[1]);
   const int cz = cell_axis(xi.z, g.origin[2], g.inv_cell[2], g.dim[2]);
   for (int dx = -1; dx <= 1; ++dx)
     for (int dy = -1; dy <= 1; ++dy) {
       const Run r = run_of(g, cell_start, cx, cy, cz, dx, dy);
-      test_run(sorted, r.b, r.e, xi, h2, hits);
+      uint32_t u = r.b;
+      for (; u + 4u <= r.e; u += 4u) {
+        float4 c[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) c[m] = __ldg(sorted + u + m);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) each(dist2_rn(xyz(c[m]) - xi) <= h2, __float_as_uint(c[m].w));
+      }
+      for (; u < r.e; ++u) {
+        const float4 c = __ldg(sorted + u);
+        each(dist2_rn(xyz(c) - xi) <= h2, __float_as_uint(c.w));
+      }
     }
 }
 
@@ -658,47 +671,25 @@ __global__ void __launch_bounds__(128) k_ns_count(uint32_t n, GridParams g, floa
   if (t >= n) return;
   const float4 x = sorted[t];
   uint32_t c = 0;
-  test_cells27(g, cell_start, sorted, xyz(x), h2, [&](uint32_t, unsigned mask) { c += (uint32_t)__popc(mask); });
+  test_cells27(g, cell_start, sorted, xyz(x), h2, [&](bool in, uint32_t) { c += in ? 1u : 0u; });
   count[__float_as_uint(x.w)] = c;
 }
 
 // The lists, written only if they all fit (offset[n] <= capacity).  A thread
-// finds one particle's neighbours; its warp keeps the first kListRows of each
-// lane in shared memory (row q, lane l at 33 q + l: both sides free of bank
-// conflicts) and then writes each particle's run with all lanes, coalesced.
-// Neighbours past kListRows go straight to global memory.
-constexpr uint32_t kListRows = 48;
-constexpr uint32_t kListWarps = 4;
-__global__ void __launch_bounds__(32 * kListWarps) k_ns_list(uint32_t n, GridParams g, float h2,
-                                                             const float4* __restrict__ sorted,
-                                                             const uint32_t* __restrict__ cell_start,
-                                                             const uint32_t* __restrict__ offset,
-                                                             uint32_t* __restrict__ list, uint32_t capacity) {
-  __shared__ uint32_t s_rows[kListWarps][kListRows * 33u];
+// writes its particle's run as it finds it: the id arrives with the candidate.
+__global__ void __launch_bounds__(128) k_ns_list(uint32_t n, GridParams g, float h2,
+                                                 const float4* __restrict__ sorted,
+                                                 const uint32_t* __restrict__ cell_start,
+                                                 const uint32_t* __restrict__ offset, uint32_t* __restrict__ list,
+                                                 uint32_t capacity) {
   chain_begin(sorted, cell_start, offset);
-  if (__ldg(offset + n) > capacity) return;
-  const uint32_t lane = threadIdx.x & 31u, t = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t* rows = s_rows[threadIdx.x >> 5];
-  uint32_t q = 0, at = 0;
-  if (t < n) {
-    const float4 x = sorted[t];
-    at = __ldg(offset + __float_as_uint(x.w));
-    test_cells27(g, cell_start, sorted, xyz(x), h2, [&](uint32_t u0, unsigned mask) {
-      for_each_hit(u0, mask, [&](uint32_t u) {
-        const uint32_t id = __float_as_uint(__ldg(&sorted[u].w));
-        if (q < kListRows)
-          rows[33u * q + lane] = id;
-        else
-          list[at + q] = id;
-        ++q;
-      });
-    });
-  }
-  __syncwarp();
-  for (int p = 0; p < 32; ++p) {
-    const uint32_t cnt = min(__shfl_sync(kFull, q, p), kListRows), to = __shfl_sync(kFull, at, p);
-    for (uint32_t r = lane; r < cnt; r += 32u) list[to + r] = rows[33u * r + (uint32_t)p];
-  }
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n || __ldg(offset + n) > capacity) return;
+  const float4 x = sorted[t];
+  uint32_t* out = list + __ldg(offset + __float_as_uint(x.w));
+  test_cells27(g, cell_start, sorted, xyz(x), h2, [&](bool in, uint32_t id) {
+    if (in) *out++ = id;
+  });
 }
 
 // ---- metrics --------------------------------------------------------------------------
@@ -988,7 +979,7 @@ cudaError_t launch_ns_list(uint32_t n, const GridParams& g, float h2, const floa
                            const uint32_t* offset, uint32_t* list, uint32_t capacity, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   // an ordinary launch: the total is read back between the scan and this kernel
-  return launch_chain(false, k_ns_list, blocks_for(n, 32 * kListWarps), 32 * kListWarps, 0, st, n, g, h2, sorted,
+  return launch_chain(false, k_ns_list, blocks_for(n, 128), 128, 0, st, n, g, h2, sorted,
                       cell_start, offset, list, capacity);
 }
 cudaError_t launch_metrics(SimParams p, FieldParams f, const float* sdf, const float4* pos, const float4* vel,
