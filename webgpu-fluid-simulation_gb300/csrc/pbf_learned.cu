@@ -301,10 +301,17 @@ __global__ void __launch_bounds__(32 * kTrainWarps) k_mlp_grad(const float* __re
   }
 }
 
-// Adam (Kingma & Ba 2015) on the flat FP32 parameters.
-__global__ void k_adam(float* __restrict__ P, const float* __restrict__ G, float* __restrict__ M, float* __restrict__ V,
-                       int n, float lr, float b1, float b2, float eps, float c1, float c2) {
+// Adam (Kingma & Ba 2015) on the flat FP32 parameters.  Also hands the batch's
+// loss over and clears gradient and loss for the next batch (a memset between
+// the batches otherwise).
+__global__ void k_adam(float* __restrict__ P, float* __restrict__ G, float* __restrict__ M, float* __restrict__ V,
+                       int n, float lr, float b1, float b2, float eps, float c1, float c2,
+                       float* __restrict__ batch_loss) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == n) {  // the loss follows the gradient
+    *batch_loss = G[i];
+    G[i] = 0.0f;
+  }
   if (i >= n) return;
   float gr = G[i];
   float m = b1 * M[i] + (1.0f - b1) * gr;
@@ -312,6 +319,27 @@ __global__ void k_adam(float* __restrict__ P, const float* __restrict__ G, float
   M[i] = m;
   V[i] = v;
   P[i] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+  G[i] = 0.0f;
+}
+
+// Training rows in their shuffled order: row k of the training is the caller's
+// row perm[k].  The inverse first, then each uploaded chunk of the caller's
+// rows (starting at row0) goes to its places: 36 bytes read in order and
+// written to scattered 32-byte rows, where the host moved them one by one
+// through a second copy of the data.
+__global__ void k_invert(const uint32_t* __restrict__ perm, uint32_t rows, uint32_t* __restrict__ place) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < rows) place[perm[i]] = i;
+}
+__global__ void k_place_rows(const float4* __restrict__ feat, const float* __restrict__ target,
+                             const uint32_t* __restrict__ place, uint32_t row0, uint32_t rows,
+                             float4* __restrict__ feat_out, float* __restrict__ target_out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= rows) return;
+  const size_t k = place[row0 + i];
+  feat_out[2 * k] = feat[2 * (size_t)i];
+  feat_out[2 * k + 1] = feat[2 * (size_t)i + 1];
+  target_out[k] = target[i];
 }
 
 Norm norm_of(const pbf_mlp& m) {
@@ -462,10 +490,12 @@ cudaError_t launch_mlp_grad(const float* d_params, const pbf_mlp& model, const f
   return cudaGetLastError();
 }
 
-cudaError_t launch_adam(float* P, const float* G, float* M, float* V, int step, float lr, cudaStream_t st) {
+cudaError_t launch_adam(float* P, float* G, float* M, float* V, int step, float lr, float* batch_loss,
+                        cudaStream_t st) {
   const float b1 = 0.9f, b2 = 0.999f;
   float c1 = 1.0f - std::pow(b1, (float)step), c2 = 1.0f - std::pow(b2, (float)step);
-  k_adam<<<(PBF_MLP_PARAMS + 255) / 256, 256, 0, st>>>(P, G, M, V, PBF_MLP_PARAMS, lr, b1, b2, 1e-8f, c1, c2);
+  k_adam<<<(PBF_MLP_PARAMS + 1 + 255) / 256, 256, 0, st>>>(P, G, M, V, PBF_MLP_PARAMS, lr, b1, b2, 1e-8f, c1, c2,
+                                                          batch_loss);
   return cudaGetLastError();
 }
 
@@ -502,14 +532,23 @@ int pbf_mlp_init(pbf_mlp* m, uint64_t seed) {
 
 int pbf_mlp_fit_normalization(pbf_mlp* m, const float* feat, const float* target, uint32_t rows) {
   if (!m || !feat || !target || rows == 0) return PBF_EINVAL;
-  double mean[kIn] = {0}, sq[kIn] = {0}, tsq = 0;
+  // two features a vector, each sum in row order
+  typedef double pair __attribute__((vector_size(16)));
+  pair sum[kIn / 2] = {}, sum2[kIn / 2] = {};
+  double tsq = 0;
   for (uint32_t r = 0; r < rows; ++r) {
-    for (int k = 0; k < kIn; ++k) {
-      double v = feat[8 * (size_t)r + k];
-      mean[k] += v;
-      sq[k] += v * v;
+    const float* f = feat + 8 * (size_t)r;
+    for (int k = 0; k < kIn / 2; ++k) {
+      const pair v = {(double)f[2 * k], (double)f[2 * k + 1]};
+      sum[k] += v;
+      sum2[k] += v * v;
     }
     tsq += (double)target[r] * target[r];
+  }
+  double mean[kIn], sq[kIn];
+  for (int k = 0; k < kIn; ++k) {
+    mean[k] = sum[k / 2][k % 2];
+    sq[k] = sum2[k / 2][k % 2];
   }
   for (int k = 0; k < kIn; ++k) {
     double mu = mean[k] / rows, var = sq[k] / rows - mu * mu;
@@ -603,48 +642,63 @@ int pbf_mlp_train(pbf_mlp* m, const float* feat, const float* target, uint32_t r
     uint32_t j = (uint32_t)(splitmix(s) % (uint64_t)(i + 1));
     std::swap(perm[i], perm[j]);
   }
-  std::vector<float> f((size_t)rows * 8), tg(rows);
-  for (uint32_t i = 0; i < rows; ++i) {
-    std::memcpy(&f[8 * (size_t)i], feat + 8 * (size_t)perm[i], 8 * sizeof(float));
-    tg[i] = target[perm[i]];
-  }
-  float *dP = nullptr, *dF = nullptr, *dT = nullptr, *dG = nullptr, *dM = nullptr, *dV = nullptr;
-  cudaError_t e = cudaMalloc(&dP, sizeof(m->params));
-  if (e == cudaSuccess) e = cudaMalloc(&dF, f.size() * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&dT, tg.size() * sizeof(float));
-  // gradient, loss, then the device error word
-  if (e == cudaSuccess) e = cudaMalloc(&dG, (PBF_MLP_PARAMS + 2) * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemset(dG, 0, (PBF_MLP_PARAMS + 2) * sizeof(float));
+  // one allocation: parameters and moments, gradient + loss + error word + the
+  // last batch's loss, the shuffled rows, the shuffle and its inverse, and a
+  // chunk of the caller's rows on its way to them
+  const uint32_t chunk = rows < (1u << 20) ? rows : (1u << 20);
+  size_t bytes = 0;
+  auto place = [&](size_t count) {
+    const size_t at = bytes;
+    bytes += (count * sizeof(float) + 255) / 256 * 256;
+    return at;
+  };
+  const size_t oP = place(PBF_MLP_PARAMS), oM = place(PBF_MLP_PARAMS), oV = place(PBF_MLP_PARAMS),
+               oG = place(PBF_MLP_PARAMS + 3), cleared = bytes, oF = place((size_t)rows * 8), oT = place(rows),
+               oPerm = place(rows), oInv = place(rows), oRawF = place((size_t)chunk * 8), oRawT = place(chunk);
+  char* mem = nullptr;
+  cudaError_t e = cudaMalloc(&mem, bytes);
+  auto at = [&](size_t o) { return reinterpret_cast<float*>(mem + o); };
+  float *dP = at(oP), *dF = at(oF), *dT = at(oT), *dG = at(oG), *dM = at(oM), *dV = at(oV);
+  float* dLoss = dG + PBF_MLP_PARAMS;
   uint32_t* dErr = reinterpret_cast<uint32_t*>(dG + PBF_MLP_PARAMS + 1);
-  if (e == cudaSuccess) e = cudaMalloc(&dM, PBF_MLP_PARAMS * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&dV, PBF_MLP_PARAMS * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemcpy(dP, m->params, sizeof(m->params), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(dF, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(dT, tg.data(), tg.size() * sizeof(float), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(dM, 0, PBF_MLP_PARAMS * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemset(dV, 0, PBF_MLP_PARAMS * sizeof(float));
+  float* dBatchLoss = dG + PBF_MLP_PARAMS + 2;
+  uint32_t *dPerm = reinterpret_cast<uint32_t*>(at(oPerm)), *dInv = reinterpret_cast<uint32_t*>(at(oInv));
+  if (e == cudaSuccess) e = cudaMemsetAsync(mem, 0, cleared, 0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(dP, m->params, sizeof(m->params), cudaMemcpyHostToDevice, 0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(dPerm, perm.data(), (size_t)rows * 4, cudaMemcpyHostToDevice, 0);
+  if (e == cudaSuccess) {
+    k_invert<<<(rows + 255) / 256, 256, 0, 0>>>(dPerm, rows, dInv);
+    e = cudaGetLastError();
+  }
+  for (uint64_t r0 = 0; r0 < rows && e == cudaSuccess; r0 += chunk) {
+    const uint32_t c = (uint32_t)(rows - r0 < chunk ? rows - r0 : chunk);
+    e = cudaMemcpyAsync(at(oRawF), feat + 8 * r0, (size_t)c * 8 * sizeof(float), cudaMemcpyHostToDevice, 0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(at(oRawT), target + r0, (size_t)c * sizeof(float), cudaMemcpyHostToDevice, 0);
+    if (e == cudaSuccess) {
+      k_place_rows<<<(c + 255) / 256, 256, 0, 0>>>((const float4*)at(oRawF), at(oRawT), dInv, (uint32_t)r0, c,
+                                                   (float4*)dF, dT);
+      e = cudaGetLastError();
+    }
+  }
   const uint32_t batch = tc->batch < rows ? tc->batch : rows;
   const uint32_t per_epoch = rows / batch;
   double epoch_loss = 0.0;
   int step = 0;
   std::vector<float> lossbuf;
   for (uint32_t ep = 0; ep < tc->epochs && e == cudaSuccess; ++ep) {
-    float* dLoss = dG + PBF_MLP_PARAMS;
     double acc = 0.0;
     for (uint32_t b = 0; b < per_epoch && e == cudaSuccess; ++b) {
-      e = cudaMemsetAsync(dG, 0, (PBF_MLP_PARAMS + 1) * sizeof(float), 0);
-      if (e == cudaSuccess)
-        e = tc->kernel == PBF_MLP_TRAIN_TCGEN05
+      e = tc->kernel == PBF_MLP_TRAIN_TCGEN05
                 ? launch_mlp_grad_tc(dP, *m, dF + 8 * (size_t)b * batch, dT + (size_t)b * batch, batch, dG, dLoss,
                                      dErr, 0)
                 : launch_mlp_grad(dP, *m, dF + 8 * (size_t)b * batch, dT + (size_t)b * batch, batch, dG, dLoss, 0);
       ++step;
       float lr = tc->learning_rate;
       if (tc->epochs > 1) lr *= (float)(0.5 * (1.0 + std::cos(3.14159265358979 * ep / tc->epochs)));
-      if (e == cudaSuccess) e = launch_adam(dP, dG, dM, dV, step, lr, 0);
+      if (e == cudaSuccess) e = launch_adam(dP, dG, dM, dV, step, lr, dBatchLoss, 0);
       if (e == cudaSuccess && b + 1 == per_epoch) {
         float l = 0.0f;
-        e = cudaMemcpy(&l, dLoss, sizeof(float), cudaMemcpyDeviceToHost);
+        e = cudaMemcpy(&l, dBatchLoss, sizeof(float), cudaMemcpyDeviceToHost);
         acc = l / batch;
       }
     }
@@ -653,12 +707,7 @@ int pbf_mlp_train(pbf_mlp* m, const float* feat, const float* target, uint32_t r
   uint32_t herr = 0;
   if (e == cudaSuccess) e = cudaMemcpy(m->params, dP, sizeof(m->params), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(&herr, dErr, sizeof(uint32_t), cudaMemcpyDeviceToHost);
-  cudaFree(dP);
-  cudaFree(dF);
-  cudaFree(dT);
-  cudaFree(dG);
-  cudaFree(dM);
-  cudaFree(dV);
+  cudaFree(mem);
   if (final_loss) *final_loss = (float)epoch_loss;
   if (e != cudaSuccess) return PBF_ECUDA;
   return herr ? PBF_ETIMEOUT : PBF_OK;
