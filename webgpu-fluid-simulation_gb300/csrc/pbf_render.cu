@@ -233,6 +233,49 @@ __device__ inline void walk_sprite(const Sprite& s, uint32_t lane, Frag frag) {
 // the product of the x and y factors.
 __device__ inline float gauss_axis(float n) { return splat_exp((n * n) * -2.0f); }
 
+// Depth test ahead of the fragments: the smallest depth that any pixel of an
+// 8 x 8 tile holds.  Most sprites of a deep cloud lie behind the surface: at
+// 2^20 particles every covered pixel has hundreds of fragments, and reading its
+// key for each was half of the pass.  A share of the particles (one block of
+// 32 in kFirstShare, spread over the index range) is drawn first; the tiles'
+// smallest depths then reject a sprite whose bound is below them in all the
+// tiles it touches, which changes nothing in the result.
+constexpr int kTile = 8;
+constexpr uint32_t kFirstShare = 16;
+constexpr uint32_t kFirstPer = 4;            // of them a warp takes at a time
+constexpr uint32_t kTwoPhaseMin = 1u << 15;  // particles from which the extra launches pay
+constexpr int kMaxTiles = 16;                // larger sprites are not tested
+
+__global__ void __launch_bounds__(256) k_tile_min(const unsigned long long* __restrict__ keys, int W, int H, int tw,
+                                                  uint32_t* __restrict__ tile_min) {
+  // one warp per tile, two pixels a lane
+  const uint32_t lane = threadIdx.x & 31u, tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int tx = (int)tile % tw, ty = (int)tile / tw;
+  if (ty * kTile >= H) return;
+  uint32_t m = 0xffffffffu;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = tx * kTile + (int)(lane & 7u), j = ty * kTile + (int)(lane >> 3) + 4 * h;
+    if (i < W && j < H) m = min(m, (uint32_t)(keys[(size_t)j * W + i] >> 32));
+  }
+  m = __reduce_min_sync(0xffffffffu, m);
+  if (lane == 0) tile_min[tile] = m;
+}
+
+// Whether a depth sprite may win a pixel in any of its tiles.
+__device__ inline bool may_win(const Sprite& s, const uint32_t* __restrict__ tile_min, int tw) {
+  const int x0 = s.i0 / kTile, x1 = (s.i1 - 1) / kTile, y0 = s.j0 / kTile, y1 = (s.j1 - 1) / kTile;
+  if ((x1 - x0 + 1) * (y1 - y0 + 1) > kMaxTiles) return true;
+  for (int y = y0; y <= y1; ++y)
+    for (int x = x0; x <= x1; ++x)
+      if (s.dmax >= __ldg(tile_min + (size_t)y * tw + x)) return true;
+  return false;
+}
+
+// What a launch of the splat draws: all particles at once, or the first share's
+// depth sprites, or everything else.
+enum SplatPhase { kAll = 0, kFirst = 1, kRest = 2 };
+
 constexpr int kQueue = 64;  // per-warp queue of depth fragments that pass the bound test
 
 // Depth fragments that may win are queued (pixel, sprite) per warp and
@@ -255,7 +298,8 @@ __device__ inline void depth_fragments(const Cam& C, const SpriteSlot* slots, co
 }
 
 __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__ pos, uint32_t n, float R, int W, int H,
-                                               int W2, int H2, unsigned long long* keys, unsigned long long* acc) {
+                                               int W2, int H2, unsigned long long* keys, unsigned long long* acc,
+                                               int phase, const uint32_t* __restrict__ tile_min, int tw) {
   __shared__ SpriteSlot slots[8][32];
   __shared__ uint32_t qij[8][kQueue];
   __shared__ uint8_t qk[8][kQueue];
@@ -263,22 +307,29 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t lt = (1u << lane) - 1u;
-  for (uint32_t base = warp * 32; base < n; base += warps * 32) {
-    const uint32_t q = base + lane;
+  // the first share is spread thin: four particles a warp
+  const uint32_t per = phase == kFirst ? kFirstPer : 32u, parts = 32u / per;
+  const uint64_t groups = ((uint64_t)n + 31u) / 32u;
+  const uint64_t items = phase == kFirst ? (groups + kFirstShare - 1u) / kFirstShare * parts : groups;
+  for (uint64_t it = warp; it < items; it += warps) {
+    const uint64_t b = phase == kFirst ? it / parts * (kFirstShare * 32u) + it % parts * per : it * 32u;
+    if (b >= n) continue;
+    const uint32_t base = (uint32_t)b, q = base + lane;
+    const bool first = (base / 32u) % kFirstShare == 0u;  // drawn in the first phase
     SpriteSlot& mine = slots[wib][lane];
     mine.ok = 0;
-    if (q < n) {
+    const uint32_t cnt = min(per, n - base);
+    if (lane < cnt) {
       const float4 x = pos[q];
       float c[4];
       mat_vec(C.v, x.x, x.y, x.z, 1.0f, c);
-      if (make_sprite(C, c, 0.5f * R, W, H, mine.s[0])) {
-        mine.ok |= 1u;
+      if (!(phase == kRest && first) && make_sprite(C, c, 0.5f * R, W, H, mine.s[0])) {
         mine.s[0].dmax = depth_bound(C, c[2], c[3], R);
+        if (phase != kRest || may_win(mine.s[0], tile_min, tw)) mine.ok |= 1u;
       }
-      if (make_sprite(C, c, R, W2, H2, mine.s[1])) mine.ok |= 2u;
+      if (phase != kFirst && make_sprite(C, c, R, W2, H2, mine.s[1])) mine.ok |= 2u;
     }
     __syncwarp();
-    const uint32_t cnt = min(32u, n - base);
     uint32_t qn = 0;  // queued depth fragments (warp-uniform)
     for (uint32_t k = 0; k < cnt; ++k) {
       const SpriteSlot& sl = slots[wib][k];
@@ -435,6 +486,7 @@ struct pbf_renderer {
   float* volume = nullptr;
   unsigned long long* keys = nullptr;
   unsigned long long* acc = nullptr;
+  uint32_t* tile_min = nullptr;
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   float ms[2] = {0.0f, 0.0f};
 };
@@ -447,6 +499,7 @@ void release(pbf_renderer* r) {
   cudaFree(r->volume);
   cudaFree(r->keys);
   cudaFree(r->acc);
+  cudaFree(r->tile_min);
   for (auto& e : r->ev)
     if (e) cudaEventDestroy(e);
 }
@@ -510,6 +563,8 @@ int pbf_renderer_create(uint32_t width, uint32_t height, pbf_renderer** out) {
   if (e == cudaSuccess) e = cudaMalloc(&r->volume, px2 * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&r->keys, px * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMalloc(&r->acc, px2 * sizeof(unsigned long long));
+  if (e == cudaSuccess)
+    e = cudaMalloc(&r->tile_min, (size_t)((width + kTile - 1) / kTile) * ((height + kTile - 1) / kTile) * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(r->depth, 0, px * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(r->volume, 0, px2 * sizeof(float));
   for (auto& ev : r->ev)
@@ -568,8 +623,20 @@ int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_s
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned blocks = (unsigned)std::min<uint64_t>(((uint64_t)n + 255) / 256, (uint64_t)sms * 8);
-    k_splat<<<blocks, 256, 0, st>>>(C, pos, n, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc);
+    const auto blocks = [&](uint64_t warps) { return (unsigned)std::min<uint64_t>((warps + 7) / 8, (uint64_t)sms * 8); };
+    const uint64_t groups = ((uint64_t)n + 31) / 32;
+    const int tw = (r->W + kTile - 1) / kTile, th = (r->H + kTile - 1) / kTile;
+    auto splat = [&](int phase, uint64_t warps) {
+      k_splat<<<blocks(warps), 256, 0, st>>>(C, pos, n, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc, phase, r->tile_min,
+                                             tw);
+    };
+    if (n < kTwoPhaseMin) {
+      splat(kAll, groups);
+    } else {
+      splat(kFirst, (groups + kFirstShare - 1) / kFirstShare * (32 / kFirstPer));
+      k_tile_min<<<(unsigned)(((uint64_t)tw * th + 7) / 8), 256, 0, st>>>(r->keys, r->W, r->H, tw, r->tile_min);
+      splat(kRest, groups);
+    }
   }
   k_resolve<<<rows, 256, 0, st>>>(C, pos, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc, r->depth, d_scene_depth,
                                   r->volume);
