@@ -57,6 +57,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/pbf_gb300.h"
+#include "pbf_kernels.h"
 
 namespace {
 
@@ -266,6 +267,11 @@ __global__ void __launch_bounds__(256) k_tile_min(const unsigned long long* __re
 __device__ inline bool may_win(const Sprite& s, const uint32_t* __restrict__ tile_min, int tw) {
   const int x0 = s.i0 / kTile, x1 = (s.i1 - 1) / kTile, y0 = s.j0 / kTile, y1 = (s.j1 - 1) / kTile;
   if ((x1 - x0 + 1) * (y1 - y0 + 1) > kMaxTiles) return true;
+  if (x1 - x0 <= 1 && y1 - y0 <= 1) {  // most sprites: the four loads at once
+    const uint32_t *r0 = tile_min + (size_t)y0 * tw, *r1 = tile_min + (size_t)y1 * tw;
+    const uint32_t a = __ldg(r0 + x0), b = __ldg(r0 + x1), c = __ldg(r1 + x0), d = __ldg(r1 + x1);
+    return s.dmax >= min(min(a, b), min(c, d));
+  }
   for (int y = y0; y <= y1; ++y)
     for (int x = x0; x <= x1; ++x)
       if (s.dmax >= __ldg(tile_min + (size_t)y * tw + x)) return true;
@@ -297,9 +303,171 @@ __device__ inline void depth_fragments(const Cam& C, const SpriteSlot* slots, co
   if (key > *(volatile unsigned long long*)kp) atomicMax(kp, key);
 }
 
+// ---- volume sprites by tile ---------------------------------------------------------
+// The sums of a deep cloud are some 60 M additions to 100 K pixels at 2^20
+// particles; as 64-bit atomics on the map they took as long as all the rest of
+// the pass.  Sprites of at most 2 kVolHalo pixels across are sorted by the 24 x
+// 24 tile of their centre, and a CTA adds up a run of them in shared memory
+// before it adds its window (the tile and kVolHalo pixels around) to the map.
+// Integer sums: the result is the same in any order.
+constexpr int kVolTile = 24;                 // (four CTAs' windows fit an SM)
+constexpr int kVolHalo = 8;
+constexpr int kVolWin = kVolTile + 2 * kVolHalo;
+constexpr uint32_t kVolWarps = 8;
+constexpr uint32_t kVolPer = 60;             // sprites of one tile a warp takes at most
+constexpr uint32_t kVolRun = kVolWarps * kVolPer;  // sprites a CTA takes
+constexpr uint32_t kVolFew = 24;             // runs of fewer in one tile go to the map directly
+constexpr uint32_t kNoTile = 0xffffffffu;
+
+__device__ inline bool by_tile(const Sprite& s) { return s.i1 - s.i0 <= 2 * kVolHalo && s.j1 - s.j0 <= 2 * kVolHalo; }
+__device__ inline uint32_t tile_of(const Sprite& s, int vw) {
+  return (uint32_t)(((s.j0 + s.j1) >> 1) / kVolTile * vw + ((s.i0 + s.i1) >> 1) / kVolTile);
+}
+
+// Volume fragments of one sprite, its lanes' axis factors computed once:
+// add(i, j, term) for each pixel of the disc.
+template <typename Add>
+__device__ inline void volume_fragments(const Sprite& s, uint32_t lane, Add add) {
+  // per-lane axis factors: this lane's column (narrow sprites) and row j0 + lane
+  const int w = s.i1 - s.i0, h = s.j1 - s.j0;
+  float ex = 0.0f, ey = 0.0f;
+  if (w <= 32) {
+    const uint32_t m = c_recip16[w];
+    const int lc = (int)lane - (int)((lane * m) >> 16) * w;
+    ex = gauss_axis(__fmaf_rn((float)(s.i0 + lc), s.sx, s.ox));
+  }
+  if (h <= 32) ey = gauss_axis(__fmaf_rn((float)(s.j0 + (int)lane), s.sy, s.oy));
+  walk_sprite(s, lane, [&](int i, int j, bool in) {
+    float fy = __shfl_sync(0xffffffffu, ey, (j - s.j0) & 31);
+    if (!in) return;
+    const float r2 = sprite_r2(s, i, j);
+    if (r2 > 1.0f) return;
+    if (h > 32) fy = gauss_axis(__fmaf_rn((float)j, s.sy, s.oy));
+    const float fx = w <= 32 ? ex : gauss_axis(__fmaf_rn((float)i, s.sx, s.ox));
+    add(i, j, fx * fy);
+  });
+}
+
+// Particles in tile order (any order within a tile): next[t] starts as the
+// tile's first place.
+__global__ void __launch_bounds__(256) k_volume_order(uint32_t n, const uint32_t* __restrict__ tile,
+                                                      uint32_t* __restrict__ next, uint2* __restrict__ order) {
+  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+  const uint32_t t = q < n ? tile[q] : kNoTile;
+  const unsigned peers = __match_any_sync(0xffffffffu, t);
+  const int leader = __ffs(peers) - 1;
+  uint32_t at = 0u;
+  if (t != kNoTile && (int)lane == leader) at = atomicAdd(next + t, (uint32_t)__popc(peers));
+  at = __shfl_sync(0xffffffffu, at, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+  if (t != kNoTile) order[at] = make_uint2(t, q);
+}
+
+// A CTA's run of kVolRun sorted sprites, tile by tile, the tile's sprites shared
+// out among its warps.  A term exp(-2 |n|^2) is a float in [2^-3, 1], so in
+// units of 2^-26 an integer of at most 2^26, and 32-bit sums hold the kVolPer
+// sprites a warp takes.  Each warp has a window of its own, so its sums are
+// plain shared-memory reads and writes: one window per CTA took shared atomics
+// (four to five passes of the data path each) and barriers every 56 sprites.
+// A sprite is at most 16 pixels wide and high here: lanes 0 to 15 evaluate the
+// column factors and 16 to 31 the row factors at once.
+constexpr uint32_t kVolThreads = 32 * kVolWarps;
+constexpr size_t kVolSmem = sizeof(uint32_t) * kVolWarps * kVolWin * kVolWin;
+static_assert(kVolPer < 64, "32-bit sums");
+
+__global__ void __launch_bounds__(kVolThreads) k_volume_sum(Cam C, const float4* __restrict__ pos, float R, int W2, int H2,
+                                                            int vw, const uint2* __restrict__ order,
+                                                            const uint32_t* __restrict__ total, unsigned long long* acc) {
+  extern __shared__ uint32_t s_win[];
+  __shared__ uint32_t s_end;
+  constexpr uint32_t kPix = kVolWin * kVolWin;
+  const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+  uint32_t* win = s_win + wib * kPix;
+  const uint32_t first = blockIdx.x * kVolRun, last = min(first + kVolRun, *total);
+  if (first >= last) return;
+  for (uint32_t p = lane; p < kPix; p += 32u) win[p] = 0u;
+  __syncwarp();
+  uint32_t b = first;
+  while (b < last) {  // one tile's sprites [b, e)
+    const uint32_t t = order[b].x;
+    if (threadIdx.x == 0) s_end = last;
+    __syncthreads();
+    for (uint32_t k = b + threadIdx.x; k < last; k += kVolThreads)
+      if (order[k].x != t) {
+        atomicMin(&s_end, k);
+        break;
+      }
+    __syncthreads();
+    const uint32_t e = s_end;
+    const bool direct = e - b < kVolFew;
+    const int wx = (int)(t % (uint32_t)vw) * kVolTile - kVolHalo, wy = (int)(t / (uint32_t)vw) * kVolTile - kVolHalo;
+    const uint32_t per = (e - b + kVolWarps - 1u) / kVolWarps, g0 = b + wib * per, g1 = min(g0 + per, e);
+    for (uint32_t g = g0; g < g1; g += 32u) {
+      const uint32_t cnt = min(32u, g1 - g);
+      Sprite mine{};
+      if (lane < cnt) {
+        const float4 x = __ldg(pos + order[g + lane].y);
+        float c[4];
+        mat_vec(C.v, x.x, x.y, x.z, 1.0f, c);
+        make_sprite(C, c, R, W2, H2, mine);
+      }
+      for (int k = 0; k < (int)cnt; ++k) {
+        const int i0 = __shfl_sync(0xffffffffu, mine.i0, k), w = __shfl_sync(0xffffffffu, mine.i1, k) - i0;
+        const int j0 = __shfl_sync(0xffffffffu, mine.j0, k), h = __shfl_sync(0xffffffffu, mine.j1, k) - j0;
+        const float sx = __shfl_sync(0xffffffffu, mine.sx, k), ox = __shfl_sync(0xffffffffu, mine.ox, k);
+        const float sy = __shfl_sync(0xffffffffu, mine.sy, k), oy = __shfl_sync(0xffffffffu, mine.oy, k);
+        // a column or row past the sprite's gets a coordinate outside the disc
+        const bool row = lane >= 16u;
+        const int q = (int)(lane & 15u);
+        const float f = (float)((row ? j0 : i0) + q);
+        float nn = __fmaf_rn(f, row ? sy : sx, row ? oy : ox);
+        if (q >= (row ? h : w)) nn = 2.0f;
+        const float n2 = nn * nn, gs = splat_exp(n2 * -2.0f);
+        // lane -> (row of the step, column)
+        const uint32_t m = c_recip16[w], rows = (32u * m) >> 16, lr = (lane * m) >> 16;
+        const int col = (int)lane - (int)lr * w;
+        float nx = __shfl_sync(0xffffffffu, nn, col);
+        if (lr >= rows) nx = 2.0f;
+        const float ex = __shfl_sync(0xffffffffu, gs, col) * 67108864.0f;  // in units of 2^-26, exact
+        if (direct) {
+          for (int r0 = 0; r0 < h; r0 += (int)rows) {
+            const int r = r0 + (int)lr, src = min(16 + r, 31);
+            const float ny2 = __shfl_sync(0xffffffffu, n2, src), ey = __shfl_sync(0xffffffffu, gs, src);
+            if (r < h && __fmaf_rn(nx, nx, ny2) <= 1.0f)
+              atomicAdd(acc + (size_t)(j0 + r) * W2 + i0 + col, (unsigned long long)__float2uint_rn(ex * ey) << 14);
+          }
+          continue;
+        }
+        uint32_t* at = win + (j0 - wy + (int)lr) * kVolWin + (i0 - wx) + col;
+        for (int r = (int)lr; r < h + (int)lr; r += (int)rows, at += rows * kVolWin) {
+          const int src = min(16 + r, 31);
+          const float ny2 = __shfl_sync(0xffffffffu, n2, src), ey = __shfl_sync(0xffffffffu, gs, src);
+          // (a step's pixels are distinct, and the next sprite's come after them)
+          if (r < h && __fmaf_rn(nx, nx, ny2) <= 1.0f) *at += __float2uint_rn(ex * ey);
+        }
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    if (!direct) {
+      for (uint32_t p = threadIdx.x; p < kPix; p += kVolThreads) {
+        unsigned long long v = 0ull;
+#pragma unroll
+        for (uint32_t k = 0; k < kVolWarps; ++k) {
+          v += s_win[k * kPix + p];
+          s_win[k * kPix + p] = 0u;
+        }
+        if (v) atomicAdd(acc + (size_t)(wy + (int)(p / kVolWin)) * W2 + wx + (int)(p % kVolWin), v << 14);
+      }
+    }
+    b = e;
+    __syncthreads();
+  }
+}
+
 __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__ pos, uint32_t n, float R, int W, int H,
                                                int W2, int H2, unsigned long long* keys, unsigned long long* acc,
-                                               int phase, const uint32_t* __restrict__ tile_min, int tw) {
+                                               int phase, const uint32_t* __restrict__ tile_min, int tw,
+                                               uint32_t* __restrict__ vol_tile, uint32_t* __restrict__ vol_count) {
   __shared__ SpriteSlot slots[8][32];
   __shared__ uint32_t qij[8][kQueue];
   __shared__ uint8_t qk[8][kQueue];
@@ -319,6 +487,7 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
     SpriteSlot& mine = slots[wib][lane];
     mine.ok = 0;
     const uint32_t cnt = min(per, n - base);
+    uint32_t vt = kNoTile;
     if (lane < cnt) {
       const float4 x = pos[q];
       float c[4];
@@ -327,7 +496,18 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
         mine.s[0].dmax = depth_bound(C, c[2], c[3], R);
         if (phase != kRest || may_win(mine.s[0], tile_min, tw)) mine.ok |= 1u;
       }
-      if (phase != kFirst && make_sprite(C, c, R, W2, H2, mine.s[1])) mine.ok |= 2u;
+      if (phase != kFirst && make_sprite(C, c, R, W2, H2, mine.s[1])) {
+        // with phases, small volume sprites are summed by tile
+        if (phase == kRest && by_tile(mine.s[1]))
+          vt = tile_of(mine.s[1], (W2 + kVolTile - 1) / kVolTile);
+        else
+          mine.ok |= 2u;
+      }
+      if (phase == kRest) vol_tile[q] = vt;
+    }
+    if (phase == kRest) {  // the tiles' counts, one addition per warp and tile
+      const unsigned peers = __match_any_sync(0xffffffffu, vt);
+      if (vt != kNoTile && lane == (uint32_t)__ffs(peers) - 1u) atomicAdd(vol_count + vt, (uint32_t)__popc(peers));
     }
     __syncwarp();
     uint32_t qn = 0;  // queued depth fragments (warp-uniform)
@@ -337,9 +517,8 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
       if (ok & 1u) {
         const Sprite s = sl.s[0];
         const unsigned long long bound = ((unsigned long long)s.dmax << 32) | (0xffffffffull - (base + k));
-        walk_sprite(s, lane, [&](int i, int j, bool in) {
-          // only fragments whose sprite bound beats the pixel's current key can win
-          const bool pass = in && bound > *(volatile unsigned long long*)(keys + (size_t)j * W + i);
+        // only fragments whose sprite bound beats the pixel's current key can win
+        auto consider = [&](int i, int j, bool pass) {
           const unsigned m = __ballot_sync(0xffffffffu, pass);
           if (pass) {
             const uint32_t at = qn + __popc(m & lt);
@@ -358,28 +537,33 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
             }
             __syncwarp();
           }
-        });
+        };
+        const int w = s.i1 - s.i0;
+        if (w <= 32) {
+          // four steps' keys are read together: one at a time, each step of a
+          // sprite waited for its read
+          const uint32_t m = c_recip16[w];
+          const int rows = (int)((32u * m) >> 16), lr = (int)((lane * m) >> 16), i = s.i0 + (int)lane - lr * w;
+          for (int jb = s.j0 + lr; jb - lr < s.j1; jb += 4 * rows) {
+            unsigned long long key[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+              const int j = jb + h * rows;
+              key[h] = lr < rows && j < s.j1 ? *(volatile unsigned long long*)(keys + (size_t)j * W + i) : ~0ull;
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+              if (jb - lr + h * rows < s.j1) consider(i, jb + h * rows, bound > key[h]);
+          }
+        } else {
+          walk_sprite(s, lane, [&](int i, int j, bool in) {
+            consider(i, j, in && bound > *(volatile unsigned long long*)(keys + (size_t)j * W + i));
+          });
+        }
       }
       if (ok & 2u) {
-        const Sprite s = sl.s[1];
-        // per-lane axis factors: this lane's column (narrow sprites) and row j0 + lane
-        const int w = s.i1 - s.i0, h = s.j1 - s.j0;
-        float ex = 0.0f, ey = 0.0f;
-        if (w <= 32) {
-          const uint32_t m = c_recip16[w];
-          const int lc = (int)lane - (int)((lane * m) >> 16) * w;
-          ex = gauss_axis(__fmaf_rn((float)(s.i0 + lc), s.sx, s.ox));
-        }
-        if (h <= 32) ey = gauss_axis(__fmaf_rn((float)(s.j0 + (int)lane), s.sy, s.oy));
-        walk_sprite(s, lane, [&](int i, int j, bool in) {
-          float fy = __shfl_sync(0xffffffffu, ey, (j - s.j0) & 31);
-          if (!in) return;
-          const float r2 = sprite_r2(s, i, j);
-          if (r2 > 1.0f) return;
-          if (h > 32) fy = gauss_axis(__fmaf_rn((float)j, s.sy, s.oy));
-          const float fx = w <= 32 ? ex : gauss_axis(__fmaf_rn((float)i, s.sx, s.ox));
-          atomicAdd(acc + (size_t)j * W2 + i, fix40(fx * fy));
-        });
+        volume_fragments(sl.s[1], lane,
+                         [&](int i, int j, float v) { atomicAdd(acc + (size_t)j * W2 + i, fix40(v)); });
       }
     }
     __syncwarp();
@@ -487,6 +671,12 @@ struct pbf_renderer {
   unsigned long long* keys = nullptr;
   unsigned long long* acc = nullptr;
   uint32_t* tile_min = nullptr;
+  // volume sprites by tile, for up to vol_cap particles: tile per particle,
+  // order, then counts, places and the scan's scratch
+  uint32_t vol_cap = 0;
+  uint32_t* vol_tile = nullptr;
+  uint2* vol_order = nullptr;
+  uint32_t* vol_count = nullptr;
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   float ms[2] = {0.0f, 0.0f};
 };
@@ -500,6 +690,9 @@ void release(pbf_renderer* r) {
   cudaFree(r->keys);
   cudaFree(r->acc);
   cudaFree(r->tile_min);
+  cudaFree(r->vol_tile);
+  cudaFree(r->vol_order);
+  cudaFree(r->vol_count);
   for (auto& e : r->ev)
     if (e) cudaEventDestroy(e);
 }
@@ -528,6 +721,52 @@ cudaError_t launch_filter(const float* gauss, float* img, float* temp, int W, in
                                                                                               R * 5.0f, R);
   k_filter_y<<<dim3((unsigned)((W + 31) / 32), (unsigned)((H + kFilterYRows - 1) / kFilterYRows)), dim3(32, 8), 0,
                st>>>(temp, img, W, H, half, R * 5.0f, R);
+  return cudaGetLastError();
+}
+
+size_t volume_tiles(const pbf_renderer* r) {
+  return (size_t)((r->W2 + kVolTile - 1) / kVolTile) * ((r->H2 + kVolTile - 1) / kVolTile);
+}
+
+// Workspace for n particles (12 bytes each; kept, grown as needed).
+cudaError_t volume_workspace(pbf_renderer* r, uint32_t n, cudaStream_t st) {
+  const uint32_t cap = n;
+  cudaError_t e = cudaSuccess;
+  if (!r->vol_count) {
+    const size_t m = volume_tiles(r) + 1;
+    // counts and the scan's error word, places, scratch
+    e = cudaMalloc(&r->vol_count, (2 * m + 1) * sizeof(uint32_t) + pbf::scan_scratch_bytes(m) + 256);
+    if (e != cudaSuccess) return e;
+  }
+  if (cap > r->vol_cap) {
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+    cudaFree(r->vol_tile);
+    cudaFree(r->vol_order);
+    r->vol_tile = nullptr;
+    r->vol_order = nullptr;
+    r->vol_cap = 0;
+    e = cudaMalloc(&r->vol_tile, (size_t)cap * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&r->vol_order, (size_t)cap * sizeof(uint2));
+    if (e == cudaSuccess) r->vol_cap = cap;
+  }
+  return e;
+}
+
+uint32_t* volume_places(const pbf_renderer* r) { return r->vol_count + volume_tiles(r) + 2; }
+
+// The volume sprites summed by tile, once the splat has found their tiles.
+cudaError_t volume_by_tile(pbf_renderer* r, const Cam& C, const float4* pos, uint32_t n, float R, cudaStream_t st) {
+  const size_t m = volume_tiles(r) + 1;
+  uint32_t *err = r->vol_count + m, *place = volume_places(r);
+  char* scratch = reinterpret_cast<char*>(((uintptr_t)(place + m) + 255) / 256 * 256);
+  const cudaError_t e = pbf::launch_exclusive_scan(r->vol_count, place, m, scratch, err, st);
+  if (e != cudaSuccess) return e;
+  // (entry m - 1 of the counts is 0: its place is the total and stays it)
+  k_volume_order<<<(n + 255) / 256, 256, 0, st>>>(n, r->vol_tile, place, r->vol_order);
+  if (cudaFuncSetAttribute(k_volume_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVolSmem) != cudaSuccess)
+    return cudaGetLastError();
+  k_volume_sum<<<(n + kVolRun - 1) / kVolRun, kVolThreads, kVolSmem, st>>>(
+      C, pos, R, r->W2, r->H2, (r->W2 + kVolTile - 1) / kVolTile, r->vol_order, place + (m - 1), r->acc);
   return cudaGetLastError();
 }
 
@@ -628,14 +867,17 @@ int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_s
     const int tw = (r->W + kTile - 1) / kTile, th = (r->H + kTile - 1) / kTile;
     auto splat = [&](int phase, uint64_t warps) {
       k_splat<<<blocks(warps), 256, 0, st>>>(C, pos, n, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc, phase, r->tile_min,
-                                             tw);
+                                             tw, r->vol_tile, r->vol_count);
     };
-    if (n < kTwoPhaseMin) {
+    if (n < kTwoPhaseMin || volume_workspace(r, n, st) != cudaSuccess) {
+      cudaGetLastError();  // (without the workspace, everything is drawn at once)
       splat(kAll, groups);
     } else {
+      if (cudaMemsetAsync(r->vol_count, 0, (volume_tiles(r) + 2) * sizeof(uint32_t), st) != cudaSuccess) return PBF_ECUDA;
       splat(kFirst, (groups + kFirstShare - 1) / kFirstShare * (32 / kFirstPer));
       k_tile_min<<<(unsigned)(((uint64_t)tw * th + 7) / 8), 256, 0, st>>>(r->keys, r->W, r->H, tw, r->tile_min);
       splat(kRest, groups);
+      if (volume_by_tile(r, C, pos, n, R, st) != cudaSuccess) return PBF_ECUDA;
     }
   }
   k_resolve<<<rows, 256, 0, st>>>(C, pos, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc, r->depth, d_scene_depth,
