@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/pbf_gb300.h"
+#include "pbf_device.cuh"
 #include "pbf_kernels.h"
 #include "pbf_mlp.cuh"
 
@@ -307,6 +308,7 @@ __global__ void __launch_bounds__(32 * kTrainWarps) k_mlp_grad(const float* __re
 __global__ void k_adam(float* __restrict__ P, float* __restrict__ G, float* __restrict__ M, float* __restrict__ V,
                        int n, float lr, float b1, float b2, float eps, float c1, float c2,
                        float* __restrict__ batch_loss) {
+  chain_begin(P, G, M, V);
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == n) {  // the loss follows the gradient
     *batch_loss = G[i];
@@ -510,9 +512,8 @@ cudaError_t launch_adam(float* P, float* G, float* M, float* V, int step, float 
                         cudaStream_t st) {
   const float b1 = 0.9f, b2 = 0.999f;
   float c1 = 1.0f - std::pow(b1, (float)step), c2 = 1.0f - std::pow(b2, (float)step);
-  k_adam<<<(PBF_MLP_PARAMS + 1 + 255) / 256, 256, 0, st>>>(P, G, M, V, PBF_MLP_PARAMS, lr, b1, b2, 1e-8f, c1, c2,
-                                                          batch_loss);
-  return cudaGetLastError();
+  return launch_chain(true, k_adam, (PBF_MLP_PARAMS + 1 + 255) / 256, 256, 0, st, P, G, M, V, PBF_MLP_PARAMS, lr, b1,
+                      b2, 1e-8f, c1, c2, batch_loss);
 }
 
 }  // namespace pbf

@@ -43,6 +43,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/pbf_gb300.h"
+#include "pbf_device.cuh"
 #include "pbf_kernels.h"
 #include "pbf_mlp.cuh"
 
@@ -374,8 +375,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_infer_tc(const float* __r
 
 // ---- training: forward + backward on the tensor cores --------------------------------
 //
-// One CTA of 128 threads (one warpgroup), thread t serving row t of each
-// 128-row tile, TMEM holding every accumulator (512 columns: one CTA per SM):
+// One CTA of 256 threads (two warpgroups).  Thread t of either serves row t of
+// each 128-row tile: the first warpgroup its hidden units 0..31, the second
+// 32..63.  TMEM holds every accumulator (512 columns: one CTA per SM):
 //   columns   0- 63  z1 = X W1 + b1            (kept for the backward pass)
 //   columns  64-127  z2 = H1 W2 + b2           (kept for the backward pass)
 //   columns 128-143  y  = H2 w3 + b3           (hi / lo columns 0, 1)
@@ -393,18 +395,36 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_infer_tc(const float* __r
 // about 2^-16 relative accuracy; the other products take their operands in
 // bf16 at the rounding points of the mma.sync kernel (X, W, H1, H2, dZ2,
 // dZ1).  All operands are K-major, no swizzle, as in k_mlp_infer_tc.
-constexpr uint32_t kGrTmemCols = 512;
+constexpr uint32_t kGrTmemCols = 512, kGrThreads = 256;
 constexpr uint32_t kColZ1 = 0, kColZ2 = 64, kColY = 128, kColDH1 = 160, kColG1 = 256, kColG2 = 320, kColG3 = 384;
 
+// Core matrices of the tiles that are written by columns (K = the 128 rows):
+// 144 bytes apart in K, so that the 32 rows of a warp write their elements of
+// one column to different banks (128 bytes apart, four rows met in each).
+constexpr uint32_t kColLbo = 144, kColSbo = 16 * kColLbo;
+constexpr int col_tile(int m) { return m / 8 * (int)kColSbo; }
+
+// Byte offset of element (m, k) in a column-written tile.
+__device__ __forceinline__ uint32_t canon_col(uint32_t m, uint32_t k) {
+  return (m >> 3) * kColSbo + (k >> 3) * kColLbo + (m & 7u) * 16u + (k & 7u) * 2u;
+}
+
+// The gradient on its way out: the flat parameter layout is 75 rows of 64 (W1,
+// b1, W2, b2, w3) and b3; 68 floats a row here keeps 16-byte units of one
+// column in different banks.
+constexpr uint32_t kOutRows = (PBF_MLP_PARAMS - 1) / 64, kOutStride = 68;
+static_assert(OFF_B1 == 8 * 64 && OFF_W2 == 9 * 64 && OFF_B2 == 73 * 64 && OFF_W3 == 74 * 64 && OFF_B3 == 75 * 64,
+              "the flat layout is whole rows of 64, then b3");
+
 struct GrSmem {
-  alignas(128) uint8_t x1[128 * 16 * 2];    // X rows (K = 16: 8 features, ones at 8, 9)
-  alignas(128) uint8_t hA[128 * 64 * 2];    // H1 rows, then H2 rows, then dZ2 rows
-  alignas(128) uint8_t tH1[128 * 128 * 2];  // A of [dW2; db2]: H1^T, ones (row 64); rows 65+ unused
-  alignas(128) uint8_t tX[128 * 128 * 2];   // A of [dW1; db1]: X^T, ones (row 8); rows 9+ unused
-  alignas(128) uint8_t tH2[128 * 128 * 2];  // A of [dw3; db3]: H2^T, ones (row 64); rows 65+ unused
-  alignas(128) uint8_t tDZ2[64 * 128 * 2];  // B: dZ2^T (N = 64 x K = rows)
-  alignas(128) uint8_t tDZ1[64 * 128 * 2];  // B: dZ1^T
-  alignas(128) uint8_t tDY[16 * 128 * 2];   // B: dy hi (N row 0), lo (row 1); rows 2+ unused
+  alignas(128) uint8_t x1[128 * 16 * 2];     // X rows (K = 16: 8 features, ones at 8, 9)
+  alignas(128) uint8_t hA[128 * 64 * 2];     // H1 rows, then H2 rows, then dZ2 rows
+  alignas(128) uint8_t tH1[col_tile(128)];   // A of [dW2; db2]: H1^T, ones (row 64); rows 65+ unused
+  alignas(128) uint8_t tX[col_tile(128)];    // A of [dW1; db1]: X^T, ones (row 8); rows 9+ unused
+  alignas(128) uint8_t tH2[col_tile(128)];   // A of [dw3; db3]: H2^T, ones (row 64); rows 65+ unused
+  alignas(128) uint8_t tDZ2[col_tile(64)];   // B: dZ2^T (N = 64 x K = rows)
+  alignas(128) uint8_t tDZ1[col_tile(64)];   // B: dZ1^T
+  alignas(128) uint8_t tDY[col_tile(16)];    // B: dy hi (N row 0), lo (row 1); rows 2+ unused
   alignas(128) uint8_t b1[64 * 16 * 2];     // W1'^T with b1 hi / lo in K rows 8, 9
   alignas(128) uint8_t b2[64 * 64 * 2];     // W2^T (N = out, K = in)
   alignas(128) uint8_t b2b[64 * 16 * 2];    // b2 hi / lo in K rows 8, 9
@@ -414,8 +434,8 @@ struct GrSmem {
   float w3[64];                             // w3 in FP32 (dZ2's factor)
   alignas(8) uint64_t mbar;
   uint32_t tmem;
-  uint32_t failed;
 };
+static_assert(sizeof(GrSmem::tH1) >= kOutRows * kOutStride * sizeof(float), "the gradient is staged over H1^T");
 
 __device__ __forceinline__ void st_bf16(uint8_t* tile, uint32_t off, float v) {
   *reinterpret_cast<__nv_bfloat16*>(tile + off) = __float2bfloat16_rn(v);
@@ -439,47 +459,29 @@ __device__ __forceinline__ bool gr_mma_step(GrSmem& sm, uint32_t mbar, uint32_t&
   return ok;
 }
 
-__global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict__ P, Norm nm,
-                                                      const float* __restrict__ feat,
-                                                      const float* __restrict__ target, uint32_t rows,
-                                                      float inv_batch, float* __restrict__ G,
-                                                      float* __restrict__ loss, uint32_t* err) {
+// Bound by the serial chain of a tile (six products, each waited for, and the
+// element work between them): at 8192 rows 64 CTAs have one tile each.  So two
+// threads share a row, the weights are staged in 16-byte units with all their
+// loads in flight, and the gradient leaves as 16-byte reductions over
+// consecutive addresses (a row per thread before: 32 lines an instruction).
+// A batch of 8192, this kernel and k_adam: 29 us with one warpgroup, scalar
+// staging and a row per thread out, 14.2 now, 9.7 with both launched early.
+__global__ void __launch_bounds__(kGrThreads, 1) k_mlp_grad_tc(const float* __restrict__ P, Norm nm,
+                                                             const float* __restrict__ feat,
+                                                             const float* __restrict__ target, uint32_t rows,
+                                                             float inv_batch, float* __restrict__ G,
+                                                             float* __restrict__ loss, uint32_t* err) {
   extern __shared__ __align__(128) uint8_t gr_raw[];
   GrSmem& sm = *reinterpret_cast<GrSmem*>(gr_raw);
-  const uint32_t tid = threadIdx.x, warp = tid >> 5, row = tid;
-  const __nv_bfloat16 z16 = __float2bfloat16_rn(0.0f);
-  // weights (as in k_mlp_infer_tc) and the transposed W2
-  for (uint32_t q = tid; q < 64u * 16u; q += 128u) {
-    const uint32_t n = q / 16u, k = q % 16u;
-    __nv_bfloat16 w = z16, wb = z16;
-    if (k < (uint32_t)kIn) {
-      w = __float2bfloat16_rn(P[OFF_W1 + k * kH + n]);
-    } else if (k == 8) {
-      w = bf_hi(P[OFF_B1 + n]);
-      wb = bf_hi(P[OFF_B2 + n]);
-    } else if (k == 9) {
-      w = bf_lo(P[OFF_B1 + n]);
-      wb = bf_lo(P[OFF_B2 + n]);
-    }
-    *reinterpret_cast<__nv_bfloat16*>(sm.b1 + canon(n, k, 16)) = w;
-    *reinterpret_cast<__nv_bfloat16*>(sm.b2b + canon(n, k, 16)) = wb;
-  }
-  for (uint32_t q = tid; q < 64u * 64u; q += 128u) {
-    const uint32_t i = q / 64u, j = q % 64u;  // W2[i][j]: in i, out j
-    const __nv_bfloat16 w = __float2bfloat16_rn(P[OFF_W2 + q]);
-    *reinterpret_cast<__nv_bfloat16*>(sm.b2 + canon(j, i, 64)) = w;
-    *reinterpret_cast<__nv_bfloat16*>(sm.b2t + canon(i, j, 64)) = w;
-  }
-  for (uint32_t q = tid; q < 16u * 64u; q += 128u) {
-    const uint32_t n = q / 64u, k = q % 64u;
-    const float w = P[OFF_W3 + k];
-    *reinterpret_cast<__nv_bfloat16*>(sm.b3 + canon(n, k, 64)) = n == 0 ? bf_hi(w) : n == 1 ? bf_lo(w) : z16;
-  }
-  for (uint32_t q = tid; q < 16u * 16u; q += 128u) {
-    const uint32_t n = q / 16u, k = q % 16u;
-    const float b = P[OFF_B3];
-    *reinterpret_cast<__nv_bfloat16*>(sm.b3b + canon(n, k, 16)) =
-        (n == 0 && k == 8) ? bf_hi(b) : (n == 0 && k == 9) ? bf_lo(b) : z16;
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, row = tid & 127u;
+  const uint32_t half = tid >> 7;  // warpgroup: hidden units 32 half .. 32 half + 31
+  const uint32_t mbar = smem_u32(&sm.mbar);
+  if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)),
+                 "r"(kGrTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   // constant parts of the gradient operands: the ones rows (row 64 of H1^T
   // and H2^T, row 8 of X^T) that turn the products into bias gradients.
@@ -491,27 +493,62 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict_
     const uint32_t ones2 = pack_bf16(1.0f, 1.0f);
     uint8_t* tile = tid < 16u ? sm.tH1 : tid < 32u ? sm.tH2 : sm.tX;
     const uint32_t m = tid < 32u ? 64u : 8u, k = 8u * (tid % 16u);
-    st_shared_v4(smem_u32(tile + canon(m, k, 128)), ones2, ones2, ones2, ones2);
+    st_shared_v4(smem_u32(tile + canon_col(m, k)), ones2, ones2, ones2, ones2);
   }
-  if (tid < 64u) sm.w3[tid] = P[OFF_W3 + tid];
-  st_shared_v4(smem_u32(sm.x1 + canon(row, 8, 16)), pack_bf16(1.0f, 1.0f), 0u, 0u, 0u);
-  const uint32_t mbar = smem_u32(&sm.mbar);
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
-    sm.failed = 0u;
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)),
-                 "r"(kGrTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  if (half == 0) st_shared_v4(smem_u32(sm.x1 + canon(row, 8, 16)), pack_bf16(1.0f, 1.0f), 0u, 0u, 0u);
+  chain_begin(P, feat, target);  // launched early: nothing above reads memory
+  // weights (as in k_mlp_infer_tc) and the transposed W2, eight K elements of
+  // one N row per 16-byte unit
+  {
+    float w2[2][8], w2t[2][8], w1[8];
+#pragma unroll
+    for (uint32_t c = 0; c < 2; ++c) {
+      const uint32_t u = tid + kGrThreads * c, n = u % 64u, k = 8u * (u / 64u);  // W2[i][j]: in i, out j
+#pragma unroll
+      for (uint32_t e = 0; e < 8; ++e) {
+        w2[c][e] = P[OFF_W2 + (k + e) * kH + n];   // W2^T: N = out n, K = in k + e
+        w2t[c][e] = P[OFF_W2 + u * 8u + e];        // W2: N = in u / 8, K = out 8 (u % 8) + e
+      }
+    }
+    const uint32_t n = row / 2u;  // units of b1 (first warpgroup) and b2b (second): N row n, K half row % 2
+    const bool bias = row % 2u != 0;
+    const float b = P[(half == 0 ? OFF_B1 : OFF_B2) + n];
+#pragma unroll
+    for (uint32_t e = 0; e < 8; ++e) w1[e] = (half == 0 && !bias) ? P[OFF_W1 + e * kH + n] : 0.0f;
+    const float w3 = P[OFF_W3 + tid % 64u], b3 = P[OFF_B3];
+    auto store8 = [](uint8_t* at, const float (&v)[8]) {
+      st_shared_v4(smem_u32(at), pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
+                   pack_bf16(v[6], v[7]));
+    };
+    const uint32_t b_hilo = pack_bf16(b, b - bf16_round(b)), b3_hilo = pack_bf16(b3, b3 - bf16_round(b3));
+    uint8_t* const bt = half == 0 ? sm.b1 : sm.b2b;
+    if (bias) st_shared_v4(smem_u32(bt + canon(n, 8, 16)), b_hilo, 0u, 0u, 0u);
+    else store8(bt + canon(n, 0, 16), w1);
+#pragma unroll
+    for (uint32_t c = 0; c < 2; ++c) {
+      const uint32_t u = tid + kGrThreads * c;
+      store8(sm.b2 + canon(u % 64u, 8u * (u / 64u), 64), w2[c]);
+      store8(sm.b2t + canon(u / 8u, 8u * (u % 8u), 64), w2t[c]);
+    }
+    // w3 hi / lo in N rows 0 and 1 (threads 0..63), rows 2..15 zero
+    if (tid < 64u) {
+      sm.w3[tid] = w3;
+      *reinterpret_cast<__nv_bfloat16*>(sm.b3 + canon(0, tid, 64)) = bf_hi(w3);
+      *reinterpret_cast<__nv_bfloat16*>(sm.b3 + canon(1, tid, 64)) = bf_lo(w3);
+    } else if (tid < 176u) {
+      const uint32_t q = tid - 64u;  // 14 rows of eight units
+      st_shared_v4(smem_u32(sm.b3 + canon(2u + q / 8u, 8u * (q % 8u), 64)), 0u, 0u, 0u, 0u);
+    } else if (tid < 208u) {
+      const uint32_t q = tid - 176u;  // 16 rows of two units
+      st_shared_v4(smem_u32(sm.b3b + canon(q / 2u, 8u * (q % 2u), 16)), q == 1u ? b3_hilo : 0u, 0u, 0u, 0u);
+    }
   }
   fence_async_smem();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   const uint32_t tm = sm.tmem;
-  const uint32_t lane_base = (32u * warp) << 16;
+  const uint32_t lane_base = (32u * (warp & 3u)) << 16;
   const uint64_t x1d = smem_desc(smem_u32(sm.x1), 128, 256);
   const uint64_t b1d = smem_desc(smem_u32(sm.b1), 128, 256);
   const uint64_t b2bd = smem_desc(smem_u32(sm.b2b), 128, 256);
@@ -527,19 +564,28 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict_
   for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++done_tiles) {
     const uint32_t r = tile * 128u + row;
     const bool valid = r < rows;
-    float x[8], t = 0.0f;
+    // each warpgroup takes four of the features
+    float x[4], t = 0.0f;
+    float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (valid) {
+      f = reinterpret_cast<const float4*>(feat)[2 * (size_t)r + half];
+      t = target[r] / nm.lam_scale;
+    }
+    const float fv[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = valid ? (feat[8 * (size_t)r + k] - nm.mean[k]) * nm.inv_std[k] : 0.0f;
-    if (valid) t = target[r] / nm.lam_scale;
-    st_shared_v4(smem_u32(sm.x1 + canon(row, 0, 16)), pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]),
-                 pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+    for (int k = 0; k < 4; ++k) {
+      const float mean = half == 0 ? nm.mean[k] : nm.mean[k + 4];
+      const float inv_std = half == 0 ? nm.inv_std[k] : nm.inv_std[k + 4];
+      x[k] = valid ? (fv[k] - mean) * inv_std : 0.0f;
+    }
+    *reinterpret_cast<uint2*>(sm.x1 + canon(row, 4u * half, 16)) =
+        make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
 #pragma unroll
-    for (int k = 0; k < 8; ++k) st_bf16(sm.tX, canon(k, row, 128), x[k]);
+    for (uint32_t k = 0; k < 4; ++k) st_bf16(sm.tX, canon_col(4u * half + k, row), x[k]);
     // z1 = X W1 + b1
     ok = gr_mma_step(sm, mbar, phase, [&] { mma_f16(tm + kColZ1, x1d, b1d, kIdesc64, 0u); }) && ok;
     // H1 rows (layer 2's A) and H1^T (dW2's A)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    {
       float v[32];
       tmem_ld32(tm + lane_base + kColZ1 + 32u * half, v);
 #pragma unroll
@@ -548,10 +594,10 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict_
         float h[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) h[e] = silu_h(v[j + e]);
-        st_shared_v4(hA + canon(row, 32 * half + j, 64), pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]),
+        st_shared_v4(hA + canon(row, 32u * half + j, 64), pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]),
                      pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
 #pragma unroll
-        for (int e = 0; e < 8; ++e) st_bf16(sm.tH1, canon(32 * half + j + e, row, 128), h[e]);
+        for (int e = 0; e < 8; ++e) st_bf16(sm.tH1, canon_col(32u * half + j + e, row), h[e]);
       }
     }
     // z2 = H1 W2 + b2
@@ -562,8 +608,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict_
       mma_f16(tm + kColZ2, x1d, b2bd, kIdesc64, 1u);
     }) && ok;
     // H2 rows (layer 3's A) and H2^T (dw3's A)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    {
       float v[32];
       tmem_ld32(tm + lane_base + kColZ2 + 32u * half, v);
 #pragma unroll
@@ -572,10 +617,10 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict_
         float h[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) h[e] = silu_h(v[j + e]);
-        st_shared_v4(hA + canon(row, 32 * half + j, 64), pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]),
+        st_shared_v4(hA + canon(row, 32u * half + j, 64), pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]),
                      pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
 #pragma unroll
-        for (int e = 0; e < 8; ++e) st_bf16(sm.tH2, canon(32 * half + j + e, row, 128), h[e]);
+        for (int e = 0; e < 8; ++e) st_bf16(sm.tH2, canon_col(32u * half + j + e, row), h[e]);
       }
     }
     // y = H2 w3 + b3
@@ -588,13 +633,15 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict_
     float y0, y1;
     tmem_ld2(tm + lane_base + kColY, y0, y1);
     const float err_y = valid ? (y0 + y1) - t : 0.0f;
-    lsum += err_y * err_y;
     const float dy = 2.0f * err_y * inv_batch;
-    st_bf16(sm.tDY, canon(0, row, 128), dy);
-    st_bf16(sm.tDY, canon(1, row, 128), dy - __bfloat162float(__float2bfloat16_rn(dy)));
+    if (half == 0) {
+      lsum += err_y * err_y;
+      st_bf16(sm.tDY, canon_col(0, row), dy);
+    } else {
+      st_bf16(sm.tDY, canon_col(1, row), dy - bf16_round(dy));
+    }
     // dZ2 = dy w3 silu'(z2): rows (dH1's A) and transposed (dW2's B)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    {
       float v[32];
       tmem_ld32(tm + lane_base + kColZ2 + 32u * half, v);
 #pragma unroll
@@ -602,11 +649,11 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict_
         const int j = 8 * kb;
         float d[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) d[e] = dy * sm.w3[32 * half + j + e] * dsilu_f(v[j + e]);
-        st_shared_v4(hA + canon(row, 32 * half + j, 64), pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]),
+        for (int e = 0; e < 8; ++e) d[e] = dy * sm.w3[32u * half + j + e] * dsilu_f(v[j + e]);
+        st_shared_v4(hA + canon(row, 32u * half + j, 64), pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]),
                      pack_bf16(d[4], d[5]), pack_bf16(d[6], d[7]));
 #pragma unroll
-        for (int e = 0; e < 8; ++e) st_bf16(sm.tDZ2, canon(32 * half + j + e, row, 128), d[e]);
+        for (int e = 0; e < 8; ++e) st_bf16(sm.tDZ2, canon_col(32u * half + j + e, row), d[e]);
       }
     }
     // dH1 = dZ2 W2^T
@@ -616,25 +663,22 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict_
                 kIdesc64, ks > 0 ? 1u : 0u);
     }) && ok;
     // dZ1 = dH1 silu'(z1), transposed (dW1's B)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    {
       float g[32], z[32];
       tmem_ld32(tm + lane_base + kColDH1 + 32u * half, g);
       tmem_ld32(tm + lane_base + kColZ1 + 32u * half, z);
 #pragma unroll
-      for (int e = 0; e < 32; ++e) st_bf16(sm.tDZ1, canon(32 * half + e, row, 128), g[e] * dsilu_f(z[e]));
+      for (int e = 0; e < 32; ++e) st_bf16(sm.tDZ1, canon_col(32u * half + e, row), g[e] * dsilu_f(z[e]));
     }
     // the gradient products over the tile's rows, accumulated across tiles
     const uint32_t acc0 = done_tiles > 0 ? 1u : 0u;
     ok = gr_mma_step(sm, mbar, phase, [&] {
       for (uint32_t ks = 0; ks < 8; ++ks) {
         const uint32_t a = ks > 0 ? 1u : acc0;
-        mma_f16(tm + kColG1, smem_desc(tH1 + 256u * ks, 128, 2048), smem_desc(tDZ2 + 256u * ks, 128, 2048), kIdesc64,
-                a);
-        mma_f16(tm + kColG2, smem_desc(tX + 256u * ks, 128, 2048), smem_desc(tDZ1 + 256u * ks, 128, 2048), kIdesc64,
-                a);
-        mma_f16(tm + kColG3, smem_desc(tH2 + 256u * ks, 128, 2048), smem_desc(tDY + 256u * ks, 128, 2048), kIdesc16,
-                a);
+        auto desc = [&](uint32_t tile) { return smem_desc(tile + 2u * kColLbo * ks, kColLbo, kColSbo); };
+        mma_f16(tm + kColG1, desc(tH1), desc(tDZ2), kIdesc64, a);
+        mma_f16(tm + kColG2, desc(tX), desc(tDZ1), kIdesc64, a);
+        mma_f16(tm + kColG3, desc(tH2), desc(tDY), kIdesc16, a);
       }
     }) && ok;
     ok = !__syncthreads_or(!ok);
@@ -645,35 +689,30 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* __restrict_
     mbar_wait(mbar, phase);
     if (tid == 0 && err) atomicOr(err, PBF_DEVERR_MMA_TIMEOUT);
   } else if (done_tiles > 0) {
-    // row m of the accumulators: [dW2; db2], [dW1; db1], [dw3; db3]
+    // row m of the accumulators: [dW2; db2], [dW1; db1], [dw3; db3], staged in
+    // the flat layout over H1^T (the products that read it are done)
+    float* const out = reinterpret_cast<float*>(sm.tH1);
+    auto stage = [&](uint32_t to, const float (&v)[32]) {
+      float4* q = reinterpret_cast<float4*>(out + to * kOutStride + 32u * half);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      float v[32];
-      tmem_ld32(tm + lane_base + kColG1 + 32u * half, v);
-      if (row < 64u) {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) atomicAdd(G + OFF_W2 + row * kH + 32 * half + e, v[e]);
-      } else if (row == 64u) {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) atomicAdd(G + OFF_B2 + 32 * half + e, v[e]);
-      }
-      tmem_ld32(tm + lane_base + kColG2 + 32u * half, v);
-      if (row < (uint32_t)kIn) {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) atomicAdd(G + OFF_W1 + row * kH + 32 * half + e, v[e]);
-      } else if (row == (uint32_t)kIn) {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) atomicAdd(G + OFF_B1 + 32 * half + e, v[e]);
-      }
-    }
-    float g0, g1;
+      for (int e = 0; e < 8; ++e) q[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+    };
+    float v[32], g0, g1;
+    tmem_ld32(tm + lane_base + kColG1 + 32u * half, v);
+    if (row <= 64u) stage(OFF_W2 / 64 + row, v);
+    tmem_ld32(tm + lane_base + kColG2 + 32u * half, v);
+    if (row <= (uint32_t)kIn) stage(OFF_W1 / 64 + row, v);
     tmem_ld2(tm + lane_base + kColG3, g0, g1);
-    if (row < 64u) atomicAdd(G + OFF_W3 + row, g0 + g1);
-    else if (row == 64u) atomicAdd(G + OFF_B3, g0 + g1);
+    if (half == 0 && row < 64u) out[OFF_W3 / 64 * kOutStride + row] = g0 + g1;
+    if (half == 0 && row == 64u) atomicAdd(G + OFF_B3, g0 + g1);
+    __syncthreads();
+    for (uint32_t u = tid; u < kOutRows * 16u; u += kGrThreads)
+      atomicAdd(reinterpret_cast<float4*>(G) + u,
+                *reinterpret_cast<const float4*>(out + u / 16u * kOutStride + 4u * (u % 16u)));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if ((tid & 31u) == 0) atomicAdd(loss, lsum);
+  if (half == 0 && (tid & 31u) == 0) atomicAdd(loss, lsum);
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -749,9 +788,8 @@ cudaError_t launch_mlp_grad_tc(const float* d_params, const pbf_mlp& model, cons
   const uint32_t tiles = (rows + 127u) / 128u;
   // one CTA per SM at most: each holds all 512 TMEM columns
   const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)sms);
-  k_mlp_grad_tc<<<grid, 128, sizeof(GrSmem), st>>>(d_params, nm, d_feat, d_target, rows, 1.0f / (float)rows,
-                                                   d_grad, d_loss, d_err);
-  return cudaGetLastError();
+  return launch_chain(true, k_mlp_grad_tc, grid, kGrThreads, sizeof(GrSmem), st, d_params, nm, d_feat, d_target, rows,
+                      1.0f / (float)rows, d_grad, d_loss, d_err);
 }
 
 }  // namespace pbf
