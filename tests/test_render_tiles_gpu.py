@@ -1,7 +1,8 @@
-"""The splat's two-phase path (a first share, the tiles' depth test, volume
-sprites summed by tile) at its edges, bit for bit against the restatement: the
-particle count where it begins, crowded tiles, sprites too large for a tile's
-window, and maps whose sides are no multiple of a tile."""
+"""The splat at the edges of its split over warps and of its two-phase path (a
+first share, the tiles' depth test, volume sprites summed by tile), bit for bit
+against the restatement: the particle counts where they change, crowded tiles,
+sprites too large for a tile's window, and maps whose sides are no multiple of
+a tile."""
 import numpy as np
 import pytest
 
@@ -14,7 +15,10 @@ torch = pytest.importorskip("torch")
 
 @pytest.mark.parametrize("n,W,H,R,spread", [(32767, 321, 177, 0.02, 0.5), (32768, 321, 177, 0.02, 0.5),
                                             (40001, 640, 360, 0.02, 0.03), (33000, 203, 95, 0.2, 0.6),
-                                            (50000, 1023, 577, 0.01, 2.5)])
+                                            (50000, 1023, 577, 0.01, 2.5), (524287, 1280, 820, 0.01, 0.5),
+                                            (524288, 1280, 820, 0.01, 0.5), (524288, 1023, 1031, 0.01, 2.5),
+                                            (600001, 1031, 1023, 0.02, 0.03), (3000, 1031, 1023, 0.02, 0.3),
+                                            (10001, 320, 200, 0.05, 0.3)])
 def test_two_phase_splat(n, W, H, R, spread):
     rng = np.random.default_rng(n + W)
     p = np.zeros((n, 4), np.float32)

@@ -16,11 +16,11 @@ namespace pbf {
 // while the stream's previous kernel ends (programmatic dependent launch), so
 // a chain of short kernels does not pay a full launch gap per link.
 template <class... P, class... A>
-cudaError_t launch_chain(bool early, void (*kernel)(P...), unsigned grid, int block, size_t smem, cudaStream_t st,
+cudaError_t launch_chain(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                          A&&... args) {
   cudaLaunchConfig_t c{};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3((unsigned)block);
+  c.gridDim = grid;
+  c.blockDim = block;
   c.dynamicSmemBytes = smem;
   c.stream = st;
   cudaLaunchAttribute at{};

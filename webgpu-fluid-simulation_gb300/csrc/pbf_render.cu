@@ -57,16 +57,19 @@
 #include <cuda_runtime.h>
 
 #include "../../include/pbf_gb300.h"
+#include "pbf_device.cuh"
 #include "pbf_kernels.h"
 
 namespace {
 
 constexpr int kMaxHalf = 16;          // MaxFilterSize 32 >> 1
 constexpr int kFilterX = 128;         // texels per block of the x pass
-constexpr int kFilterYRows = 64;      // rows per block of the y pass
+constexpr int kFilterYRows = 64;      // rows per block of the y pass, at most
 constexpr double kFix = 1099511627776.0;  // 2^40
 
-__constant__ float c_gauss[kMaxHalf + 1];
+struct Gauss {
+  float w[kMaxHalf + 1];  // the filter's weights by distance
+};
 
 struct Cam {
   float v[16];  // view, column-major
@@ -185,9 +188,12 @@ __device__ inline float splat_exp(float x) {
 
 __device__ inline uint32_t depth_bits(float d) { return __float_as_uint(d); }
 
+// Also clears the words of `zero` (the volume tiles' counts and the scan's
+// scratch).
 __global__ void k_init(const float* scene, unsigned long long* keys, unsigned long long* acc, int W, int H, int W2,
-                       int H2) {
+                       int H2, uint32_t* zero, uint32_t words) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+  for (uint32_t q = y * gridDim.x * blockDim.x + x; q < words; q += gridDim.x * gridDim.y * blockDim.x) zero[q] = 0u;
   if (x >= W) return;
   const size_t p = (size_t)y * W + x;
   float s = scene ? scene[p] : 0.0f;
@@ -243,12 +249,19 @@ __device__ inline float gauss_axis(float n) { return splat_exp((n * n) * -2.0f);
 // tiles it touches, which changes nothing in the result.
 constexpr int kTile = 8;
 constexpr uint32_t kFirstShare = 16;
-constexpr uint32_t kFirstPer = 4;            // of them a warp takes at a time
-constexpr uint32_t kTwoPhaseMin = 1u << 15;  // particles from which the extra launches pay
+// The two phases and the volume sums by tile pay for their five extra launches
+// (about 25 us) and for the particles' second reading where there are many
+// particles and their sprites many pixels.  A frame at 2^20 particles (all at
+// once, tiled): 320 x 180 277 and 277 us, 960 x 540 351 and 327, 1280 x 720 437
+// and 367, 1920 x 1080 789 and 556; at 2^19 and 1920 x 1080 447 and 435, at 2^18
+// 289 and 312.
+constexpr uint32_t kTiledMin = 1u << 19;
+constexpr uint64_t kTiledWork = 1ull << 39;  // particles times pixels
 constexpr int kMaxTiles = 16;                // larger sprites are not tested
 
 __global__ void __launch_bounds__(256) k_tile_min(const unsigned long long* __restrict__ keys, int W, int H, int tw,
                                                   uint32_t* __restrict__ tile_min) {
+  pbf::chain_begin(keys);
   // one warp per tile, two pixels a lane
   const uint32_t lane = threadIdx.x & 31u, tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int tx = (int)tile % tw, ty = (int)tile / tw;
@@ -352,6 +365,7 @@ __device__ inline void volume_fragments(const Sprite& s, uint32_t lane, Add add)
 // tile's first place.
 __global__ void __launch_bounds__(256) k_volume_order(uint32_t n, const uint32_t* __restrict__ tile,
                                                       uint32_t* __restrict__ next, uint2* __restrict__ order) {
+  pbf::chain_begin(tile, next, order);
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
   const uint32_t t = q < n ? tile[q] : kNoTile;
   const unsigned peers = __match_any_sync(0xffffffffu, t);
@@ -382,6 +396,7 @@ __global__ void __launch_bounds__(kVolThreads) k_volume_sum(Cam C, const float4*
   constexpr uint32_t kPix = kVolWin * kVolWin;
   const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
   uint32_t* win = s_win + wib * kPix;
+  pbf::chain_begin(pos, order, total, acc);
   const uint32_t first = blockIdx.x * kVolRun, last = min(first + kVolRun, *total);
   if (first >= last) return;
   for (uint32_t p = lane; p < kPix; p += 32u) win[p] = 0u;
@@ -466,7 +481,7 @@ __global__ void __launch_bounds__(kVolThreads) k_volume_sum(Cam C, const float4*
 
 __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__ pos, uint32_t n, float R, int W, int H,
                                                int W2, int H2, unsigned long long* keys, unsigned long long* acc,
-                                               int phase, const uint32_t* __restrict__ tile_min, int tw,
+                                               int phase, uint32_t per, const uint32_t* __restrict__ tile_min, int tw,
                                                uint32_t* __restrict__ vol_tile, uint32_t* __restrict__ vol_count) {
   __shared__ SpriteSlot slots[8][32];
   __shared__ uint32_t qij[8][kQueue];
@@ -475,12 +490,13 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t lt = (1u << lane) - 1u;
-  // the first share is spread thin: four particles a warp
-  const uint32_t per = phase == kFirst ? kFirstPer : 32u, parts = 32u / per;
-  const uint64_t groups = ((uint64_t)n + 31u) / 32u;
-  const uint64_t items = phase == kFirst ? (groups + kFirstShare - 1u) / kFirstShare * parts : groups;
+  pbf::chain_begin(pos, keys, acc, tile_min, vol_tile, vol_count);
+  // `per` particles (a power of two) of a block of 32 a warp
+  const uint32_t parts = 32u / per;
+  const uint64_t stride = phase == kFirst ? kFirstShare * 32u : 32u;
+  const uint64_t items = ((uint64_t)n + stride - 1u) / stride * parts;
   for (uint64_t it = warp; it < items; it += warps) {
-    const uint64_t b = phase == kFirst ? it / parts * (kFirstShare * 32u) + it % parts * per : it * 32u;
+    const uint64_t b = it / parts * stride + it % parts * per;
     if (b >= n) continue;
     const uint32_t base = (uint32_t)b, q = base + lane;
     const bool first = (base / 32u) % kFirstShare == 0u;  // drawn in the first phase
@@ -539,7 +555,12 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
           }
         };
         const int w = s.i1 - s.i0;
-        if (w <= 32) {
+        const int rows1 = w <= 32 ? (int)((32u * c_recip16[w]) >> 16) : 0;
+        if (w > 32 || s.j1 - s.j0 <= rows1) {  // one step, or rows of many
+          walk_sprite(s, lane, [&](int i, int j, bool in) {
+            consider(i, j, in && bound > *(volatile unsigned long long*)(keys + (size_t)j * W + i));
+          });
+        } else {
           // four steps' keys are read together: one at a time, each step of a
           // sprite waited for its read
           const uint32_t m = c_recip16[w];
@@ -555,10 +576,6 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
             for (int h = 0; h < 4; ++h)
               if (jb - lr + h * rows < s.j1) consider(i, jb + h * rows, bound > key[h]);
           }
-        } else {
-          walk_sprite(s, lane, [&](int i, int j, bool in) {
-            consider(i, j, in && bound > *(volatile unsigned long long*)(keys + (size_t)j * W + i));
-          });
         }
       }
       if (ok & 2u) {
@@ -577,6 +594,7 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
 __global__ void k_resolve(Cam C, const float4* __restrict__ pos, float R, int W, int H, int W2, int H2,
                           const unsigned long long* keys, const unsigned long long* acc, float* depth, float* scene,
                           float* volume) {
+  pbf::chain_begin(pos, keys, acc, depth, scene, volume);
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   if (x >= W) return;
   const size_t p = (size_t)y * W + x;
@@ -605,7 +623,8 @@ __global__ void k_resolve(Cam C, const float4* __restrict__ pos, float R, int W,
 
 // The narrow-range filter for one texel given its window v[0 .. 2 half]
 // (centre v[half]); false when the centre is not positive (no write).
-__device__ inline bool narrow_range(const float* v, int stride, int half, float threshold, float mu, float& result) {
+__device__ inline bool narrow_range(const Gauss& G, const float* v, int stride, int half, float threshold, float mu,
+                                    float& result) {
   const float center = v[half * stride];
   if (!(center > 0.0f)) return false;
   float value_sum = center, weight_sum = 1.0f;
@@ -613,7 +632,7 @@ __device__ inline bool narrow_range(const float* v, int stride, int half, float 
   const float bound_high = center + mu;
   for (int i = 1; i <= half; ++i) {
     float a = v[(half - i) * stride], b = v[(half + i) * stride];
-    const float g = c_gauss[i];
+    const float g = G.w[i];
     if (a < lo || b < lo) continue;
     a = a > hi ? bound_high : a;
     b = b > hi ? bound_high : b;
@@ -626,10 +645,12 @@ __device__ inline bool narrow_range(const float* v, int stride, int half, float 
   return true;
 }
 
-__global__ void __launch_bounds__(kFilterX) k_filter_x(const float* __restrict__ src, float* __restrict__ dst, int W,
-                                                      int H, int half, float threshold, float mu) {
+__global__ void __launch_bounds__(kFilterX) k_filter_x(const __grid_constant__ Gauss G, const float* __restrict__ src,
+                                                      float* __restrict__ dst, int W, int H, int half, float threshold,
+                                                      float mu) {
   __shared__ float row[kFilterX + 2 * kMaxHalf];
   const int x0 = blockIdx.x * kFilterX, y = blockIdx.y;
+  pbf::chain_begin(src, dst);
   const float* s = src + (size_t)y * W;
   for (int k = threadIdx.x; k < kFilterX + 2 * kMaxHalf; k += kFilterX)
     row[k] = s[min(max(x0 - kMaxHalf + k, 0), W - 1)];
@@ -637,23 +658,25 @@ __global__ void __launch_bounds__(kFilterX) k_filter_x(const float* __restrict__
   const int x = x0 + threadIdx.x;
   if (x >= W) return;
   float r;
-  dst[(size_t)y * W + x] = narrow_range(row + threadIdx.x, 1, half, threshold, mu, r) ? r : 0.0f;
+  dst[(size_t)y * W + x] = narrow_range(G, row + threadIdx.x, 1, half, threshold, mu, r) ? r : 0.0f;
 }
 
-__global__ void __launch_bounds__(256) k_filter_y(const float* __restrict__ src, float* __restrict__ dst, int W, int H,
-                                                  int half, float threshold, float mu) {
+__global__ void __launch_bounds__(256) k_filter_y(const __grid_constant__ Gauss G, const float* __restrict__ src,
+                                                  float* __restrict__ dst, int W, int H, int rows, int half,
+                                                  float threshold, float mu) {
   __shared__ float col[kFilterYRows + 2 * kMaxHalf][33];
-  const int x = blockIdx.x * 32 + threadIdx.x, y0 = blockIdx.y * kFilterYRows;
+  const int x = blockIdx.x * 32 + threadIdx.x, y0 = blockIdx.y * rows;
   const int xc = min(x, W - 1);
-  for (int k = threadIdx.y; k < kFilterYRows + 2 * kMaxHalf; k += 8)
+  pbf::chain_begin(src, dst);
+  for (int k = threadIdx.y; k < rows + 2 * kMaxHalf; k += 8)
     col[k][threadIdx.x] = src[(size_t)min(max(y0 - kMaxHalf + k, 0), H - 1) * W + xc];
   __syncthreads();
   if (x >= W) return;
-  for (int q = threadIdx.y; q < kFilterYRows; q += 8) {
+  for (int q = threadIdx.y; q < rows; q += 8) {
     const int y = y0 + q;
     if (y >= H) break;
     float r;
-    if (narrow_range(&col[q][threadIdx.x], 33, half, threshold, mu, r)) dst[(size_t)y * W + x] = r;
+    if (narrow_range(G, &col[q][threadIdx.x], 33, half, threshold, mu, r)) dst[(size_t)y * W + x] = r;
   }
 }
 
@@ -664,7 +687,7 @@ struct pbf_renderer {
   pbf_render_options opt{};
   pbf_camera cam{};
   bool has_cam = false;
-  float gauss[kMaxHalf + 1] = {};
+  Gauss gauss{};
   float* depth = nullptr;
   float* temp = nullptr;
   float* volume = nullptr;
@@ -710,64 +733,65 @@ void gauss_table(uint32_t filter_size, float* g) {
 }
 
 // TextureFilter.execute: x pass img -> temp, y pass temp -> img.
-cudaError_t launch_filter(const float* gauss, float* img, float* temp, int W, int H, uint32_t filter_size, float R,
+cudaError_t launch_filter(const Gauss& gauss, float* img, float* temp, int W, int H, uint32_t filter_size, float R,
                           cudaStream_t st) {
   if (filter_size < 2) return cudaSuccess;
-  cudaError_t e = cudaMemcpyToSymbolAsync(c_gauss, gauss, sizeof(float) * (kMaxHalf + 1), 0, cudaMemcpyHostToDevice,
-                                          st);
-  if (e != cudaSuccess) return e;
   const int half = (int)(filter_size >> 1);
-  k_filter_x<<<dim3((unsigned)((W + kFilterX - 1) / kFilterX), (unsigned)H), kFilterX, 0, st>>>(img, temp, W, H, half,
-                                                                                              R * 5.0f, R);
-  k_filter_y<<<dim3((unsigned)((W + 31) / 32), (unsigned)((H + kFilterYRows - 1) / kFilterYRows)), dim3(32, 8), 0,
-               st>>>(temp, img, W, H, half, R * 5.0f, R);
-  return cudaGetLastError();
+  const cudaError_t e = pbf::launch_chain(true, k_filter_x, dim3((unsigned)((W + kFilterX - 1) / kFilterX), (unsigned)H),
+                                          dim3(kFilterX), 0, st, gauss, img, temp, W, H, half, R * 5.0f, R);
+  if (e != cudaSuccess) return e;
+  // 64 rows a block read 1.5 texels per texel written, 16 rows 3: worth it where
+  // the blocks are too few for the device
+  const int rows = (int64_t)W * H < (1 << 20) ? 16 : kFilterYRows;
+  return pbf::launch_chain(true, k_filter_y, dim3((unsigned)((W + 31) / 32), (unsigned)((H + rows - 1) / rows)),
+                           dim3(32, 8), 0, st, gauss, temp, img, W, H, rows, half, R * 5.0f, R);
 }
 
 size_t volume_tiles(const pbf_renderer* r) {
   return (size_t)((r->W2 + kVolTile - 1) / kVolTile) * ((r->H2 + kVolTile - 1) / kVolTile);
 }
 
-// Workspace for n particles (12 bytes each; kept, grown as needed).
+// Workspace for n particles (12 bytes each; kept, grown as needed) and, per
+// renderer, the words that k_init clears: the tiles' counts, the scan's error
+// word, the tiles' places and the scan's scratch.
+size_t volume_places_at(const pbf_renderer* r) { return volume_tiles(r) + 2; }
+size_t volume_scratch_at(const pbf_renderer* r) { return (volume_places_at(r) + volume_tiles(r) + 1 + 63) / 64 * 64; }
+size_t volume_words(const pbf_renderer* r) {
+  return volume_scratch_at(r) + (pbf::scan_scratch_bytes(volume_tiles(r) + 1) + 3) / 4;
+}
+
 cudaError_t volume_workspace(pbf_renderer* r, uint32_t n, cudaStream_t st) {
-  const uint32_t cap = n;
   cudaError_t e = cudaSuccess;
-  if (!r->vol_count) {
-    const size_t m = volume_tiles(r) + 1;
-    // counts and the scan's error word, places, scratch
-    e = cudaMalloc(&r->vol_count, (2 * m + 1) * sizeof(uint32_t) + pbf::scan_scratch_bytes(m) + 256);
-    if (e != cudaSuccess) return e;
-  }
-  if (cap > r->vol_cap) {
+  if (!r->vol_count && (e = cudaMalloc(&r->vol_count, volume_words(r) * sizeof(uint32_t))) != cudaSuccess) return e;
+  if (n > r->vol_cap) {
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
     cudaFree(r->vol_tile);
     cudaFree(r->vol_order);
     r->vol_tile = nullptr;
     r->vol_order = nullptr;
     r->vol_cap = 0;
-    e = cudaMalloc(&r->vol_tile, (size_t)cap * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&r->vol_order, (size_t)cap * sizeof(uint2));
-    if (e == cudaSuccess) r->vol_cap = cap;
+    e = cudaMalloc(&r->vol_tile, (size_t)n * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&r->vol_order, (size_t)n * sizeof(uint2));
+    if (e == cudaSuccess) r->vol_cap = n;
   }
   return e;
 }
 
-uint32_t* volume_places(const pbf_renderer* r) { return r->vol_count + volume_tiles(r) + 2; }
-
 // The volume sprites summed by tile, once the splat has found their tiles.
 cudaError_t volume_by_tile(pbf_renderer* r, const Cam& C, const float4* pos, uint32_t n, float R, cudaStream_t st) {
   const size_t m = volume_tiles(r) + 1;
-  uint32_t *err = r->vol_count + m, *place = volume_places(r);
-  char* scratch = reinterpret_cast<char*>(((uintptr_t)(place + m) + 255) / 256 * 256);
-  const cudaError_t e = pbf::launch_exclusive_scan(r->vol_count, place, m, scratch, err, st);
-  if (e != cudaSuccess) return e;
+  uint32_t *err = r->vol_count + m, *place = r->vol_count + volume_places_at(r);
+  cudaError_t e = pbf::launch_exclusive_scan_cleared(r->vol_count, place, m, r->vol_count + volume_scratch_at(r), err, st,
+                                                     pbf::ScanExtra{}, true);
   // (entry m - 1 of the counts is 0: its place is the total and stays it)
-  k_volume_order<<<(n + 255) / 256, 256, 0, st>>>(n, r->vol_tile, place, r->vol_order);
-  if (cudaFuncSetAttribute(k_volume_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVolSmem) != cudaSuccess)
-    return cudaGetLastError();
-  k_volume_sum<<<(n + kVolRun - 1) / kVolRun, kVolThreads, kVolSmem, st>>>(
-      C, pos, R, r->W2, r->H2, (r->W2 + kVolTile - 1) / kVolTile, r->vol_order, place + (m - 1), r->acc);
-  return cudaGetLastError();
+  if (e == cudaSuccess)
+    e = pbf::launch_chain(true, k_volume_order, (n - 1u) / 256u + 1u, 256, 0, st, n, r->vol_tile, place, r->vol_order);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_volume_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVolSmem);
+  if (e == cudaSuccess)
+    e = pbf::launch_chain(true, k_volume_sum, (n - 1u) / kVolRun + 1u, kVolThreads, kVolSmem, st, C, pos, R, r->W2, r->H2,
+                          (r->W2 + kVolTile - 1) / kVolTile, r->vol_order, place + (m - 1), r->acc);
+  return e;
 }
 
 bool finite16(const float* m) {
@@ -831,7 +855,7 @@ int pbf_renderer_set_config(pbf_renderer* r, const pbf_render_options* o) {
       !std::isfinite(o->particle_radius))
     return PBF_EINVAL;
   r->opt = *o;
-  gauss_table(o->filter_size, r->gauss);
+  gauss_table(o->filter_size, r->gauss.w);
   return PBF_OK;
 }
 
@@ -857,31 +881,47 @@ int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_s
   const float4* pos = (const float4*)d_positions;
   cudaEventRecord(r->ev[0], st);
   const dim3 rows((unsigned)((r->W + 255) / 256), (unsigned)r->H);
-  k_init<<<rows, 256, 0, st>>>(d_scene_depth, r->keys, r->acc, r->W, r->H, r->W2, r->H2);
+  bool tiled = n >= kTiledMin && (uint64_t)r->W * r->H * n >= kTiledWork;
+  if (tiled && volume_workspace(r, n, st) != cudaSuccess) {
+    cudaGetLastError();  // without the workspace, everything is drawn at once
+    tiled = false;
+  }
+  k_init<<<rows, 256, 0, st>>>(d_scene_depth, r->keys, r->acc, r->W, r->H, r->W2, r->H2, r->vol_count,
+                               tiled ? (uint32_t)volume_words(r) : 0u);
+  cudaError_t e = cudaSuccess;
   if (n) {
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const auto blocks = [&](uint64_t warps) { return (unsigned)std::min<uint64_t>((warps + 7) / 8, (uint64_t)sms * 8); };
-    const uint64_t groups = ((uint64_t)n + 31) / 32;
     const int tw = (r->W + kTile - 1) / kTile, th = (r->H + kTile - 1) / kTile;
-    auto splat = [&](int phase, uint64_t warps) {
-      k_splat<<<blocks(warps), 256, 0, st>>>(C, pos, n, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc, phase, r->tile_min,
-                                             tw, r->vol_tile, r->vol_count);
+    auto splat = [&](int phase, uint64_t particles) {
+      // Few particles are spread over the device, as a warp walks its own one
+      // after another (8000 at 1920 x 1080, a frame: 32 a warp 219 us, 2 a warp
+      // 73); many are taken in blocks that set their sprites up with most lanes
+      // (2^20 at 320 x 180: 2 a warp 541 us, 16 a warp 291).  Between, finer is
+      // also more even: 2^18 at 1920 x 1080 433 us with 32, 321 with 8.
+      uint32_t per = phase == kRest ? 32 : phase == kFirst ? 4 : n >= kTiledMin ? 16 : 8;
+      while (phase == kAll && per > 1 && particles < (uint64_t)sms * 32 * per) per /= 2;
+      const uint64_t warps = (particles + per - 1) / per;
+      return pbf::launch_chain(true, k_splat, (unsigned)((warps + 7) / 8), 256, 0, st, C, pos, n, R, r->W,
+                               r->H, r->W2, r->H2, r->keys, r->acc, phase, per, r->tile_min, tw, r->vol_tile,
+                               r->vol_count);
     };
-    if (n < kTwoPhaseMin || volume_workspace(r, n, st) != cudaSuccess) {
-      cudaGetLastError();  // (without the workspace, everything is drawn at once)
-      splat(kAll, groups);
+    if (!tiled) {
+      e = splat(kAll, n);
     } else {
-      if (cudaMemsetAsync(r->vol_count, 0, (volume_tiles(r) + 2) * sizeof(uint32_t), st) != cudaSuccess) return PBF_ECUDA;
-      splat(kFirst, (groups + kFirstShare - 1) / kFirstShare * (32 / kFirstPer));
-      k_tile_min<<<(unsigned)(((uint64_t)tw * th + 7) / 8), 256, 0, st>>>(r->keys, r->W, r->H, tw, r->tile_min);
-      splat(kRest, groups);
-      if (volume_by_tile(r, C, pos, n, R, st) != cudaSuccess) return PBF_ECUDA;
+      e = splat(kFirst, ((uint64_t)n + kFirstShare - 1) / kFirstShare);
+      if (e == cudaSuccess)
+        e = pbf::launch_chain(true, k_tile_min, (unsigned)(((uint64_t)tw * th + 7) / 8), 256, 0, st, r->keys, r->W, r->H,
+                              tw, r->tile_min);
+      if (e == cudaSuccess) e = splat(kRest, n);
+      if (e == cudaSuccess) e = volume_by_tile(r, C, pos, n, R, st);
     }
   }
-  k_resolve<<<rows, 256, 0, st>>>(C, pos, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc, r->depth, d_scene_depth,
-                                  r->volume);
+  if (e == cudaSuccess)
+    e = pbf::launch_chain(true, k_resolve, rows, 256, 0, st, C, pos, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc, r->depth,
+                          d_scene_depth, r->volume);
+  if (e != cudaSuccess) return PBF_ECUDA;
   cudaEventRecord(r->ev[1], st);
   if (launch_filter(r->gauss, r->depth, r->temp, r->W, r->H, r->opt.filter_size, R, st) != cudaSuccess)
     return PBF_ECUDA;
@@ -899,8 +939,8 @@ int pbf_texture_filter(const pbf_render_options* o, float* d_texture, uint32_t w
     return PBF_EINVAL;
   if (o->filter_size < 2 || width == 0 || height == 0) return PBF_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  float g[kMaxHalf + 1];
-  gauss_table(o->filter_size, g);
+  Gauss g;
+  gauss_table(o->filter_size, g.w);
   float* temp = nullptr;
   if (cudaMallocAsync(&temp, (size_t)width * height * sizeof(float), st) != cudaSuccess) return PBF_ECUDA;
   cudaError_t e = launch_filter(g, d_texture, temp, (int)width, (int)height, o->filter_size, o->particle_radius, st);
