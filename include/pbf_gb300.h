@@ -357,10 +357,11 @@ const char* pbf_ns_last_error(const pbf_ns* ns);
 /* Per-phase device times of pbf_ns_run (no counterpart in the reference):
  * when enabled, each run records CUDA events on the context's stream and
  * pbf_ns_timings returns the last run's phases in milliseconds after
- * synchronising: [0] cell keys (ParticleInsert), [1] the stable radix-sort
- * passes (CountingSort; the last one also counts the cells), [2] cell
- * offsets (ExclusiveScan of the counts), [3] outputs (ranks, copies of
- * counts, offsets and order).  PBF_ESTATE before a timed run. */
+ * synchronising: [0] cell keys (ParticleInsert) and the first digit counts,
+ * [1] the stable radix-sort passes (CountingSort; the last one also counts the
+ * cells and writes the order), [2] cell offsets (ExclusiveScan of the counts;
+ * it writes the caller's counts and offsets too), [3] ranks.  PBF_ESTATE
+ * before a timed run. */
 int pbf_ns_set_timing(pbf_ns* ns, int enable);
 int pbf_ns_timings(pbf_ns* ns, float ms[4]);
 

@@ -436,8 +436,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
     const ClearArgs clear{(uint32_t*)h->scan_scratch,
                           (uint32_t)(scan_scratch_bytes((size_t)g.cells + 1) / sizeof(uint32_t)), h->big_count.p,
                           h->band_count.p};
-    launch_chain(early, ps.predict, grid_of(h, n), h->blk, 0, st, p, g, h->tab, h->pos[c].p, h->vel.p, h->acc.p, h->xs[1].p,
-                 h->key.p, h->rank.p, counts, clear);
+    launch_chain(early, ps.predict, grid_of(h, n), h->blk, 0, st, p, g, h->tab, h->pos[c].p, h->vel.p, h->acc.p,
+                 h->xs[1].p, h->key.p, h->rank.p, counts, clear);
   }
   CU(h, cudaGetLastError());
   if (ev) CU(h, cudaEventRecord(ev[1], st));
@@ -548,11 +548,11 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   } else {
     KScope ks(h, K_NBR_BUILD);
     if (h->build == PBF_BUILD_PAIR)
-      launch_chain(early, ps.nbr_build2, grid_of(h, (n + 1) / 2), h->blk, 0, st, p, g, h->tab, h->xs[0].p, h->cell_start.p,
-                   ms, h->nbr_list.p, h->nbr_count.p, h->nbr_max.p, h->err_word.p);
+      launch_chain(early, ps.nbr_build2, grid_of(h, (n + 1) / 2), h->blk, 0, st, p, g, h->tab, h->xs[0].p,
+                   h->cell_start.p, ms, h->nbr_list.p, h->nbr_count.p, h->nbr_max.p, h->err_word.p);
     else if (h->build == PBF_BUILD_WARP)
-      launch_chain(early, ps.nbr_build_warp, grid_of(h, n), h->blk, 0, st, p, g, h->tab, h->xs[0].p, h->cell_start.p, ms,
-                   h->nbr_list.p, h->nbr_count.p, h->nbr_max.p, h->err_word.p);
+      launch_chain(early, ps.nbr_build_warp, grid_of(h, n), h->blk, 0, st, p, g, h->tab, h->xs[0].p, h->cell_start.p,
+                   ms, h->nbr_list.p, h->nbr_count.p, h->nbr_max.p, h->err_word.p);
     else
       launch_chain(early, ps.nbr_build, grid_of(h, n), h->blk, 0, st, p, g, h->tab, h->xs[0].p, h->cell_start.p, ms,
                    h->nbr_list.p, h->nbr_count.p, h->nbr_max.p, h->err_word.p);
@@ -798,14 +798,14 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   } else if (ps.xsph_split) {  // fast mode: XSPH's sum split over the two passes
     {
       KScope ks(h, K_VORTICITY);
-      launch_chain(early, ps.vorticity_split, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->vel.p, ms, h->nbr_count.p,
-                   h->nbr_list.p, h->omega.p, h->normal.p, h->visc.p, h->coh.p);
+      launch_chain(early, ps.vorticity_split, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->vel.p, ms,
+                   h->nbr_count.p, h->nbr_list.p, h->omega.p, h->normal.p, h->visc.p, h->coh.p);
     }
     CU(h, cudaGetLastError());
     {
       KScope ks(h, K_XSPH);
-      launch_chain(early, ps.xsph_split, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->omega.p, h->normal.p, h->visc.p,
-                   h->coh.p, ms, h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
+      launch_chain(early, ps.xsph_split, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->omega.p, h->normal.p,
+                   h->visc.p, h->coh.p, ms, h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
     }
     CU(h, cudaGetLastError());
   } else {
@@ -918,7 +918,8 @@ void release_all(pbf_handle* h) {
                          &h->omega,  &h->normal, &h->dp,    &h->out_pos, &h->out_tmp, &h->xs0};
   for (auto* b : f4s) b->release();
   DBuf<uint32_t>* u32s[] = {&h->ids[0],   &h->ids[1],      &h->key,      &h->rank,      &h->perm_raw,
-                            &h->id_raw,   &h->perm,        &h->tmp_a,    &h->tmp_b,     &h->cell_count[0], &h->cell_count[1],
+                            &h->id_raw,   &h->perm,        &h->tmp_a,    &h->tmp_b,     &h->cell_count[0],
+                            &h->cell_count[1],
                             &h->cell_start, &h->big_list,  &h->big_count, &h->nbr_count, &h->nbr_max,
                             &h->nbr_list, &h->err_word,    &h->m_u,      &h->skey,      &h->cb_mask};
   for (auto* b : u32s) b->release();

@@ -693,7 +693,8 @@ int pbf_mlp_train(pbf_mlp* m, const float* feat, const float* target, uint32_t r
   for (uint64_t r0 = 0; r0 < rows && e == cudaSuccess; r0 += chunk) {
     const uint32_t c = (uint32_t)(rows - r0 < chunk ? rows - r0 : chunk);
     e = cudaMemcpyAsync(at(oRawF), feat + 8 * r0, (size_t)c * 8 * sizeof(float), cudaMemcpyHostToDevice, 0);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(at(oRawT), target + r0, (size_t)c * sizeof(float), cudaMemcpyHostToDevice, 0);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(at(oRawT), target + r0, (size_t)c * sizeof(float), cudaMemcpyHostToDevice, 0);
     if (e == cudaSuccess) {
       k_place_rows<<<(c + 255) / 256, 256, 0, 0>>>((const float4*)at(oRawF), at(oRawT), dInv, (uint32_t)r0, c,
                                                    (float4*)dF, dT);

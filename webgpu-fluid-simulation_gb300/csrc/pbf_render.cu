@@ -37,6 +37,11 @@
 // exponential is this file's own (splat_exp), so the CPU restatement can
 // produce the same bits.
 //
+// Many particles on a large map are drawn in two phases: a share of the depth
+// sprites, then everything else behind a depth test per 8 x 8 tile, with the
+// small volume sprites sorted by tile and summed in shared memory.  Fewer are
+// drawn at once, 1 to 16 of them a warp.  Neither changes a bit of the result.
+//
 // The filter is the reference's narrow-range filter, separable, x then y,
 // with its sample window of 32 + 32 texels per 32-texel block: the centre it
 // reads for texel p is p - (16 - filterSize/2), so filter sizes below 32
@@ -385,9 +390,10 @@ constexpr uint32_t kVolThreads = 32 * kVolWarps;
 constexpr size_t kVolSmem = sizeof(uint32_t) * kVolWarps * kVolWin * kVolWin;
 static_assert(kVolPer < 64, "32-bit sums");
 
-__global__ void __launch_bounds__(kVolThreads) k_volume_sum(Cam C, const float4* __restrict__ pos, float R, int W2, int H2,
-                                                            int vw, const uint2* __restrict__ order,
-                                                            const uint32_t* __restrict__ total, unsigned long long* acc) {
+__global__ void __launch_bounds__(kVolThreads) k_volume_sum(Cam C, const float4* __restrict__ pos, float R, int W2,
+                                                            int H2, int vw, const uint2* __restrict__ order,
+                                                            const uint32_t* __restrict__ total,
+                                                            unsigned long long* acc) {
   extern __shared__ uint32_t s_win[];
   __shared__ uint32_t s_end;
   constexpr uint32_t kPix = kVolWin * kVolWin;
@@ -694,8 +700,8 @@ struct pbf_renderer {
   unsigned long long* keys = nullptr;
   unsigned long long* acc = nullptr;
   uint32_t* tile_min = nullptr;
-  // volume sprites by tile, for up to vol_cap particles: tile per particle,
-  // order, then counts, places and the scan's scratch
+  // volume sprites by tile, for up to vol_cap particles: tile and rank in it
+  // per particle, order, then counts, places and the scan's scratch
   uint32_t vol_cap = 0;
   uint2* vol_tile = nullptr;
   uint2* vol_order = nullptr;
@@ -737,8 +743,9 @@ cudaError_t launch_filter(const Gauss& gauss, float* img, float* temp, int W, in
                           cudaStream_t st) {
   if (filter_size < 2) return cudaSuccess;
   const int half = (int)(filter_size >> 1);
-  const cudaError_t e = pbf::launch_chain(true, k_filter_x, dim3((unsigned)((W + kFilterX - 1) / kFilterX), (unsigned)H),
-                                          dim3(kFilterX), 0, st, gauss, img, temp, W, H, half, R * 5.0f, R);
+  const dim3 segments((unsigned)((W + kFilterX - 1) / kFilterX), (unsigned)H);
+  const cudaError_t e = pbf::launch_chain(true, k_filter_x, segments, dim3(kFilterX), 0, st, gauss, img, temp, W, H, half,
+                                          R * 5.0f, R);
   if (e != cudaSuccess) return e;
   // 64 rows a block read 1.5 texels per texel written, 16 rows 3: worth it where
   // the blocks are too few for the device
@@ -781,16 +788,17 @@ cudaError_t volume_workspace(pbf_renderer* r, uint32_t n, cudaStream_t st) {
 cudaError_t volume_by_tile(pbf_renderer* r, const Cam& C, const float4* pos, uint32_t n, float R, cudaStream_t st) {
   const size_t m = volume_tiles(r) + 1;
   uint32_t *err = r->vol_count + m, *place = r->vol_count + volume_places_at(r);
-  cudaError_t e = pbf::launch_exclusive_scan_cleared(r->vol_count, place, m, r->vol_count + volume_scratch_at(r), err, st,
-                                                     pbf::ScanExtra{}, true);
+  uint32_t* scratch = r->vol_count + volume_scratch_at(r);
+  cudaError_t e =
+      pbf::launch_exclusive_scan_cleared(r->vol_count, place, m, scratch, err, st, pbf::ScanExtra{}, true);
   // (entry m - 1 of the counts is 0: its place is the total and stays it)
   if (e == cudaSuccess)
     e = pbf::launch_chain(true, k_volume_order, (n - 1u) / 256u + 1u, 256, 0, st, n, r->vol_tile, place, r->vol_order);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_volume_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVolSmem);
   if (e == cudaSuccess)
-    e = pbf::launch_chain(true, k_volume_sum, (n - 1u) / kVolRun + 1u, kVolThreads, kVolSmem, st, C, pos, R, r->W2, r->H2,
-                          (r->W2 + kVolTile - 1) / kVolTile, r->vol_order, place + (m - 1), r->acc);
+    e = pbf::launch_chain(true, k_volume_sum, (n - 1u) / kVolRun + 1u, kVolThreads, kVolSmem, st, C, pos, R, r->W2,
+                          r->H2, (r->W2 + kVolTile - 1) / kVolTile, r->vol_order, place + (m - 1), r->acc);
   return e;
 }
 
@@ -912,15 +920,15 @@ int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_s
     } else {
       e = splat(kFirst, ((uint64_t)n + kFirstShare - 1) / kFirstShare);
       if (e == cudaSuccess)
-        e = pbf::launch_chain(true, k_tile_min, (unsigned)(((uint64_t)tw * th + 7) / 8), 256, 0, st, r->keys, r->W, r->H,
-                              tw, r->tile_min);
+        e = pbf::launch_chain(true, k_tile_min, (unsigned)(((uint64_t)tw * th + 7) / 8), 256, 0, st, r->keys, r->W,
+                              r->H, tw, r->tile_min);
       if (e == cudaSuccess) e = splat(kRest, n);
       if (e == cudaSuccess) e = volume_by_tile(r, C, pos, n, R, st);
     }
   }
   if (e == cudaSuccess)
-    e = pbf::launch_chain(true, k_resolve, rows, 256, 0, st, C, pos, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc, r->depth,
-                          d_scene_depth, r->volume);
+    e = pbf::launch_chain(true, k_resolve, rows, 256, 0, st, C, pos, R, r->W, r->H, r->W2, r->H2, r->keys, r->acc,
+                          r->depth, d_scene_depth, r->volume);
   if (e != cudaSuccess) return PBF_ECUDA;
   cudaEventRecord(r->ev[1], st);
   if (launch_filter(r->gauss, r->depth, r->temp, r->W, r->H, r->opt.filter_size, R, st) != cudaSuccess)

@@ -1,8 +1,8 @@
 // pbf_sort.cu — integer pipeline of the neighbour search: single-pass
 // decoupled look-back exclusive scan, counting-sort scatter, stable
 // within-cell order by particle id, the stable LSD radix sort of the
-// stand-alone search, state gather, id-order export and the per-step
-// metrics reduction.
+// stand-alone search, the state moved along with the order, id-order export
+// and the per-step metrics reduction.
 //
 // Reference counterparts (relative to the reference root):
 //   ExclusiveScan.execute + scanShader.ts  src/simulator/neighbor/exclusiveScan.ts:134-166,
@@ -935,7 +935,8 @@ cudaError_t launch_sort_by_cell(GridParams g, uint32_t n, const uint32_t* ids, S
                                                       b.err, st, ScanExtra{b.count_next}, early);
   if (e != cudaSuccess) return e;
   if (n == 0) return cudaSuccess;
-  e = launch_chain(early, k_scatter, blocks_for(n, 256), 256, 0, st, n, b.key, b.rank, b.cell_start, ids, b.perm_raw, b.id_raw);
+  e = launch_chain(early, k_scatter, blocks_for(n, 256), 256, 0, st, n, b.key, b.rank, b.cell_start, ids, b.perm_raw,
+                   b.id_raw);
   if (e != cudaSuccess) return e;
   int passes = (int)((id_bits + 7) / 8);
   if (passes < 1) passes = 1;

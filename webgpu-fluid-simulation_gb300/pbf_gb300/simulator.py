@@ -505,8 +505,8 @@ class NeighborSearch:
         self._check(self._lib.pbf_ns_set_timing(self._h, 1 if enable else 0), "pbf_ns_set_timing")
 
     def timings(self):
-        """The last timed run's phases in ms: [cell keys + counts, scan of the
-        counts, counting-sort reorder, outputs]."""
+        """The last timed run's phases in ms: [cell keys and first digit counts,
+        sort passes, cell offsets, ranks]."""
         ms = (ctypes.c_float * 4)()
         self._check(self._lib.pbf_ns_timings(self._h, ms), "pbf_ns_timings")
         return [float(x) for x in ms]
