@@ -363,6 +363,17 @@ void prefer_l1(const PassSet& ps) {
       cudaGetLastError();  // a hint only
 }
 
+// The passes with several lanes a slot, for the plain solve of a small scene;
+// null where one lane a slot is as fast.  Exact mode, four iterations, two
+// substeps, graph replay: 2,197 slots one / four / eight lanes 250 / 148 / 117
+// us (three handles at once 87 / 52 / 42 each), 8,000 slots 305 / 177 / 144 (105
+// / 66 / 59), 27,000 slots 340 / 214 / 238 (133 / 115 / 136); at 68,921 slots the
+// device is full and more lanes only add work: 413 / 421 (214 / 285).
+const LaneSet* lane_set(const PassSet& ps, uint32_t n) {
+  const LaneSet& s = ps.lanes[n <= (1u << 14) ? 0 : 1];
+  return s.lanes && n <= (1u << 15) ? &s : nullptr;
+}
+
 void invalidate_graph(pbf_handle* h) {
   for (auto& g : h->graphs) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -465,6 +476,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   const FieldParams f = h->fp;
   const uint32_t ms = h->nbr_slice;
   const float sub_index = (float)(h->substep_counter % h->cfg.substeps);
+  const LaneSet* ls = (!cb && !h->learned && h->trace_cap == 0) ? lane_set(ps, n) : nullptr;
+  const unsigned walk_grid = ls ? nblocks(n * ls->lanes, h->blk) : grid_of(h, n);
   // Boundary sampling works on a band list (BandArgs): the
   // band pass builds it at x*_0, each delta-p pass marks the band of the next
   // iteration at the positions it writes, and the sampling kernel interpolates
@@ -612,8 +625,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
           auto kl = fe ? cs.lambda_feat : (al.stats && adaptive ? cs.lambda_stats : cs.lambda);
           kl<<<cbg, 128, cb_smem(h, 1), st>>>(p, A, f.loaded, h->bdata.p, h->xs[a].p, h->xl.p, al);
         } else {
-          auto kl = fe ? ps.lambda_feat : (al.stats && adaptive ? ps.lambda_stats : ps.lambda);
-          launch_chain(early, kl, grid_of(h, n), h->blk, 0, st, p, f.loaded, h->bdata.p, h->xs[a].p, ms, h->nbr_count.p,
+          auto kl = ls ? ls->lambda : fe ? ps.lambda_feat : (al.stats && adaptive ? ps.lambda_stats : ps.lambda);
+          launch_chain(early, kl, walk_grid, h->blk, 0, st, p, f.loaded, h->bdata.p, h->xs[a].p, ms, h->nbr_count.p,
                        h->nbr_list.p, h->xl.p, al);
         }
       }
@@ -642,8 +655,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
           cs.deltap<<<cbg, 128, cb_smem(h, 1), st>>>(p, A, ad, f.loaded, h->xl.p, h->bdata.p, h->xs[1 - a].p,
                                                      h->capture ? h->dp.p : nullptr);
         else
-          launch_chain(early, ps.deltap, grid_of(h, n), h->blk, 0, st, p, ad, f.loaded, h->xl.p, h->bdata.p, ms,
-                       h->nbr_count.p, h->nbr_list.p, h->xs[1 - a].p, h->capture ? h->dp.p : nullptr);
+          launch_chain(early, ls ? ls->deltap : ps.deltap, walk_grid, h->blk, 0, st, p, ad, f.loaded, h->xl.p,
+                       h->bdata.p, ms, h->nbr_count.p, h->nbr_list.p, h->xs[1 - a].p, h->capture ? h->dp.p : nullptr);
       }
       if (cudaGetLastError() != cudaSuccess) { *rc = PBF_ECUDA; return a; }
       a = 1 - a;
@@ -712,8 +725,8 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
       cs.density_velocity<<<cbg, 128, cb_smem(h, 1), st>>>(p, A, ad, h->xs[a].p, h->pos[cc].p, h->vel.p,
                                                             cb_memb(h) == kMemMaskHost ? nullptr : h->nbr_count.p);
     else
-      launch_chain(early, ps.density_velocity, grid_of(h, n), h->blk, 0, st, p, ad, h->xs[a].p, ms, h->nbr_count.p,
-                   h->nbr_list.p, h->pos[cc].p, h->vel.p);
+      launch_chain(early, ls ? ls->density_velocity : ps.density_velocity, walk_grid, h->blk, 0, st, p, ad, h->xs[a].p,
+                   ms, h->nbr_count.p, h->nbr_list.p, h->pos[cc].p, h->vel.p);
   }
   CU(h, cudaGetLastError());
   if (rec) CU(h, launch_stats_record(h->stats.p, h->trace_err.p, st));
@@ -811,14 +824,14 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   } else {
     {
       KScope ks(h, K_VORTICITY);
-      launch_chain(early, ps.vorticity, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->vel.p, ms, h->nbr_count.p,
-                   h->nbr_list.p, h->omega.p, h->normal.p);
+      launch_chain(early, ls ? ls->vorticity : ps.vorticity, walk_grid, h->blk, 0, st, p, h->pos[cc].p, h->vel.p, ms,
+                   h->nbr_count.p, h->nbr_list.p, h->omega.p, h->normal.p);
     }
     CU(h, cudaGetLastError());
     {
       KScope ks(h, K_XSPH);
-      launch_chain(early, ps.xsph, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->vel.p, h->omega.p, h->normal.p, ms,
-                   h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
+      launch_chain(early, ls ? ls->xsph : ps.xsph, walk_grid, h->blk, 0, st, p, h->pos[cc].p, h->vel.p, h->omega.p,
+                   h->normal.p, ms, h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
     }
     CU(h, cudaGetLastError());
   }

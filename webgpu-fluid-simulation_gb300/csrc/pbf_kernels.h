@@ -36,6 +36,21 @@ cudaError_t launch_chain(bool early, void (*kernel)(P...), dim3 grid, dim3 block
 // within the noise (2215, 2208), and 16 batched scenes got 1 % slower.
 constexpr uint32_t kEarlyMax = 1u << 18;
 
+// The neighbour passes with several lanes a slot, for small scenes.
+struct LaneSet {
+  uint32_t lanes = 0;
+  void (*lambda)(SimParams, int, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*, float4*,
+                 SolverAux) = nullptr;
+  void (*deltap)(SimParams, SolverAux, int, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*,
+                 float4*, float4*) = nullptr;
+  void (*density_velocity)(SimParams, SolverAux, const float4*, uint32_t, const uint32_t*, const uint32_t*, float4*,
+                           float4*) = nullptr;
+  void (*vorticity)(SimParams, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*, float4*,
+                    float4*) = nullptr;
+  void (*xsph)(SimParams, const float4*, const float4*, const float4*, const float4*, uint32_t, const uint32_t*,
+               const uint32_t*, float4*, ExportArgs) = nullptr;
+};
+
 // The step's passes of one variant: single scene or batch (scene table),
 // one tile per CTA or persistent (grid-stride).
 struct PassSet {
@@ -66,6 +81,7 @@ struct PassSet {
                     float4*);
   void (*xsph)(SimParams, const float4*, const float4*, const float4*, const float4*, uint32_t, const uint32_t*,
                const uint32_t*, float4*, ExportArgs);
+  LaneSet lanes[2];  // more lanes first; lanes = 0 where not built
   // fast mode: XSPH's neighbour sum split over the vorticity and XSPH passes (null in exact mode)
   void (*vorticity_split)(SimParams, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*,
                           float4*, float4*, float4*, float4*);

@@ -569,6 +569,43 @@ __device__ __forceinline__ void for_each_neighbor2(const uint32_t* __restrict__ 
   }
 }
 
+// The walk shared by kL lanes: each evaluates every kL-th neighbour (load(j):
+// its records, term(records): its terms), and all add the terms up in list
+// order, handed round by shuffles.  A lane that finds no entry left evaluates
+// slot 0 and its terms are not taken.  The same additions of the same terms:
+// without FMA contraction (exact mode) the same bits as one lane's walk.
+template <class T>
+__device__ __forceinline__ T shfl_term(unsigned mates, const T& t, uint32_t from) {
+  constexpr int kN = sizeof(T) / sizeof(float);
+  T o;
+  const float* a = reinterpret_cast<const float*>(&t);
+  float* b = reinterpret_cast<float*>(&o);
+#pragma unroll
+  for (int k = 0; k < kN; ++k) b[k] = __shfl_sync(mates, a[k], (int)from);
+  return o;
+}
+template <int kL, class Load, class Term, class Take>
+__device__ __forceinline__ void walk_lanes(const uint32_t* __restrict__ list, uint32_t base, uint32_t cnt, Load&& load,
+                                           Term&& term, Take&& take) {
+  const uint32_t lane = threadIdx.x & 31u, sub = lane % kL, first = lane - sub;
+  const unsigned mates = (kL == 32 ? 0xffffffffu : (1u << kL) - 1u) << first;
+  const uint32_t* l = list + base;
+  auto index = [&](uint32_t q) { return q < cnt ? __ldcs(l + 32u * q) : 0u; };
+  auto rec = load(index(sub));
+  uint32_t j = index(kL + sub);
+  for (uint32_t q = 0; q < cnt; q += kL) {
+    const auto next = load(j);  // a batch's records and the indices after them are under way
+    j = index(q + 2u * kL + sub);
+    const auto mine = term(rec);
+#pragma unroll
+    for (uint32_t m = 0; m < kL; ++m) {
+      const auto t = shfl_term(mates, mine, first + m);
+      if (q + m < cnt) take(t);
+    }
+    rec = next;
+  }
+}
+
 // Whether the boundary sample of a particle can be non-zero: per field cell,
 // 0 when all 32 volume nodes are zero (the interpolated volume is then zero)
 // or the SDF provably stays >= h over the cell; then bData = 0 exactly.
@@ -730,13 +767,21 @@ struct LamSum {
     sum2 = 0.0f;
     dens = 0.0f;
   }
-  __device__ __forceinline__ void add(const SimParams& p, float4 xj) {
+  // one neighbour's terms, and their addition (apart for the lane walk)
+  struct Term {
+    f3 gk;
+    float w;
+  };
+  __device__ __forceinline__ Term term(const SimParams& p, float4 xj) const {
     Pair q = make_pair_of(xi - xyz(xj));
-    f3 gk = spiky_p(p, q);
-    grad = grad + gk;
-    sum2 = sum2 + dot3(gk, gk);
-    dens = dens + poly6_p(p, q);
+    return {spiky_p(p, q), poly6_p(p, q)};
   }
+  __device__ __forceinline__ void take(const Term& t) {
+    grad = grad + t.gk;
+    sum2 = sum2 + dot3(t.gk, t.gk);
+    dens = dens + t.w;
+  }
+  __device__ __forceinline__ void add(const SimParams& p, float4 xj) { take(term(p, xj)); }
 };
 // ConstrainSolve's sum (pressureConstrain.ts:127-141) over packed (x*_j, lambda_j).
 struct DpSum {
@@ -747,10 +792,15 @@ struct DpSum {
     li = xli.w;
     pu = mk(0.f, 0.f, 0.f);
   }
-  __device__ __forceinline__ void add(const SimParams& p, float4 xj) {
+  struct Term {
+    f3 pu;
+  };
+  __device__ __forceinline__ Term term(const SimParams& p, float4 xj) const {
     Pair q = make_pair_of(xi - xyz(xj));
-    pu = pu + (li + xj.w) * spiky_p(p, q);
+    return {(li + xj.w) * spiky_p(p, q)};
   }
+  __device__ __forceinline__ void take(const Term& t) { pu = pu + t.pu; }
+  __device__ __forceinline__ void add(const SimParams& p, float4 xj) { take(term(p, xj)); }
 };
 // AttributeUpdate's density sum (attributeUpdate.ts:40-49).
 struct DensSum {
@@ -760,10 +810,14 @@ struct DensSum {
     xi = x;
     dens = 0.0f;
   }
-  __device__ __forceinline__ void add(const SimParams& p, float4 xj) {
-    Pair q = make_pair_of(xi - xyz(xj));
-    dens = dens + poly6_p(p, q);
+  struct Term {
+    float w;
+  };
+  __device__ __forceinline__ Term term(const SimParams& p, float4 xj) const {
+    return {poly6_p(p, make_pair_of(xi - xyz(xj)))};
   }
+  __device__ __forceinline__ void take(const Term& t) { dens = dens + t.w; }
+  __device__ __forceinline__ void add(const SimParams& p, float4 xj) { take(term(p, xj)); }
 };
 // VorticityConfinement's sums (vorticityConfinement.ts:46-61): omega and the Akinci normal.
 struct VortSum {
@@ -774,14 +828,21 @@ struct VortSum {
     om = mk(0.f, 0.f, 0.f);
     nm = mk(0.f, 0.f, 0.f);
   }
-  __device__ __forceinline__ void add(const SimParams& p, float4 pj, float4 vj) {
+  struct Term {
+    f3 om, nm;
+  };
+  __device__ __forceinline__ Term term(const SimParams& p, float4 pj, float4 vj) const {
     Pair q = make_pair_of(xi - xyz(pj));
     f3 vd = xyz(vj) - vi;
     float volume = fdiv(p.m, pj.w);
     f3 gw = spiky_p(p, q);
-    om = om + volume * cross3(vd, gw);
-    nm = nm + volume * gw;
+    return {volume * cross3(vd, gw), volume * gw};
   }
+  __device__ __forceinline__ void take(const Term& t) {
+    om = om + t.om;
+    nm = nm + t.nm;
+  }
+  __device__ __forceinline__ void add(const SimParams& p, float4 pj, float4 vj) { take(term(p, pj, vj)); }
 };
 // XSPH + vorticity force + Akinci tension sums (XSPH.ts:57-81), single pass.
 struct XsphSum {
@@ -796,16 +857,26 @@ struct XsphSum {
     eta = mk(0.f, 0.f, 0.f);
     ten = mk(0.f, 0.f, 0.f);
   }
-  __device__ __forceinline__ void add(const SimParams& p, float4 pj, float4 vj, float4 nj) {
+  struct Term {
+    f3 vu, eta, ten;
+  };
+  __device__ __forceinline__ Term term(const SimParams& p, float4 pj, float4 vj, float4 nj) const {
     float rj = pj.w;
     Pair q = make_pair_of(xi - xyz(pj));
     f3 vd = xyz(vj) - vi;
     float kij = fdiv(p.two_rho0, ri + rj);
-    vu = vu + fdiv3(poly6_p(p, q) * vd, rj);
-    eta = eta + fdiv3(nj.w * spiky_p(p, q), rj);  // nj: (normal_j, |omega_j|)
     f3 coh = p.m * cohesion_p(p, q);
     f3 curv = ni - xyz(nj);
-    ten = ten - kij * (coh + curv);
+    return {fdiv3(poly6_p(p, q) * vd, rj), fdiv3(nj.w * spiky_p(p, q), rj),  // nj: (normal_j, |omega_j|)
+            kij * (coh + curv)};
+  }
+  __device__ __forceinline__ void take(const Term& t) {
+    vu = vu + t.vu;
+    eta = eta + t.eta;
+    ten = ten - t.ten;
+  }
+  __device__ __forceinline__ void add(const SimParams& p, float4 pj, float4 vj, float4 nj) {
+    take(term(p, pj, vj, nj));
   }
 };
 // Fast mode's split: the vorticity pass also sums XSPH's viscosity term and
@@ -1229,6 +1300,120 @@ __global__ void __launch_bounds__(256) k_xsph_split(SimParams p, const float4* _
   }
 }
 
+// The passes of a scene too small to fill the device, kL lanes a slot
+// (walk_lanes).  Exact mode: a neighbour's terms are long chains (IEEE square
+// roots and divisions), and with one lane a slot a pass took as long at 2,000
+// slots as at 69,000 (XSPH 65 us).
+struct Rec2 {
+  float4 a, b;
+};
+struct Rec3 {
+  float4 a, b, c;
+};
+
+template <uint32_t kL>
+__global__ void __launch_bounds__(256) k_lambda_lanes(SimParams p, int have_field, const float4* __restrict__ bdata,
+                                                      const float4* __restrict__ xs, uint32_t max_nbr,
+                                                      const uint32_t* __restrict__ nbr_cnt,
+                                                      const uint32_t* __restrict__ nbr_list, float4* __restrict__ xl,
+                                                      SolverAux a) {
+  chain_begin(bdata, xs, nbr_cnt, nbr_list, a.lam_sum);
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, t = g / kL;
+  if (t >= p.n) return;
+  uint32_t b, e;
+  list_slice(max_nbr, nbr_cnt, t, b, e);
+  LamSum acc;
+  acc.init(xyz(xs[t]));
+  walk_lanes<kL>(
+      nbr_list, b, e, [&](uint32_t j) { return __ldg(xs + j); }, [&](float4 xj) { return acc.term(p, xj); },
+      [&](const LamSum::Term& x) { acc.take(x); });
+  if (g % kL == 0) lambda_finish<0, false>(p, have_field, bdata, xl, a, t, acc, e);
+}
+
+template <uint32_t kL>
+__global__ void __launch_bounds__(256) k_deltap_lanes(SimParams p, SolverAux a, int have_field,
+                                                      const float4* __restrict__ xl, const float4* __restrict__ bdata,
+                                                      uint32_t max_nbr, const uint32_t* __restrict__ nbr_cnt,
+                                                      const uint32_t* __restrict__ nbr_list,
+                                                      float4* __restrict__ xs_out, float4* __restrict__ dp_out) {
+  chain_begin(xl, bdata, nbr_cnt, nbr_list);
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, t = g / kL;
+  if (t >= p.n) return;
+  uint32_t b, e;
+  list_slice(max_nbr, nbr_cnt, t, b, e);
+  DpSum acc;
+  acc.init(xl[t]);
+  walk_lanes<kL>(
+      nbr_list, b, e, [&](uint32_t j) { return __ldg(xl + j); }, [&](float4 xj) { return acc.term(p, xj); },
+      [&](const DpSum::Term& x) { acc.take(x); });
+  if (g % kL != 0) return;
+  const f3 dp = deltap_finish<false>(p, have_field, bdata, t, acc);
+  if (dp_out) dp_out[t] = f4(dp, 0.0f);
+  const f3 xn = clamp_rand(p, acc.xi + dp);
+  xs_out[t] = f4(xn, 0.0f);
+  if (a.band.list) band_mark<false>(p, a.band, a.tab, t, xn);
+}
+
+template <uint32_t kL>
+__global__ void __launch_bounds__(256) k_density_velocity_lanes(SimParams p, SolverAux, const float4* __restrict__ xs,
+                                                                uint32_t max_nbr, const uint32_t* __restrict__ nbr_cnt,
+                                                                const uint32_t* __restrict__ nbr_list,
+                                                                float4* __restrict__ pos, float4* __restrict__ vel) {
+  chain_begin(xs, nbr_cnt, nbr_list, pos);
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, t = g / kL;
+  if (t >= p.n) return;
+  uint32_t b, e;
+  list_slice(max_nbr, nbr_cnt, t, b, e);
+  DensSum acc;
+  acc.init(xyz(xs[t]));
+  walk_lanes<kL>(
+      nbr_list, b, e, [&](uint32_t j) { return __ldg(xs + j); }, [&](float4 xj) { return acc.term(p, xj); },
+      [&](const DensSum::Term& x) { acc.take(x); });
+  if (g % kL == 0) density_finish<false>(p, pos, vel, t, acc);
+}
+
+template <uint32_t kL>
+__global__ void __launch_bounds__(256) k_vorticity_lanes(SimParams p, const float4* __restrict__ pos,
+                                                         const float4* __restrict__ vel, uint32_t max_nbr,
+                                                         const uint32_t* __restrict__ nbr_cnt,
+                                                         const uint32_t* __restrict__ nbr_list,
+                                                         float4* __restrict__ omega, float4* __restrict__ normal) {
+  chain_begin(pos, vel, nbr_cnt, nbr_list);
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, t = g / kL;
+  if (t >= p.n) return;
+  uint32_t b, e;
+  list_slice(max_nbr, nbr_cnt, t, b, e);
+  VortSum acc;
+  acc.init(xyz(pos[t]), xyz(vel[t]));
+  walk_lanes<kL>(
+      nbr_list, b, e, [&](uint32_t j) { return Rec2{__ldg(pos + j), __ldg(vel + j)}; },
+      [&](const Rec2& r) { return acc.term(p, r.a, r.b); }, [&](const VortSum::Term& x) { acc.take(x); });
+  if (g % kL == 0) vorticity_finish(p, omega, normal, t, acc);
+}
+
+template <uint32_t kL>
+__global__ void __launch_bounds__(256) k_xsph_lanes(SimParams p, const float4* __restrict__ pos,
+                                                    const float4* __restrict__ vel, const float4* __restrict__ omega,
+                                                    const float4* __restrict__ normal, uint32_t max_nbr,
+                                                    const uint32_t* __restrict__ nbr_cnt,
+                                                    const uint32_t* __restrict__ nbr_list, float4* __restrict__ acc,
+                                                    ExportArgs ex) {
+  chain_begin(pos, vel, omega, normal, nbr_cnt, nbr_list, ex.id);
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, t = g / kL;
+  if (t >= p.n) return;
+  uint32_t b, e;
+  list_slice(max_nbr, nbr_cnt, t, b, e);
+  XsphSum s;
+  const float4 pi = pos[t];
+  s.init(pi, xyz(vel[t]), xyz(normal[t]));
+  walk_lanes<kL>(
+      nbr_list, b, e, [&](uint32_t j) { return Rec3{__ldg(pos + j), __ldg(vel + j), __ldg(normal + j)}; },
+      [&](const Rec3& r) { return s.term(p, r.a, r.b, r.c); }, [&](const XsphSum::Term& x) { s.take(x); });
+  if (g % kL != 0) return;
+  if (ex.id) ex.out[ex.id[t]] = pi;
+  xsph_finish(p, acc, t, s, xyz(omega[t]));
+}
+
 #include "pbf_cellblock.cuh"
 
 // Launch table for this precision variant: [batch][persistent] pass sets.
@@ -1248,6 +1433,20 @@ void fill_set(PassSet* ps) {
   ps->density_velocity = k_density_velocity<P>;
   ps->vorticity = k_vorticity<P>;
   ps->xsph = k_xsph<P>;
+  if constexpr (!kFast && !B && !P) {
+    ps->lanes[0] = LaneSet{8,
+                           k_lambda_lanes<8>,
+                           k_deltap_lanes<8>,
+                           k_density_velocity_lanes<8>,
+                           k_vorticity_lanes<8>,
+                           k_xsph_lanes<8>};
+    ps->lanes[1] = LaneSet{4,
+                           k_lambda_lanes<4>,
+                           k_deltap_lanes<4>,
+                           k_density_velocity_lanes<4>,
+                           k_vorticity_lanes<4>,
+                           k_xsph_lanes<4>};
+  }
   if constexpr (kFast) {
     ps->vorticity_split = k_vorticity_split<P>;
     ps->xsph_split = k_xsph_split<P>;
