@@ -1,5 +1,4 @@
-"""The neighbour passes with several lanes a slot (small scenes, exact mode)
-against the same passes with one lane a slot, bit for bit, at the sizes where
+"""The neighbour passes with several lanes a slot (small scenes) against the same passes with one lane a slot, bit for bit, at the sizes where
 the number of lanes changes and where a warp or block is partly filled."""
 import numpy as np
 import pytest
@@ -14,13 +13,15 @@ FIELDS = (L.FIELD_POSITION, L.FIELD_VELOCITY, L.FIELD_ACCELERATION, L.FIELD_PRED
 
 
 @pytest.mark.parametrize("field", [False, True])
-@pytest.mark.parametrize("n", [1, 2, 7, 9, 33, 1025, 1 << 14, (1 << 14) + 1, 1 << 15, (1 << 15) + 1])
-def test_lanes_equal_one_lane(n, field):
+@pytest.mark.parametrize("fp,n", [(L.FP_EXACT, n) for n in (1, 2, 7, 9, 33, 1025, 1 << 14, (1 << 14) + 1, 1 << 15,
+                                                            (1 << 15) + 1)] +
+                         [(L.FP_FAST, n) for n in (1, 9, 1025, 1 << 12, (1 << 12) + 1, 1 << 13, (1 << 13) + 1)])
+def test_lanes_equal_one_lane(fp, n, field):
     """Persistent grids (ctas_per_sm) take one lane a slot at every size."""
     rng = np.random.default_rng(n)
     sc = scenes.reference_scene("boundary_small")
     cfg = scenes.copy_config(sc.config)
-    cfg.fp_mode, cfg.max_particles, cfg.max_neighbors = L.FP_EXACT, n, 1024
+    cfg.fp_mode, cfg.max_particles, cfg.max_neighbors = fp, n, 1024
     side = 0.04 * max(n, 8) ** (1.0 / 3.0) * 0.5
     pts = np.zeros((n, 4), np.float32)
     pts[:, :3] = 0.5 + min(side, 0.9) * (rng.random((n, 3)) - 0.5)
@@ -33,7 +34,7 @@ def test_lanes_equal_one_lane(n, field):
             if field:
                 sim.set_boundary_field(f["res"], f["origin"], f["extent"], f["sdf"], f["vol"])
             sim.set_capture(True)
-            sim.step(1)
+            sim.step(2)
             sim.synchronize()
             out.append([sim.copy_field(q) for q in FIELDS])
     for a, b in zip(*out):

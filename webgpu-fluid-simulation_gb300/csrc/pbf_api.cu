@@ -364,14 +364,19 @@ void prefer_l1(const PassSet& ps) {
 }
 
 // The passes with several lanes a slot, for the plain solve of a small scene;
-// null where one lane a slot is as fast.  Exact mode, four iterations, two
-// substeps, graph replay: 2,197 slots one / four / eight lanes 250 / 148 / 117
-// us (three handles at once 87 / 52 / 42 each), 8,000 slots 305 / 177 / 144 (105
-// / 66 / 59), 27,000 slots 340 / 214 / 238 (133 / 115 / 136); at 68,921 slots the
-// device is full and more lanes only add work: 413 / 421 (214 / 285).
+// null where one lane a slot is as fast.  Four iterations, two substeps, graph
+// replay, one / four / eight lanes in us (three handles at once, each):
+//   exact  2,197 slots  250 / 148 / 117 (87 / 52 / 42)
+//          8,000        305 / 177 / 144 (105 / 66 / 59)
+//         27,000        340 / 214 / 238 (133 / 115 / 136)
+//         68,921        413 / 421 / 457 (214 / 285 / 365): the device is full
+//   fast   2,197        105 /  96 /  88 (39 / 35 / 33)
+//          8,000        124 / 114 / 111 (47 / 46 / 48)
+//         27,000        132 / 146 / 182 (58 / 76 / 104)
 const LaneSet* lane_set(const PassSet& ps, uint32_t n) {
-  const LaneSet& s = ps.lanes[n <= (1u << 14) ? 0 : 1];
-  return s.lanes && n <= (1u << 15) ? &s : nullptr;
+  for (const LaneSet& s : ps.lanes)
+    if (n <= s.max_n) return &s;
+  return nullptr;
 }
 
 void invalidate_graph(pbf_handle* h) {
@@ -811,13 +816,13 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   } else if (ps.xsph_split) {  // fast mode: XSPH's sum split over the two passes
     {
       KScope ks(h, K_VORTICITY);
-      launch_chain(early, ps.vorticity_split, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->vel.p, ms,
+      launch_chain(early, ls ? ls->vorticity_split : ps.vorticity_split, walk_grid, h->blk, 0, st, p, h->pos[cc].p, h->vel.p, ms,
                    h->nbr_count.p, h->nbr_list.p, h->omega.p, h->normal.p, h->visc.p, h->coh.p);
     }
     CU(h, cudaGetLastError());
     {
       KScope ks(h, K_XSPH);
-      launch_chain(early, ps.xsph_split, grid_of(h, n), h->blk, 0, st, p, h->pos[cc].p, h->omega.p, h->normal.p,
+      launch_chain(early, ls ? ls->xsph_split : ps.xsph_split, walk_grid, h->blk, 0, st, p, h->pos[cc].p, h->omega.p, h->normal.p,
                    h->visc.p, h->coh.p, ms, h->nbr_count.p, h->nbr_list.p, h->acc.p, ex);
     }
     CU(h, cudaGetLastError());

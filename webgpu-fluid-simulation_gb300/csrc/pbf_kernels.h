@@ -38,7 +38,7 @@ constexpr uint32_t kEarlyMax = 1u << 18;
 
 // The neighbour passes with several lanes a slot, for small scenes.
 struct LaneSet {
-  uint32_t lanes = 0;
+  uint32_t lanes = 0, max_n = 0;  // up to max_n slots
   void (*lambda)(SimParams, int, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*, float4*,
                  SolverAux) = nullptr;
   void (*deltap)(SimParams, SolverAux, int, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*,
@@ -49,6 +49,10 @@ struct LaneSet {
                     float4*) = nullptr;
   void (*xsph)(SimParams, const float4*, const float4*, const float4*, const float4*, uint32_t, const uint32_t*,
                const uint32_t*, float4*, ExportArgs) = nullptr;
+  void (*vorticity_split)(SimParams, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*,
+                          float4*, float4*, float4*, float4*) = nullptr;
+  void (*xsph_split)(SimParams, const float4*, const float4*, const float4*, const float4*, const float4*, uint32_t,
+                     const uint32_t*, const uint32_t*, float4*, ExportArgs) = nullptr;
 };
 
 // The step's passes of one variant: single scene or batch (scene table),
@@ -81,7 +85,7 @@ struct PassSet {
                     float4*);
   void (*xsph)(SimParams, const float4*, const float4*, const float4*, const float4*, uint32_t, const uint32_t*,
                const uint32_t*, float4*, ExportArgs);
-  LaneSet lanes[2];  // more lanes first; lanes = 0 where not built
+  LaneSet lanes[2];  // more lanes first; max_n = 0 where not built
   // fast mode: XSPH's neighbour sum split over the vorticity and XSPH passes (null in exact mode)
   void (*vorticity_split)(SimParams, const float4*, const float4*, uint32_t, const uint32_t*, const uint32_t*,
                           float4*, float4*, float4*, float4*);

@@ -573,7 +573,8 @@ __device__ __forceinline__ void for_each_neighbor2(const uint32_t* __restrict__ 
 // its records, term(records): its terms), and all add the terms up in list
 // order, handed round by shuffles.  A lane that finds no entry left evaluates
 // slot 0 and its terms are not taken.  The same additions of the same terms:
-// without FMA contraction (exact mode) the same bits as one lane's walk.
+// the same bits as one lane's walk, also with FMA contraction as long as a
+// Term keeps apart the factors that one lane's walk multiplies as it adds.
 template <class T>
 __device__ __forceinline__ T shfl_term(unsigned mates, const T& t, uint32_t from) {
   constexpr int kN = sizeof(T) / sizeof(float);
@@ -793,13 +794,14 @@ struct DpSum {
     pu = mk(0.f, 0.f, 0.f);
   }
   struct Term {
-    f3 pu;
+    f3 gk;
+    float l;
   };
   __device__ __forceinline__ Term term(const SimParams& p, float4 xj) const {
     Pair q = make_pair_of(xi - xyz(xj));
-    return {(li + xj.w) * spiky_p(p, q)};
+    return {spiky_p(p, q), li + xj.w};
   }
-  __device__ __forceinline__ void take(const Term& t) { pu = pu + t.pu; }
+  __device__ __forceinline__ void take(const Term& t) { pu = pu + t.l * t.gk; }
   __device__ __forceinline__ void add(const SimParams& p, float4 xj) { take(term(p, xj)); }
 };
 // AttributeUpdate's density sum (attributeUpdate.ts:40-49).
@@ -893,18 +895,26 @@ struct VortSplitSum {
     vu = mk(0.f, 0.f, 0.f);
     cs = mk(0.f, 0.f, 0.f);
   }
-  __device__ __forceinline__ void add(const SimParams& p, float4 pj, float4 vj) {
+  struct Term {
+    f3 cr, gw, vd, co;
+    float volume, wr, kij;
+  };
+  __device__ __forceinline__ Term term(const SimParams& p, float4 pj, float4 vj) const {
     Pair q = make_pair_of(xi - xyz(pj));
     f3 vd = xyz(vj) - vi;
     const float inv_rj = frcp_fast(pj.w);
     const float volume = p.m * inv_rj;
     f3 gw = spiky_p(p, q);
-    om = om + volume * cross3(vd, gw);
-    nm = nm + volume * gw;
-    vu = vu + (poly6_p(p, q) * inv_rj) * vd;
     const float kij = p.two_rho0 * frcp_fast(ri + pj.w);
-    cs = cs + kij * (p.m * cohesion_p(p, q));
+    return {cross3(vd, gw), gw, vd, p.m * cohesion_p(p, q), volume, poly6_p(p, q) * inv_rj, kij};
   }
+  __device__ __forceinline__ void take(const Term& t) {
+    om = om + t.volume * t.cr;
+    nm = nm + t.volume * t.gw;
+    vu = vu + t.wr * t.vd;
+    cs = cs + t.kij * t.co;
+  }
+  __device__ __forceinline__ void add(const SimParams& p, float4 pj, float4 vj) { take(term(p, pj, vj)); }
 };
 // ... and the XSPH pass the vorticity-force eta and the curvature part.
 struct XsphSplitSum {
@@ -917,12 +927,19 @@ struct XsphSplitSum {
     eta = mk(0.f, 0.f, 0.f);
     cv = mk(0.f, 0.f, 0.f);
   }
-  __device__ __forceinline__ void add(const SimParams& p, float4 pj, float4 nj) {  // nj: (normal_j, |omega_j|)
+  struct Term {
+    f3 gw, cu;
+    float wr, kij;
+  };
+  __device__ __forceinline__ Term term(const SimParams& p, float4 pj, float4 nj) const {  // nj: (normal_j, |omega_j|)
     Pair q = make_pair_of_lib(xi - xyz(pj));
-    eta = eta + (nj.w * frcp_fast(pj.w)) * spiky_p(p, q);
-    const float kij = p.two_rho0 * frcp_fast(ri + pj.w);
-    cv = cv + kij * (ni - xyz(nj));
+    return {spiky_p(p, q), ni - xyz(nj), nj.w * frcp_fast(pj.w), p.two_rho0 * frcp_fast(ri + pj.w)};
   }
+  __device__ __forceinline__ void take(const Term& t) {
+    eta = eta + t.wr * t.gw;
+    cv = cv + t.kij * t.cu;
+  }
+  __device__ __forceinline__ void add(const SimParams& p, float4 pj, float4 nj) { take(term(p, pj, nj)); }
 };
 
 // LambdaCalculation (pressureConstrain.ts:31-85).  Writes xl[t] = (x*, lambda):
@@ -1301,9 +1318,9 @@ __global__ void __launch_bounds__(256) k_xsph_split(SimParams p, const float4* _
 }
 
 // The passes of a scene too small to fill the device, kL lanes a slot
-// (walk_lanes).  Exact mode: a neighbour's terms are long chains (IEEE square
-// roots and divisions), and with one lane a slot a pass took as long at 2,000
-// slots as at 69,000 (XSPH 65 us).
+// (walk_lanes).  With one lane a slot such a pass is the chain of one slot's
+// neighbours and takes as long at 2,000 slots as at 69,000: in exact mode, with
+// its IEEE square roots and divisions, 65 us for XSPH.
 struct Rec2 {
   float4 a, b;
 };
@@ -1414,6 +1431,70 @@ __global__ void __launch_bounds__(256) k_xsph_lanes(SimParams p, const float4* _
   xsph_finish(p, acc, t, s, xyz(omega[t]));
 }
 
+template <uint32_t kL>
+__global__ void __launch_bounds__(256) k_vorticity_split_lanes(SimParams p, const float4* __restrict__ pos,
+                                                               const float4* __restrict__ vel, uint32_t max_nbr,
+                                                               const uint32_t* __restrict__ nbr_cnt,
+                                                               const uint32_t* __restrict__ nbr_list,
+                                                               float4* __restrict__ omega, float4* __restrict__ normal,
+                                                               float4* __restrict__ visc,
+                                                               float4* __restrict__ coh_sum) {
+  chain_begin(pos, vel, nbr_cnt, nbr_list);
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, t = g / kL;
+  if (t >= p.n) return;
+  uint32_t b, e;
+  list_slice(max_nbr, nbr_cnt, t, b, e);
+  VortSplitSum s;
+  s.init(pos[t], xyz(vel[t]));
+  walk_lanes<kL>(
+      nbr_list, b, e, [&](uint32_t j) { return Rec2{__ldg(pos + j), __ldg(vel + j)}; },
+      [&](const Rec2& r) { return s.term(p, r.a, r.b); }, [&](const VortSplitSum::Term& x) { s.take(x); });
+  if (g % kL == 0) vorticity_split_finish(p, omega, normal, visc, coh_sum, t, s);
+}
+
+template <uint32_t kL>
+__global__ void __launch_bounds__(256) k_xsph_split_lanes(SimParams p, const float4* __restrict__ pos,
+                                                          const float4* __restrict__ omega,
+                                                          const float4* __restrict__ normal,
+                                                          const float4* __restrict__ visc,
+                                                          const float4* __restrict__ coh_sum, uint32_t max_nbr,
+                                                          const uint32_t* __restrict__ nbr_cnt,
+                                                          const uint32_t* __restrict__ nbr_list,
+                                                          float4* __restrict__ acc, ExportArgs ex) {
+  chain_begin(pos, omega, normal, visc, coh_sum, nbr_cnt, nbr_list, ex.id);
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, t = g / kL;
+  if (t >= p.n) return;
+  uint32_t b, e;
+  list_slice(max_nbr, nbr_cnt, t, b, e);
+  XsphSplitSum s;
+  const float4 pi = pos[t];
+  s.init(pi, xyz(normal[t]));
+  walk_lanes<kL>(
+      nbr_list, b, e, [&](uint32_t j) { return Rec2{__ldg(pos + j), __ldg(normal + j)}; },
+      [&](const Rec2& r) { return s.term(p, r.a, r.b); }, [&](const XsphSplitSum::Term& x) { s.take(x); });
+  if (g % kL != 0) return;
+  if (ex.id) ex.out[ex.id[t]] = pi;
+  xsph_split_finish(p, acc, t, s, xyz(omega[t]), visc[t], coh_sum[t]);
+}
+
+template <uint32_t kL>
+LaneSet lane_passes(uint32_t max_n) {
+  LaneSet s;
+  s.lanes = kL;
+  s.max_n = max_n;
+  s.lambda = k_lambda_lanes<kL>;
+  s.deltap = k_deltap_lanes<kL>;
+  s.density_velocity = k_density_velocity_lanes<kL>;
+  if constexpr (kFast) {
+    s.vorticity_split = k_vorticity_split_lanes<kL>;
+    s.xsph_split = k_xsph_split_lanes<kL>;
+  } else {
+    s.vorticity = k_vorticity_lanes<kL>;
+    s.xsph = k_xsph_lanes<kL>;
+  }
+  return s;
+}
+
 #include "pbf_cellblock.cuh"
 
 // Launch table for this precision variant: [batch][persistent] pass sets.
@@ -1433,19 +1514,9 @@ void fill_set(PassSet* ps) {
   ps->density_velocity = k_density_velocity<P>;
   ps->vorticity = k_vorticity<P>;
   ps->xsph = k_xsph<P>;
-  if constexpr (!kFast && !B && !P) {
-    ps->lanes[0] = LaneSet{8,
-                           k_lambda_lanes<8>,
-                           k_deltap_lanes<8>,
-                           k_density_velocity_lanes<8>,
-                           k_vorticity_lanes<8>,
-                           k_xsph_lanes<8>};
-    ps->lanes[1] = LaneSet{4,
-                           k_lambda_lanes<4>,
-                           k_deltap_lanes<4>,
-                           k_density_velocity_lanes<4>,
-                           k_vorticity_lanes<4>,
-                           k_xsph_lanes<4>};
+  if constexpr (!B && !P) {
+    ps->lanes[0] = lane_passes<8>(kFast ? 1u << 12 : 1u << 14);
+    ps->lanes[1] = lane_passes<4>(kFast ? 1u << 13 : 1u << 15);
   }
   if constexpr (kFast) {
     ps->vorticity_split = k_vorticity_split<P>;
