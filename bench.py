@@ -831,7 +831,7 @@ def batch_arm(args, dist):
         "tuner_trials": trials,
         "e2e": {"value": total * sub * args.steps / e2e_s, "unit": UNIT,
                 "h2d_bytes_per_step": ctypes.sizeof(L.Options), "d2h_bytes_per_step": int(host.nbytes)},
-        "gpu_launches": (sub * (11 + 3 * iters_max) + 1) * args.steps,
+        "gpu_launches": sub * (10 + 3 * iters_max) * args.steps,
         "roofline": roof, "clocks": clk,
         "scene_metrics": {"scenes": len(merged), "nonfinite": sum(m["nonfinite"] for m in merged.values()),
                           "penetrations": sum(m["penetrations"] for m in merged.values()),
@@ -957,12 +957,13 @@ def render_arm(args, dist):
             "raster_ms": statistics.mean(raster), "filter_ms": statistics.mean(filt),
             "e2e": {"value": e2e_ms, "unit": "ms", "h2d_bytes_per_step": int(p.nbytes),
                     "d2h_bytes_per_step": int(W * H * 4)},
-            "gpu_launches": 5 * args.steps,
+            # init, two splats with the tiles' depths between, volume scan, order and sums, resolve, filter x and y
+            "gpu_launches": 10 * args.steps,
             "roofline": {"bound": "hbm", "kernel": "k_splat", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "peak_kind": peak_kind, "traffic": 18.2e6,
+                         "frac": achieved / peak, "peak_kind": peak_kind, "traffic": None,
                          "alg_bytes_per_launch": alg, "avg_launch_ms": statistics.mean(raster),
-                         "note": "instruction-issue bound (ncu: 70 % issue active, L2 17 %); the HBM fraction "
-                                 "only shows how little of the frame is memory traffic"},
+                         "note": "instruction-issue bound (ncu, issue active: k_splat 62 %, k_volume_sum 79 %); the "
+                                 "HBM fraction only shows how little of the frame is memory traffic"},
             "clocks": clk, "cpu_baseline": cpu}
     if dist.rank == 0:
         print(json.dumps(line), flush=True)
@@ -1199,14 +1200,14 @@ def ns_arm(args, dist):
                        "l2": "inputs of 256 MB each, larger than the 129 MB L2", "phase_ms": per_input},
             "e2e": {"value": e2e, "unit": "particles/s", "h2d_bytes_per_step": int(2 * 16 * n),
                     "d2h_bytes_per_step": int(2 * (12 * n + 4 * cells + 4 * (cells + 1)))},
-            # per search: keys, 3 x (digit counts, matrix scan, record move), offsets scan, ranks
-            "gpu_launches": 2 * 12 * args.steps,
+            # per search: keys + digits, 3 x (matrix scan, record move), 2 digit counts, offsets scan, ranks
+            "gpu_launches": 2 * 11 * args.steps,
             "roofline": {"bound": "hbm", "kernel": top, "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind, "traffic": None,
                          "alg_bytes_per_launch": alg, "avg_launch_ms": mean_phase[top],
                          "phases_ms": mean_phase,
-                         "note": "a phase of pbf_ns_run timed by its own CUDA events; sort_passes is 3 x (digit "
-                                 "count, scan of the digit x tile matrix, record move), 9 launches"},
+                         "note": "a phase of pbf_ns_run timed by its own CUDA events; sort_passes is 3 x (scan of the "
+                                 "digit x tile matrix, record move) and 2 digit counts, 8 launches"},
             "clocks": clk, "cpu_baseline": cpu}
     if dist.rank == 0:
         print(json.dumps(line), flush=True)

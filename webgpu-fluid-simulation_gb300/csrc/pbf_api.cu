@@ -364,7 +364,7 @@ void prefer_l1(const PassSet& ps) {
 }
 
 // The passes with several lanes a slot, for the plain solve of a small scene;
-// null where one lane a slot is as fast.  Four iterations, two substeps, graph
+// null where one lane a slot is as fast.  A substep of four iterations, graph
 // replay, one / four / eight lanes in us (three handles at once, each):
 //   exact  2,197 slots  250 / 148 / 117 (87 / 52 / 42)
 //          8,000        305 / 177 / 144 (105 / 66 / 59)
