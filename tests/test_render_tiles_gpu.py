@@ -18,7 +18,9 @@ torch = pytest.importorskip("torch")
                                             (50000, 1023, 577, 0.01, 2.5), (524287, 1280, 820, 0.01, 0.5),
                                             (524288, 1280, 820, 0.01, 0.5), (524288, 1023, 1031, 0.01, 2.5),
                                             (600001, 1031, 1023, 0.02, 0.03), (3000, 1031, 1023, 0.02, 0.3),
-                                            (10001, 320, 200, 0.05, 0.3)])
+                                            (10001, 320, 200, 0.05, 0.3), (393215, 1600, 880, 0.01, 2.5),
+                                            (393216, 1600, 880, 0.01, 2.5), (655359, 320, 200, 0.01, 0.5),
+                                            (655360, 320, 200, 0.01, 0.5)])
 def test_two_phase_splat(n, W, H, R, spread):
     rng = np.random.default_rng(n + W)
     p = np.zeros((n, 4), np.float32)

@@ -256,12 +256,22 @@ constexpr int kTile = 8;
 constexpr uint32_t kFirstShare = 16;
 // The two phases and the volume sums by tile pay for their five extra launches
 // (about 25 us) and for the particles' second reading where there are many
-// particles and their sprites many pixels.  A frame at 2^20 particles (all at
-// once, tiled): 320 x 180 277 and 277 us, 960 x 540 351 and 327, 1280 x 720 437
-// and 367, 1920 x 1080 789 and 556; at 2^19 and 1920 x 1080 447 and 435, at 2^18
-// 289 and 312.
-constexpr uint32_t kTiledMin = 1u << 19;
+// particles, or fewer with sprites of many pixels.  A frame, all at once (with 8
+// or 16 particles a warp) and tiled:
+//              320 x 180   960 x 540   1280 x 720   1600 x 900   1920 x 1080
+//   1,048,576  290  250    356  289    445  332     579  409     789  524
+//     700,000  207  187    260  225    321  260     466  324     567  420
+//     524,288  166  178    215  224    266  268     344  327     466  431
+//     393,216  147  139    174  172    211  204     286  259     355  335
+//     262,144  112  126    149  194    186  249     242  320     321  429
+// (Powers of two are the worst for the first share here: the particles lie in
+// index order on a lattice, and every 16th block falls on the same lines.)
+constexpr uint32_t kTiledAlways = 5u << 17;
+constexpr uint32_t kTiledMin = 3u << 17;
 constexpr uint64_t kTiledWork = 1ull << 39;  // particles times pixels
+inline bool takes_tiles(uint32_t n, int W, int H) {
+  return n >= kTiledAlways || (n >= kTiledMin && (uint64_t)W * H * n >= kTiledWork);
+}
 constexpr int kMaxTiles = 16;                // larger sprites are not tested
 
 __global__ void __launch_bounds__(256) k_tile_min(const unsigned long long* __restrict__ keys, int W, int H, int tw,
@@ -280,6 +290,8 @@ __global__ void __launch_bounds__(256) k_tile_min(const unsigned long long* __re
   m = __reduce_min_sync(0xffffffffu, m);
   if (lane == 0) tile_min[tile] = m;
 }
+
+constexpr uint64_t kSmallMap = 3u << 17;  // pixels (768 x 512)
 
 // Whether a depth sprite may win a pixel in any of its tiles.
 __device__ inline bool may_win(const Sprite& s, const uint32_t* __restrict__ tile_min, int tw) {
@@ -482,6 +494,8 @@ __global__ void __launch_bounds__(kVolThreads) k_volume_sum(Cam C, const float4*
   }
 }
 
+// kSteps: the keys of four steps of a depth sprite are read together.
+template <bool kSteps>
 __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__ pos, uint32_t n, float R, int W, int H,
                                                int W2, int H2, unsigned long long* keys, unsigned long long* acc,
                                                int phase, uint32_t per, const uint32_t* __restrict__ tile_min, int tw,
@@ -562,7 +576,7 @@ __global__ void __launch_bounds__(256) k_splat(Cam C, const float4* __restrict__
         };
         const int w = s.i1 - s.i0;
         const int rows1 = w <= 32 ? (int)((32u * c_recip16[w]) >> 16) : 0;
-        if (w > 32 || s.j1 - s.j0 <= rows1) {  // one step, or rows of many
+        if (!kSteps || w > 32 || s.j1 - s.j0 <= rows1) {  // one step, or rows of many
           walk_sprite(s, lane, [&](int i, int j, bool in) {
             consider(i, j, in && bound > *(volatile unsigned long long*)(keys + (size_t)j * W + i));
           });
@@ -889,7 +903,7 @@ int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_s
   const float4* pos = (const float4*)d_positions;
   cudaEventRecord(r->ev[0], st);
   const dim3 rows((unsigned)((r->W + 255) / 256), (unsigned)r->H);
-  bool tiled = n >= kTiledMin && (uint64_t)r->W * r->H * n >= kTiledWork;
+  bool tiled = takes_tiles(n, r->W, r->H);
   if (tiled && volume_workspace(r, n, st) != cudaSuccess) {
     cudaGetLastError();  // without the workspace, everything is drawn at once
     tiled = false;
@@ -905,13 +919,19 @@ int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_s
     auto splat = [&](int phase, uint64_t particles) {
       // Few particles are spread over the device, as a warp walks its own one
       // after another (8000 at 1920 x 1080, a frame: 32 a warp 219 us, 2 a warp
-      // 73); many are taken in blocks that set their sprites up with most lanes
-      // (2^20 at 320 x 180: 2 a warp 541 us, 16 a warp 291).  Between, finer is
-      // also more even: 2^18 at 1920 x 1080 433 us with 32, 321 with 8.
-      uint32_t per = phase == kRest ? 32 : phase == kFirst ? 4 : n >= kTiledMin ? 16 : 8;
+      // 73); many are taken in blocks that set their sprites up with most lanes,
+      // more of them where the sprites are small (320 x 180: 300,000 with 8 a warp
+      // 120 us, with 32 112; 450,000 161 and 146).  On large maps finer is also
+      // more even: 2^18 at 1920 x 1080 433 us with 32, 321 with 8.
+      const uint64_t pixels = (uint64_t)r->W * r->H;
+      const uint32_t sixteen = pixels < kSmallMap ? 150000u : 400000u;  // particles from which a warp takes 16
+      uint32_t per = pixels < kSmallMap && n >= 300000u ? 32 : n >= sixteen ? 16 : 8;
+      if (phase != kAll) per = phase == kRest ? 32 : 4;
       while (phase == kAll && per > 1 && particles < (uint64_t)sms * 32 * per) per /= 2;
       const uint64_t warps = (particles + per - 1) / per;
-      return pbf::launch_chain(true, k_splat, (unsigned)((warps + 7) / 8), 256, 0, st, C, pos, n, R, r->W,
+      // on maps below 2^19 pixels most sprites are a step or two: reading ahead cost 2 to 4 % there
+      auto kernel = phase == kAll && pixels < (1u << 19) ? k_splat<false> : k_splat<true>;
+      return pbf::launch_chain(true, kernel, (unsigned)((warps + 7) / 8), 256, 0, st, C, pos, n, R, r->W,
                                r->H, r->W2, r->H2, r->keys, r->acc, phase, per, r->tile_min, tw, r->vol_tile,
                                r->vol_count);
     };
