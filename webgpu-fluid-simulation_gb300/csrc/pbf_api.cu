@@ -75,6 +75,12 @@ struct pbf_handle {
   int count_buf = 0;         // the buffer that the next substep counts into
   bool count_clear = false;  // ... and whether it is known to be all zero
   int xs_final = 0;          // the xs buffer holding the last substep's x*
+  // A caller has recorded substeps into a graph of its own.  When that graph
+  // runs, and on which buffers, this side cannot know, so from then on every
+  // substep clears the counts it uses, counts into one fixed buffer (that of
+  // the last substep before) and leaves its x* in one fixed buffer.
+  bool caller_graph = false;
+  bool own_capture = false;  // the capture under way on the stream is capture_frame's
   DBuf<uint32_t> nbr_count, nbr_max, nbr_list;
   DBuf<uint32_t> band_list[2], band_count;  // boundary band lists (ping-pong) and their lengths
   // cell-block passes (PBF_BUILD_CELLBLOCK_*): cell key and x*_0 per sorted
@@ -101,6 +107,7 @@ struct pbf_handle {
   struct FrameGraph {
     cudaGraphExec_t exec = nullptr;
     int cur = 0, count_buf = 0;
+    bool caller_graph = false;
   };
   FrameGraph graphs[2];
   bool graph_enabled = false;
@@ -386,6 +393,26 @@ void invalidate_graph(pbf_handle* h) {
   }
 }
 
+// Whether a caller is recording the handle's stream into a graph of its own.
+bool caller_captures(const pbf_handle* h) {
+  if (h->own_capture) return false;
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->stream, &s) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream beside another one's capture: the launches report it
+    return false;
+  }
+  return s != cudaStreamCaptureStatusNone;
+}
+
+// The captured frame that fits the current buffers, or null.
+pbf_handle::FrameGraph* frame_graph(pbf_handle* h) {
+  for (auto& q : h->graphs)
+    if (q.exec && q.cur == h->cur && q.count_buf == h->count_buf && q.caller_graph == h->caller_graph &&
+        (h->count_clear || h->caller_graph))
+      return &q;
+  return nullptr;
+}
+
 // Reads and clears the device error word.  A neighbour-list overflow (a
 // particle with more neighbours than the per-particle slice) grows the slice
 // to 1.25x the largest count seen; the results of that substep are invalid
@@ -444,8 +471,11 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   const bool early = n <= kEarlyMax;
   if (ev) CU(h, cudaEventRecord(ev[0], st));
   // neighborSearch.clearBuffer + TimeIntegration (+ ParticleInsert counts)
-  uint32_t* const counts = h->cell_count[h->count_buf].p;
-  if (!h->count_clear) CU(h, cudaMemsetAsync(counts, 0, ((size_t)g.cells + 1) * sizeof(uint32_t), st));
+  if (caller_captures(h)) h->caller_graph = true;
+  const int count_at = h->caller_graph ? 1 - h->count_buf : h->count_buf;
+  uint32_t* const counts = h->cell_count[count_at].p;
+  if (h->caller_graph || !h->count_clear)
+    CU(h, cudaMemsetAsync(counts, 0, ((size_t)g.cells + 1) * sizeof(uint32_t), st));
   h->count_clear = false;
   {
     KScope ks(h, K_PREDICT);
@@ -458,8 +488,9 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
   CU(h, cudaGetLastError());
   if (ev) CU(h, cudaEventRecord(ev[1], st));
   // cell scan + counting sort (stable by id) + reorder of the state
-  SortBuffers sb{h->key.p,    h->rank.p,  counts,    h->cell_count[1 - h->count_buf].p, h->cell_start.p, h->perm_raw.p,
-                 h->id_raw.p, h->perm.p,  h->tmp_a.p, h->tmp_b.p,                       h->big_list.p,   h->big_count.p,
+  uint32_t* const count_next = h->caller_graph ? nullptr : h->cell_count[1 - count_at].p;
+  SortBuffers sb{h->key.p,    h->rank.p, counts,     count_next,  h->cell_start.p, h->perm_raw.p,
+                 h->id_raw.p, h->perm.p, h->tmp_a.p, h->tmp_b.p,  h->big_list.p,   h->big_count.p,
                  h->scan_scratch, h->err_word.p};
   // the learned start's and trace capture's features: the previous multiplier
   // sum moves with the state
@@ -473,8 +504,10 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
       G.xs0_out = h->xs0.p;
     }
     CU(h, launch_sort_by_cell(g, n, h->ids[c].p, sb, h->id_bits, G, st));
-    h->count_buf = 1 - h->count_buf;
-    h->count_clear = true;
+    if (!h->caller_graph) {
+      h->count_buf = 1 - h->count_buf;
+      h->count_clear = true;
+    }
   }
   h->cur = nx;
   const int cc = nx;
@@ -784,7 +817,10 @@ int substep(pbf_handle* h, cudaEvent_t* ev, bool* exported = nullptr) {
                                         dim3(256), args, 0, st));
     }
   }
-  h->xs_final = a;
+  if (!h->caller_graph)
+    h->xs_final = a;
+  else if (a != h->xs_final)
+    CU(h, cudaMemcpyAsync(h->xs[h->xs_final].p, h->xs[a].p, (size_t)n * sizeof(float4), cudaMemcpyDeviceToDevice, st));
   // per-kernel timing keeps the export a launch of its own
   const bool ex_here = exported && !cb && !h->ktiming;
   const ExportArgs ex = ex_here ? ExportArgs{h->ids[cc].p, h->out_pos.p} : ExportArgs{nullptr, nullptr};
@@ -861,18 +897,21 @@ int frame(pbf_handle* h, uint32_t substeps) {
 
 // Records a frame that starts from the current buffers; nothing runs.
 int capture_frame(pbf_handle* h, pbf_handle::FrameGraph* g) {
-  if (!h->count_clear) {  // the frame relies on its counts being clear
+  if (caller_captures(h)) return fail(h, PBF_ECUDA, "graph capture: the stream is being captured by its owner");
+  if (!h->caller_graph && !h->count_clear) {  // the frame relies on its counts being clear
     CU(h, cudaMemsetAsync(h->cell_count[h->count_buf].p, 0, ((size_t)h->gp.cells + 1) * sizeof(uint32_t), h->stream));
     h->count_clear = true;
   }
   const int cur = h->cur, buf = h->count_buf;
   cudaGraph_t graph = nullptr;
   CU(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+  h->own_capture = true;
   const int rc = frame(h, h->cfg.substeps);
+  h->own_capture = false;
   cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
   h->cur = cur;
   h->count_buf = buf;
-  h->count_clear = true;
+  h->count_clear = !h->caller_graph;
   if (rc == PBF_OK && e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, graph, 0);
   if (graph) cudaGraphDestroy(graph);
   if (rc) return rc;
@@ -882,6 +921,7 @@ int capture_frame(pbf_handle* h, pbf_handle::FrameGraph* g) {
   }
   g->cur = cur;
   g->count_buf = buf;
+  g->caller_graph = h->caller_graph;
   return PBF_OK;
 }
 
@@ -1714,7 +1754,11 @@ int pbf_step(pbf_handle* h, uint32_t frames) {
   // Trace capture samples a different particle subset every substep (its salt
   // and the substep counter are host values a graph would freeze), so it
   // runs eagerly, as per-kernel timing does.
-  if (!h->graph_enabled || h->ktiming || h->trace_cap > 0) {
+  // A frame that a caller records into a graph of its own is recorded kernel
+  // by kernel: a captured frame of the handle would rely on counts that only
+  // the handle's own order of steps keeps clear.
+  const bool recorded = (h->graphs[0].exec || h->graphs[1].exec) && caller_captures(h);
+  if (!h->graph_enabled || h->ktiming || h->trace_cap > 0 || recorded) {
     for (uint32_t f = 0; f < frames; ++f) {
       int rc = frame(h, h->cfg.substeps);
       if (rc) return rc;
@@ -1724,9 +1768,7 @@ int pbf_step(pbf_handle* h, uint32_t frames) {
   // Each substep swaps the state and count buffers, so a frame's graph fits
   // the buffers it was captured from.
   for (uint32_t f = 0; f < frames; ++f) {
-    pbf_handle::FrameGraph* g = nullptr;
-    for (auto& q : h->graphs)
-      if (q.exec && q.cur == h->cur && q.count_buf == h->count_buf && h->count_clear) g = &q;
+    pbf_handle::FrameGraph* g = frame_graph(h);
     if (!g) {
       // single substeps since the last capture may have left other buffers
       // current than either graph starts from
@@ -1738,7 +1780,7 @@ int pbf_step(pbf_handle* h, uint32_t frames) {
     CU(h, cudaGraphLaunch(g->exec, h->stream));
     if (h->cfg.substeps % 2 != 0) {
       h->cur = 1 - h->cur;
-      h->count_buf = 1 - h->count_buf;
+      if (!h->caller_graph) h->count_buf = 1 - h->count_buf;
     }
   }
   return PBF_OK;
