@@ -347,8 +347,10 @@ int pbf_ns_run(pbf_ns* ns, const float* d_pos4, uint32_t n, uint32_t* d_keys,
 /* Neighbour lists in the reference layout (NeighborCount + particle scan +
  * NeighborList, neighborShader.ts:101-246): d_nbr_offset has n+1 entries and
  * d_nbr_list holds particle ids.  Call after pbf_ns_run with the same positions.
- * Fails with PBF_ECAPACITY (writing nothing past capacity) if the lists need
- * more than `capacity` entries; *total receives the needed size. */
+ * Fails with PBF_ECAPACITY (writing no list) if the lists need more than
+ * `capacity` entries; *total receives the needed size, 0xffffffff if it is
+ * larger.  PBF_ETIMEOUT: a scan of this call or of the searches before it gave
+ * up its bounded wait, the lists are not valid. */
 int pbf_ns_lists(pbf_ns* ns, const float* d_pos4, uint32_t n, float radius,
                  uint32_t* d_nbr_offset, uint32_t* d_nbr_list, uint32_t capacity,
                  uint32_t* total);

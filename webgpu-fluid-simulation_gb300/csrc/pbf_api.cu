@@ -2475,13 +2475,21 @@ int pbf_get_scene_metrics(pbf_handle* h, uint32_t scene, pbf_metrics* out) {
 // ---- neighbour search alone -------------------------------------------------------
 }  // extern "C"
 
+// What a search hands back besides its arrays: the error word and the
+// neighbours of the last pbf_ns_lists, all together.
+struct NsStatus {
+  uint32_t err, pad;
+  unsigned long long total;
+};
+
 struct pbf_ns {
   GridParams g;
   uint32_t max_n;
   cudaStream_t stream;
   bool own_stream;
   std::string err;
-  DBuf<uint32_t> key, rank, cell_count, cell_start, perm_raw, id_raw, perm, tmp_a, tmp_b, big_list, big_count, err_word;
+  DBuf<uint32_t> key, rank, cell_count, cell_start, perm_raw, id_raw, perm, tmp_a, tmp_b, big_list, big_count;
+  DBuf<uint32_t> err_word;   // NsStatus
   DBuf<uint32_t> nbr_count;  // by particle id (pbf_ns_lists)
   DBuf<float4> sorted;       // pbf_ns_lists: positions in sorted order, the id in w
   void* scan_scratch = nullptr;
@@ -2549,7 +2557,7 @@ int pbf_ns_create(const pbf_grid* grid, uint32_t max_particles, void* stream, pb
   A(s->cell_start.alloc(cells + 1));
   A(s->big_list.alloc(cells));
   A(s->big_count.alloc(1));
-  A(s->err_word.alloc(1));
+  A(s->err_word.alloc(sizeof(NsStatus) / sizeof(uint32_t)));
   A(s->nbr_count.alloc(n + 1));
   size_t sb = scan_scratch_bytes(cells + 1), sb2 = scan_scratch_bytes(n + 1);
   A(cudaMalloc(&s->scan_scratch, sb > sb2 ? sb : sb2));
@@ -2650,16 +2658,22 @@ int pbf_ns_lists(pbf_ns* s, const float* d_pos4, uint32_t n, float radius, uint3
   // the sorted positions' workspace: allocated by the first call, kept with the context
   if (!s->sorted.p) NSCU(s, s->sorted.alloc(s->max_n));
   const float h2 = (float)((double)radius * (double)radius);
+  unsigned long long* total_word = &((NsStatus*)s->err_word.p)->total;
   NSCU(s, launch_ns_count(n, s->g, h2, s->perm.p, (const float4*)d_pos4, s->cell_start.p, s->sorted.p, s->nbr_count.p,
-                          d_nbr_offset, s->scan_scratch, s->err_word.p, st));
-  uint32_t tot = 0;
-  NSCU(s, cudaMemcpyAsync(&tot, d_nbr_offset + n, 4, cudaMemcpyDeviceToHost, st));
+                          d_nbr_offset, total_word, s->scan_scratch, s->err_word.p, st));
   // the kernel itself compares the total with the capacity, so it is queued before the host knows
   if (d_nbr_list)
-    NSCU(s, launch_ns_list(n, s->g, h2, s->sorted.p, s->cell_start.p, d_nbr_offset, d_nbr_list, capacity, st));
+    NSCU(s, launch_ns_list(n, s->g, h2, s->sorted.p, s->cell_start.p, s->nbr_count.p, d_nbr_offset, total_word,
+                           d_nbr_list, capacity, st));
+  NsStatus got{};
+  NSCU(s, cudaMemcpyAsync(&got, s->err_word.p, sizeof(got), cudaMemcpyDeviceToHost, st));
   NSCU(s, cudaStreamSynchronize(st));
-  if (total) *total = tot;
-  if (tot > capacity) return nsfail(s, PBF_ECAPACITY, "neighbour lists exceed capacity");
+  if (total) *total = (uint32_t)std::min<unsigned long long>(got.total, 0xffffffffull);
+  if (got.err & PBF_DEVERR_SCAN_TIMEOUT) {
+    NSCU(s, cudaMemsetAsync(s->err_word.p, 0, sizeof(uint32_t), st));
+    return nsfail(s, PBF_ETIMEOUT, "scan look-back wait gave up");
+  }
+  if (got.total > capacity) return nsfail(s, PBF_ECAPACITY, "neighbour lists exceed capacity");
   return PBF_OK;
 }
 

@@ -209,14 +209,15 @@ cudaError_t launch_scatter_by_id_u32(uint32_t n, const uint32_t* id, const uint3
                                      cudaStream_t st);
 // Neighbour lists of the stand-alone search (27 cells, |d|^2 <= h2): sorted[t]
 // = (position, id) of order[t], the neighbour count by particle id (n + 1
-// entries, the last 0) and its exclusive scan offset; then the lists of
-// neighbour ids at offset[id], written only if offset[n] <= capacity.  scan:
-// scan_scratch_bytes(n + 1) bytes.
+// entries, the last 0), its exclusive scan offset and the 64-bit sum *total;
+// then the lists of neighbour ids at offset[id], written only if *total <=
+// capacity.  scan: scan_scratch_bytes(n + 1) bytes.
 cudaError_t launch_ns_count(uint32_t n, const GridParams& g, float h2, const uint32_t* order, const float4* pos,
-                            const uint32_t* cell_start, float4* sorted, uint32_t* count, uint32_t* offset, void* scan,
-                            uint32_t* err, cudaStream_t st);
+                            const uint32_t* cell_start, float4* sorted, uint32_t* count, uint32_t* offset,
+                            unsigned long long* total, void* scan, uint32_t* err, cudaStream_t st);
 cudaError_t launch_ns_list(uint32_t n, const GridParams& g, float h2, const float4* sorted, const uint32_t* cell_start,
-                           const uint32_t* offset, uint32_t* list, uint32_t capacity, cudaStream_t st);
+                           const uint32_t* count, const uint32_t* offset, const unsigned long long* total,
+                           uint32_t* list, uint32_t capacity, cudaStream_t st);
 
 // Metrics (max / mean density error, kinetic energy, non-finite and penetration counts).
 struct MetricsAccum {

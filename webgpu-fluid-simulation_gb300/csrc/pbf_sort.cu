@@ -623,19 +623,21 @@ __global__ void k_scatter_u32(uint32_t n, const uint32_t* __restrict__ id, const
 // list kernel has a neighbour's id at hand.
 __global__ void __launch_bounds__(256) k_ns_sorted(uint32_t n, const uint32_t* __restrict__ order,
                                                    const float4* __restrict__ pos, float4* __restrict__ sorted,
-                                                   uint32_t* __restrict__ scan, uint32_t scan_words) {
+                                                   uint32_t* __restrict__ scan, uint32_t scan_words,
+                                                   unsigned long long* total) {
   chain_begin(order, pos);
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   for (uint32_t i = t; i < scan_words; i += gridDim.x * blockDim.x) scan[i] = 0u;  // of the scan between the traversals
+  if (t == 0u) *total = 0ull;
   if (t >= n) return;
-  const uint32_t o = order[t];
+  const uint32_t o = min(order[t], n - 1u);  // (after a sort whose scan gave up, an entry may be unwritten)
   float4 x = __ldg(pos + o);
   x.w = __uint_as_float(o);
   sorted[t] = x;
 }
 
 // each(in, id): every candidate in order, in: whether it is a neighbour.  Four
-// loads in flight; the last group of a run repeats its last candidate.
+// loads in flight; the last, partial group of a run is taken one by one.
 template <class Each>
 __device__ __forceinline__ void test_cells27(const GridParams& g, const uint32_t* __restrict__ cell_start,
                                              const float4* __restrict__ sorted, f3 xi, float h2, Each&& each) {
@@ -660,35 +662,45 @@ __device__ __forceinline__ void test_cells27(const GridParams& g, const uint32_t
     }
 }
 
-// Counts by particle id; entry n receives 0, so a scan of n + 1 ends in the total.
+// Counts by particle id; entry n receives 0, so a scan of n + 1 ends in the
+// total modulo 2^32.  *total is the whole sum: 65,536 points within a radius
+// of each other already have 2^32 neighbours.
 __global__ void __launch_bounds__(128) k_ns_count(uint32_t n, GridParams g, float h2,
                                                   const float4* __restrict__ sorted,
                                                   const uint32_t* __restrict__ cell_start,
-                                                  uint32_t* __restrict__ count) {
+                                                  uint32_t* __restrict__ count, unsigned long long* total) {
   chain_begin(sorted, cell_start);
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t == n) count[n] = 0u;
-  if (t >= n) return;
-  const float4 x = sorted[t];
   uint32_t c = 0;
-  test_cells27(g, cell_start, sorted, xyz(x), h2, [&](bool in, uint32_t) { c += in ? 1u : 0u; });
-  count[__float_as_uint(x.w)] = c;
+  if (t < n) {
+    const float4 x = sorted[t];
+    test_cells27(g, cell_start, sorted, xyz(x), h2, [&](bool in, uint32_t) { c += in ? 1u : 0u; });
+    count[__float_as_uint(x.w)] = c;
+  }
+  const uint32_t lo = __reduce_add_sync(kFull, c & 0xffffu), hi = __reduce_add_sync(kFull, c >> 16);
+  if ((threadIdx.x & 31u) == 0u && t < n) atomicAdd(total, ((unsigned long long)hi << 16) + lo);
 }
 
-// The lists, written only if they all fit (offset[n] <= capacity).  A thread
+// The lists, written only if they all fit (*total <= capacity).  A thread
 // writes its particle's run as it finds it: the id arrives with the candidate.
+// Each run is tested against the capacity all the same: offsets are too small
+// after a scan that gave up.
 __global__ void __launch_bounds__(128) k_ns_list(uint32_t n, GridParams g, float h2,
                                                  const float4* __restrict__ sorted,
                                                  const uint32_t* __restrict__ cell_start,
+                                                 const uint32_t* __restrict__ count,
                                                  const uint32_t* __restrict__ offset, uint32_t* __restrict__ list,
-                                                 uint32_t capacity) {
-  chain_begin(sorted, cell_start, offset);
+                                                 uint32_t capacity, const unsigned long long* __restrict__ total) {
+  chain_begin(sorted, cell_start, count, offset, total);
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n || __ldg(offset + n) > capacity) return;
+  if (t >= n || *total > capacity) return;
   const float4 x = sorted[t];
-  uint32_t* out = list + __ldg(offset + __float_as_uint(x.w));
-  test_cells27(g, cell_start, sorted, xyz(x), h2, [&](bool in, uint32_t id) {
-    if (in) *out++ = id;
+  const uint32_t id = __float_as_uint(x.w), first = __ldg(offset + id);
+  if ((uint64_t)first + __ldg(count + id) > capacity) return;
+  uint32_t* out = list + first;
+  test_cells27(g, cell_start, sorted, xyz(x), h2, [&](bool in, uint32_t j) {
+    if (in) *out++ = j;
   });
 }
 
@@ -965,23 +977,24 @@ cudaError_t launch_scatter_by_id_u32(uint32_t n, const uint32_t* id, const uint3
   return cudaGetLastError();
 }
 cudaError_t launch_ns_count(uint32_t n, const GridParams& g, float h2, const uint32_t* order, const float4* pos,
-                            const uint32_t* cell_start, float4* sorted, uint32_t* count, uint32_t* offset, void* scan,
-                            uint32_t* err, cudaStream_t st) {
+                            const uint32_t* cell_start, float4* sorted, uint32_t* count, uint32_t* offset,
+                            unsigned long long* total, void* scan, uint32_t* err, cudaStream_t st) {
   const bool early = n <= kEarlyMax;
   const size_t m = (size_t)n + 1;
   cudaError_t e = launch_chain(early, k_ns_sorted, blocks_for(m, 256), 256, 0, st, n, order, pos, sorted,
-                               reinterpret_cast<uint32_t*>(scan), (uint32_t)(scan_scratch_bytes(m) / sizeof(uint32_t)));
+                               reinterpret_cast<uint32_t*>(scan), (uint32_t)(scan_scratch_bytes(m) / sizeof(uint32_t)),
+                               total);
   if (e != cudaSuccess) return e;
-  e = launch_chain(early, k_ns_count, blocks_for(m, 128), 128, 0, st, n, g, h2, sorted, cell_start, count);
+  e = launch_chain(early, k_ns_count, blocks_for(m, 128), 128, 0, st, n, g, h2, sorted, cell_start, count, total);
   if (e != cudaSuccess) return e;
   return launch_exclusive_scan_cleared(count, offset, m, scan, err, st, ScanExtra{}, early);
 }
 cudaError_t launch_ns_list(uint32_t n, const GridParams& g, float h2, const float4* sorted, const uint32_t* cell_start,
-                           const uint32_t* offset, uint32_t* list, uint32_t capacity, cudaStream_t st) {
+                           const uint32_t* count, const uint32_t* offset, const unsigned long long* total,
+                           uint32_t* list, uint32_t capacity, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  // an ordinary launch: the total is read back between the scan and this kernel
-  return launch_chain(false, k_ns_list, blocks_for(n, 128), 128, 0, st, n, g, h2, sorted,
-                      cell_start, offset, list, capacity);
+  return launch_chain(n <= kEarlyMax, k_ns_list, blocks_for(n, 128), 128, 0, st, n, g, h2, sorted, cell_start, count,
+                      offset, list, capacity, total);
 }
 cudaError_t launch_metrics(SimParams p, FieldParams f, const float* sdf, const float4* pos, const float4* vel,
                            const uint32_t* nbr_count, uint32_t n, float* accum_f, double* accum_d, uint32_t* accum_u,
