@@ -193,8 +193,7 @@ __device__ inline float splat_exp(float x) {
 
 __device__ inline uint32_t depth_bits(float d) { return __float_as_uint(d); }
 
-// Also clears the words of `zero` (the volume tiles' counts and the scan's
-// scratch).
+// Also clears the words of `zero` (the volume tiles' counts).
 __global__ void k_init(const float* scene, unsigned long long* keys, unsigned long long* acc, int W, int H, int W2,
                        int H2, uint32_t* zero, uint32_t words) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
@@ -376,6 +375,39 @@ __device__ inline void volume_fragments(const Sprite& s, uint32_t lane, Add add)
     const float fx = w <= 32 ? ex : gauss_axis(__fmaf_rn((float)i, s.sx, s.ox));
     add(i, j, fx * fy);
   });
+}
+
+// The tiles' first places: the exclusive scan of their counts by one CTA, which
+// waits on no other, so a place is always that of its count: a look-back scan
+// that gave up would leave entries of the order unwritten, which k_volume_sum
+// takes for tiles and particles.  One round up to 1,024 tiles (1920 x 1080 has
+// 920, 3840 x 2160 3,600); a frame of 2^20 particles takes 523 us at 1920 x 1080
+// and 2,179 at 3840 x 2160, 524 and 2,180 with the look-back scan.
+constexpr uint32_t kPlaceThreads = 1024;
+
+__global__ void __launch_bounds__(kPlaceThreads) k_volume_places(const uint32_t* __restrict__ count, uint32_t m,
+                                                                 uint32_t* __restrict__ place) {
+  __shared__ uint32_t s_warp[32];
+  const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+  pbf::chain_begin(count);
+  uint32_t before = 0u;
+  for (uint32_t b = 0; b < m; b += kPlaceThreads) {
+    const uint32_t t = b + threadIdx.x, v = t < m ? count[t] : 0u;
+    uint32_t x = v;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31u) s_warp[wib] = x;
+    __syncthreads();
+    uint32_t w = s_warp[lane];
+    const uint32_t total = __reduce_add_sync(0xffffffffu, w);
+    const uint32_t mine = __reduce_add_sync(0xffffffffu, lane < wib ? w : 0u);
+    if (t < m) place[t] = before + mine + x - v;
+    before += total;
+    __syncthreads();
+  }
 }
 
 // Particles in tile order (any order within a tile): place[t] is the tile's
@@ -715,7 +747,7 @@ struct pbf_renderer {
   unsigned long long* acc = nullptr;
   uint32_t* tile_min = nullptr;
   // volume sprites by tile, for up to vol_cap particles: tile and rank in it
-  // per particle, order, then counts, places and the scan's scratch
+  // per particle, order, then the tiles' counts and places
   uint32_t vol_cap = 0;
   uint2* vol_tile = nullptr;
   uint2* vol_order = nullptr;
@@ -772,15 +804,11 @@ size_t volume_tiles(const pbf_renderer* r) {
   return (size_t)((r->W2 + kVolTile - 1) / kVolTile) * ((r->H2 + kVolTile - 1) / kVolTile);
 }
 
-// Workspace for n particles (16 bytes each; kept, grown as needed) and, per
-// renderer, the words that k_init clears: the tiles' counts, the scan's error
-// word, the tiles' places and the scan's scratch.
-size_t volume_places_at(const pbf_renderer* r) { return volume_tiles(r) + 2; }
-size_t volume_scratch_at(const pbf_renderer* r) { return (volume_places_at(r) + volume_tiles(r) + 1 + 63) / 64 * 64; }
-size_t volume_words(const pbf_renderer* r) {
-  return volume_scratch_at(r) + (pbf::scan_scratch_bytes(volume_tiles(r) + 1) + 3) / 4;
-}
+// Words per renderer: the tiles' counts and a 0 after them, which k_init clears,
+// then the places of both.
+size_t volume_words(const pbf_renderer* r) { return 2 * (volume_tiles(r) + 1); }
 
+// Workspace for n particles (16 bytes each; kept, grown as needed).
 cudaError_t volume_workspace(pbf_renderer* r, uint32_t n, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   if (!r->vol_count && (e = cudaMalloc(&r->vol_count, volume_words(r) * sizeof(uint32_t))) != cudaSuccess) return e;
@@ -801,11 +829,9 @@ cudaError_t volume_workspace(pbf_renderer* r, uint32_t n, cudaStream_t st) {
 // The volume sprites summed by tile, once the splat has found their tiles.
 cudaError_t volume_by_tile(pbf_renderer* r, const Cam& C, const float4* pos, uint32_t n, float R, cudaStream_t st) {
   const size_t m = volume_tiles(r) + 1;
-  uint32_t *err = r->vol_count + m, *place = r->vol_count + volume_places_at(r);
-  uint32_t* scratch = r->vol_count + volume_scratch_at(r);
-  cudaError_t e =
-      pbf::launch_exclusive_scan_cleared(r->vol_count, place, m, scratch, err, st, pbf::ScanExtra{}, true);
-  // (entry m - 1 of the counts is 0: its place is the total and stays it)
+  uint32_t* place = r->vol_count + m;
+  // (entry m - 1 of the counts is 0: its place is the total)
+  cudaError_t e = pbf::launch_chain(true, k_volume_places, 1, kPlaceThreads, 0, st, r->vol_count, (uint32_t)m, place);
   if (e == cudaSuccess)
     e = pbf::launch_chain(true, k_volume_order, (n - 1u) / 256u + 1u, 256, 0, st, n, r->vol_tile, place, r->vol_order);
   if (e == cudaSuccess)
@@ -909,7 +935,7 @@ int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_s
     tiled = false;
   }
   k_init<<<rows, 256, 0, st>>>(d_scene_depth, r->keys, r->acc, r->W, r->H, r->W2, r->H2, r->vol_count,
-                               tiled ? (uint32_t)volume_words(r) : 0u);
+                               tiled ? (uint32_t)volume_tiles(r) + 1u : 0u);
   cudaError_t e = cudaSuccess;
   if (n) {
     int sms = 0, dev = 0;
