@@ -40,7 +40,7 @@
 // Many particles on a large map are drawn in two phases: a share of the depth
 // sprites, then everything else behind a depth test per 8 x 8 tile, with the
 // small volume sprites sorted by tile and summed in shared memory.  Fewer are
-// drawn at once, 1 to 16 of them a warp.  Neither changes a bit of the result.
+// drawn at once, 1 to 32 of them a warp.  Neither changes a bit of the result.
 //
 // The filter is the reference's narrow-range filter, separable, x then y,
 // with its sample window of 32 + 32 texels per 32-texel block: the centre it
@@ -255,21 +255,36 @@ constexpr int kTile = 8;
 constexpr uint32_t kFirstShare = 16;
 // The two phases and the volume sums by tile pay for their five extra launches
 // (about 25 us) and for the particles' second reading where there are many
-// particles, or fewer with sprites of many pixels.  A frame, all at once (with 8
-// or 16 particles a warp) and tiled:
-//              320 x 180   960 x 540   1280 x 720   1600 x 900   1920 x 1080
-//   1,048,576  290  250    356  289    445  332     579  409     789  524
-//     700,000  207  187    260  225    321  260     466  324     567  420
-//     524,288  166  178    215  224    266  268     344  327     466  431
-//     393,216  147  139    174  172    211  204     286  259     355  335
-//     262,144  112  126    149  194    186  249     242  320     321  429
-// (Powers of two are the worst for the first share here: the particles lie in
-// index order on a lattice, and every 16th block falls on the same lines.)
-constexpr uint32_t kTiledAlways = 5u << 17;
+// fragments and many of them to a pixel: the square root of their product,
+// particles times side^2 over the square root of the map's pixels, tells best
+// where.  Sprites of 25 pixels and more are too large to be summed by tile.  A
+// frame, all at once and tiled (us, both with the best number of particles a
+// warp):
+//   n          side  map          fill   all  tiled
+//     500,000   1.6  1920 x 1080    931   184   215
+//   1,048,576   1.6  1920 x 1080  1,953   299   332
+//     700,000   1.4   320 x 180   5,433   193   189
+//     900,000   2.7  1280 x 720   6,985   263   293
+//     524,288   2.7   640 x 360   8,138   168   193
+//     700,000   4.1  1920 x 1080  8,149   277   275
+//     400,000   8.2  3840 x 2160  9,313   461   458
+//     700,000   2.6   640 x 339   9,930   208   195
+//     900,000   4.1  1920 x 1080 10,477   342   366
+//     500,000   4.1   960 x 540  11,641   222   203
+//   1,048,576   4.1  1920 x 1080 12,207   371   340
+//     400,000   5.5  1280 x 720  12,417   207   204
+//     500,000   8.2  1920 x 1080 23,282   481   387
+//   1,048,576   8.2  1920 x 1080 48,826   792   530
+//     620,000  16.4  3840 x 2160 57,740 1,567 1,363
+//     620,000  32.8  1920 x 1080          7,135 7,363
+// (Powers of two are worst for the first share in these clouds: the particles
+// lie in index order on a lattice, and every 16th block falls on the same lines.)
+// Below kTiledMin the first share is too small: 2^18 particles at 1920 x 1080
+// with sides of 8.2 took 321 at once and 429 tiled.
 constexpr uint32_t kTiledMin = 3u << 17;
-constexpr uint64_t kTiledWork = 1ull << 39;  // particles times pixels
-inline bool takes_tiles(uint32_t n, int W, int H) {
-  return n >= kTiledAlways || (n >= kTiledMin && (uint64_t)W * H * n >= kTiledWork);
+constexpr double kTiledFill = 9.5e3, kTiledSide = 25.0;
+inline bool takes_tiles(uint32_t n, double side, int W, int H) {
+  return n >= kTiledMin && side < kTiledSide && n * side * side >= kTiledFill * std::sqrt((double)W * H);
 }
 constexpr int kMaxTiles = 16;                // larger sprites are not tested
 
@@ -289,8 +304,6 @@ __global__ void __launch_bounds__(256) k_tile_min(const unsigned long long* __re
   m = __reduce_min_sync(0xffffffffu, m);
   if (lane == 0) tile_min[tile] = m;
 }
-
-constexpr uint64_t kSmallMap = 3u << 17;  // pixels (768 x 512)
 
 // Whether a depth sprite may win a pixel in any of its tiles.
 __device__ inline bool may_win(const Sprite& s, const uint32_t* __restrict__ tile_min, int tw) {
@@ -800,6 +813,14 @@ cudaError_t launch_filter(const Gauss& gauss, float* img, float* temp, int W, in
                            dim3(32, 8), 0, st, gauss, temp, img, W, H, rows, half, R * 5.0f, R);
 }
 
+// Pixels across a particle's sprites, the same number on both maps, if it is as
+// far from the camera as the world's origin (the reference's camera looks at
+// it): what the splat's division of the work goes by.
+double sprite_side(const Cam& C, double R, int H) {
+  const double x = C.v[12], y = C.v[13], z = C.v[14];
+  return R * std::fabs((double)C.p[5]) * H / (2.0 * std::max(std::sqrt(x * x + y * y + z * z), R));
+}
+
 size_t volume_tiles(const pbf_renderer* r) {
   return (size_t)((r->W2 + kVolTile - 1) / kVolTile) * ((r->H2 + kVolTile - 1) / kVolTile);
 }
@@ -929,7 +950,8 @@ int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_s
   const float4* pos = (const float4*)d_positions;
   cudaEventRecord(r->ev[0], st);
   const dim3 rows((unsigned)((r->W + 255) / 256), (unsigned)r->H);
-  bool tiled = takes_tiles(n, r->W, r->H);
+  const double side = sprite_side(C, R, r->H);
+  bool tiled = takes_tiles(n, side, r->W, r->H);
   if (tiled && volume_workspace(r, n, st) != cudaSuccess) {
     cudaGetLastError();  // without the workspace, everything is drawn at once
     tiled = false;
@@ -945,18 +967,24 @@ int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_s
     auto splat = [&](int phase, uint64_t particles) {
       // Few particles are spread over the device, as a warp walks its own one
       // after another (8000 at 1920 x 1080, a frame: 32 a warp 219 us, 2 a warp
-      // 73); many are taken in blocks that set their sprites up with most lanes,
-      // more of them where the sprites are small (320 x 180: 300,000 with 8 a warp
-      // 120 us, with 32 112; 450,000 161 and 146).  On large maps finer is also
-      // more even: 2^18 at 1920 x 1080 433 us with 32, 321 with 8.
-      const uint64_t pixels = (uint64_t)r->W * r->H;
-      const uint32_t sixteen = pixels < kSmallMap ? 150000u : 400000u;  // particles from which a warp takes 16
-      uint32_t per = pixels < kSmallMap && n >= 300000u ? 32 : n >= sixteen ? 16 : 8;
-      if (phase != kAll) per = phase == kRest ? 32 : 4;
-      while (phase == kAll && per > 1 && particles < (uint64_t)sms * 32 * per) per /= 2;
+      // 73).  Many with small sprites are taken in blocks that set their sprites
+      // up with most lanes, with large ones fewer, which is more even (us with
+      // 8 / 16 / 32 a warp, at once: 400,000 with sides of 1.6 175 / 165 / 170,
+      // 700,000 251 / 231 / 225, 380,000 with 4.1 197 / 191 / 201, 400,000 with
+      // 32.8 4,783 / 5,097 / 5,916; the rest of the tiled path: 400,000 with 8.2
+      // 331 / 325 / 341, 1,048,576 580 / 540 / 530, 620,000 with 16.4 at 3840 x
+      // 2160 1,363 / 1,400 / 1,535).
+      uint32_t per = 4;  // the first share
+      if (phase == kAll) {
+        per = side < 4.0 && n >= 300000u ? 32 : side < 5.7 && n >= 150000u ? 16 : 8;
+        while (per > 1 && particles < (uint64_t)sms * 32 * per) per /= 2;
+      } else if (phase == kRest) {
+        per = side >= 10.5 ? 8 : side >= 6.5 && n < 800000u ? 16 : 32;
+      }
       const uint64_t warps = (particles + per - 1) / per;
-      // on maps below 2^19 pixels most sprites are a step or two: reading ahead cost 2 to 4 % there
-      auto kernel = phase == kAll && pixels < (1u << 19) ? k_splat<false> : k_splat<true>;
+      // sprites of a step or two have no keys to read ahead (620,000 with sides
+      // of 1.6: 211 us without, 217 with; 380,000 with 8.2: 371 and 355)
+      auto kernel = phase == kAll && side < 5.0 ? k_splat<false> : k_splat<true>;
       return pbf::launch_chain(true, kernel, (unsigned)((warps + 7) / 8), 256, 0, st, C, pos, n, R, r->W,
                                r->H, r->W2, r->H2, r->keys, r->acc, phase, per, r->tile_min, tw, r->vol_tile,
                                r->vol_count);
