@@ -633,7 +633,11 @@ int pbf_renderer_set_config(pbf_renderer* r, const pbf_render_options* options);
 int pbf_renderer_set_camera(pbf_renderer* r, const pbf_camera* camera);
 /* Rasterize + filter for n particles at d_positions (device float4, xyz
  * used).  d_scene_depth: NULL (a cleared depth buffer, all 0) or a device
- * float [W*H] reverse-Z depth buffer, read and updated in place. */
+ * float [W*H] reverse-Z depth buffer, read and updated in place.  From 393,216
+ * particles on, frames of many fragments use a workspace of up to 24 bytes a
+ * particle, allocated when first needed, grown by half as much again and kept
+ * until the renderer is destroyed; a frame for which it cannot be had is drawn
+ * without it. */
 int pbf_render(pbf_renderer* r, const float* d_positions, uint32_t n, float* d_scene_depth, void* stream);
 /* TextureFilter.execute (textureFilter.ts:129-160) on any device r32float
  * image of width x height, in place, with options->filter_size and

@@ -763,7 +763,7 @@ struct pbf_renderer {
   // per particle, order, then the tiles' counts and places
   uint32_t vol_cap = 0;
   uint2* vol_tile = nullptr;
-  uint2* vol_order = nullptr;
+  uint2* vol_order = nullptr;  // behind vol_tile's in one allocation
   uint32_t* vol_count = nullptr;
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   float ms[2] = {0.0f, 0.0f};
@@ -779,7 +779,6 @@ void release(pbf_renderer* r) {
   cudaFree(r->acc);
   cudaFree(r->tile_min);
   cudaFree(r->vol_tile);
-  cudaFree(r->vol_order);
   cudaFree(r->vol_count);
   for (auto& e : r->ev)
     if (e) cudaEventDestroy(e);
@@ -829,22 +828,27 @@ size_t volume_tiles(const pbf_renderer* r) {
 // then the places of both.
 size_t volume_words(const pbf_renderer* r) { return 2 * (volume_tiles(r) + 1); }
 
-// Workspace for n particles (16 bytes each; kept, grown as needed).
+// Workspace for n particles (16 bytes each), kept and grown by half as much
+// again, so that a scene that emits particles allocates a few times and not on
+// every frame.
 cudaError_t volume_workspace(pbf_renderer* r, uint32_t n, cudaStream_t st) {
-  cudaError_t e = cudaSuccess;
-  if (!r->vol_count && (e = cudaMalloc(&r->vol_count, volume_words(r) * sizeof(uint32_t))) != cudaSuccess) return e;
-  if (n > r->vol_cap) {
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-    cudaFree(r->vol_tile);
-    cudaFree(r->vol_order);
-    r->vol_tile = nullptr;
-    r->vol_order = nullptr;
-    r->vol_cap = 0;
-    e = cudaMalloc(&r->vol_tile, (size_t)n * sizeof(uint2));
-    if (e == cudaSuccess) e = cudaMalloc(&r->vol_order, (size_t)n * sizeof(uint2));
-    if (e == cudaSuccess) r->vol_cap = n;
+  if (n <= r->vol_cap) return cudaSuccess;
+  cudaError_t e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return e;
+  cudaFree(r->vol_tile);
+  r->vol_tile = nullptr;
+  r->vol_cap = 0;
+  uint32_t cap = (uint32_t)std::min<uint64_t>((uint64_t)n + n / 2, 0xfffffffeu);
+  e = cudaMalloc(&r->vol_tile, 2 * (size_t)cap * sizeof(uint2));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    cap = n;
+    e = cudaMalloc(&r->vol_tile, 2 * (size_t)cap * sizeof(uint2));
   }
-  return e;
+  if (e != cudaSuccess) return e;
+  r->vol_order = r->vol_tile + cap;
+  r->vol_cap = cap;
+  return cudaSuccess;
 }
 
 // The volume sprites summed by tile, once the splat has found their tiles.
@@ -897,6 +901,7 @@ int pbf_renderer_create(uint32_t width, uint32_t height, pbf_renderer** out) {
   if (e == cudaSuccess) e = cudaMalloc(&r->acc, px2 * sizeof(unsigned long long));
   if (e == cudaSuccess)
     e = cudaMalloc(&r->tile_min, (size_t)((width + kTile - 1) / kTile) * ((height + kTile - 1) / kTile) * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMalloc(&r->vol_count, volume_words(r) * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(r->depth, 0, px * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(r->volume, 0, px2 * sizeof(float));
   for (auto& ev : r->ev)
