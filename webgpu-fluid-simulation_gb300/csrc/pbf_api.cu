@@ -2488,7 +2488,7 @@ struct pbf_ns {
   cudaStream_t stream;
   bool own_stream;
   std::string err;
-  DBuf<uint32_t> key, rank, cell_count, cell_start, perm_raw, id_raw, perm, tmp_a, tmp_b, big_list, big_count;
+  DBuf<uint32_t> key, rank, cell_count, cell_start, perm_raw, id_raw, perm, tmp_a, tmp_b;
   DBuf<uint32_t> err_word;   // NsStatus
   DBuf<uint32_t> nbr_count;  // by particle id (pbf_ns_lists)
   DBuf<float4> sorted;       // pbf_ns_lists: positions in sorted order, the id in w
@@ -2555,8 +2555,6 @@ int pbf_ns_create(const pbf_grid* grid, uint32_t max_particles, void* stream, pb
   A(s->tmp_b.alloc(n));
   A(s->cell_count.alloc(cells + 1));
   A(s->cell_start.alloc(cells + 1));
-  A(s->big_list.alloc(cells));
-  A(s->big_count.alloc(1));
   A(s->err_word.alloc(sizeof(NsStatus) / sizeof(uint32_t)));
   A(s->nbr_count.alloc(n + 1));
   size_t sb = scan_scratch_bytes(cells + 1), sb2 = scan_scratch_bytes(n + 1);
@@ -2578,7 +2576,7 @@ int pbf_ns_destroy(pbf_ns* s) {
   if (!s) return PBF_EINVAL;
   if (s->stream) cudaStreamSynchronize(s->stream);
   DBuf<uint32_t>* bufs[] = {&s->key,   &s->rank,  &s->cell_count, &s->cell_start, &s->perm_raw, &s->id_raw, &s->perm,
-                            &s->tmp_a, &s->tmp_b, &s->big_list,   &s->big_count,  &s->err_word, &s->nbr_count};
+                            &s->tmp_a, &s->tmp_b, &s->err_word,   &s->nbr_count};
   for (auto* b : bufs) b->release();
   s->sorted.release();
   if (s->scan_scratch) cudaFree(s->scan_scratch);

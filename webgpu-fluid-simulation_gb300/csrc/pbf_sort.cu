@@ -785,16 +785,17 @@ namespace {
 size_t round256(size_t b) { return (b + 255) / 256 * 256; }
 }  // namespace
 
-// Scratch: the digit-major count matrix, its scan and one scan scratch per
-// pass; or, with few tiles, one count matrix per pass.
+// Scratch for up to n points: the digit-major count matrix, its scan and one
+// scan scratch per pass; or, for so few points that the tiles are few, one
+// count matrix per pass.
 constexpr int kMaxPasses = 4;
 size_t radix_scratch_bytes(size_t n) {
   size_t tiles = (n + kOsTile - 1) / kOsTile;
   if (tiles == 0) tiles = 1;
   const size_t m = tiles * kOsMaxRadix;
   const size_t many = 2 * round256(m * sizeof(uint32_t)) + kMaxPasses * round256(scan_scratch_bytes(m));
-  const size_t few = kMaxPasses * (size_t)kFewTiles * kOsMaxRadix * sizeof(uint32_t);
-  return many > few ? many : few;
+  const size_t few = kMaxPasses * std::min(tiles, (size_t)kFewTiles) * kOsMaxRadix * sizeof(uint32_t);
+  return tiles > kFewTiles ? std::max(many, few) : few;
 }
 
 namespace {
