@@ -127,6 +127,19 @@ def test_predicted_positions_after_a_replay(first, then):
         same(got, state(sim))
 
 
+def test_recorded_on_the_handles_own_stream():
+    """The caller records the stream that the handle made and handed out."""
+    with simulator(L.FP_EXACT, 2, None) as sim:
+        sim.step(1)
+        stream = torch.cuda.ExternalStream(sim.stream)
+        g = recorded(stream, lambda: sim.step(1))
+        sim.run()
+        sim.run()
+        replay(stream, g)
+        sim.step(1)
+        same(state(sim), plain(L.FP_EXACT, 2, 4))
+
+
 def test_first_captured_frame_is_refused_under_the_callers_capture():
     """A handle with no captured frame yet cannot capture one inside the
     caller's capture; the capture and the handle stay usable."""

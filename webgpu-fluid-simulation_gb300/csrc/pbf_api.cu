@@ -81,6 +81,9 @@ struct pbf_handle {
   // the last substep before) and leaves its x* in one fixed buffer.
   bool caller_graph = false;
   bool own_capture = false;  // the capture under way on the stream is capture_frame's
+  // The stream is the caller's, or the caller has asked for it: only then can it
+  // be under the caller's capture (asking the runtime costs a substep 0.5 us).
+  bool stream_known = false;
   DBuf<uint32_t> nbr_count, nbr_max, nbr_list;
   DBuf<uint32_t> band_list[2], band_count;  // boundary band lists (ping-pong) and their lengths
   // cell-block passes (PBF_BUILD_CELLBLOCK_*): cell key and x*_0 per sorted
@@ -395,7 +398,7 @@ void invalidate_graph(pbf_handle* h) {
 
 // Whether a caller is recording the handle's stream into a graph of its own.
 bool caller_captures(const pbf_handle* h) {
-  if (h->own_capture) return false;
+  if (h->own_capture || !h->stream_known) return false;
   cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(h->stream, &s) != cudaSuccess) {
     cudaGetLastError();  // the legacy stream beside another one's capture: the launches report it
@@ -1296,6 +1299,7 @@ int pbf_create(const pbf_config* cfg, pbf_handle** out) {
   cudaError_t e = cudaSuccess;
   if (cfg->stream) {
     h->stream = (cudaStream_t)cfg->stream;
+    h->stream_known = true;
   } else {
     e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     h->own_stream = true;
@@ -2015,7 +2019,11 @@ const float* pbf_velocity_device(pbf_handle* h) {
   if (launch_scatter_by_id(h->n, h->ids[h->cur].p, h->vel.p, h->out_tmp.p, h->stream) != cudaSuccess) return nullptr;
   return (const float*)h->out_tmp.p;
 }
-void* pbf_stream(pbf_handle* h) { return h ? (void*)h->stream : nullptr; }
+void* pbf_stream(pbf_handle* h) {
+  if (!h) return nullptr;
+  h->stream_known = true;
+  return (void*)h->stream;
+}
 
 // The frame's by-id positions are copied device to device into a staging
 // buffer on a second stream, then from there to the host on that stream, so
