@@ -43,10 +43,9 @@ __device__ __forceinline__ float4 f4(f3 v, float w) { return make_float4(v.x, v.
 // pointers given are those the kernel reads through const __restrict__ or
 // __ldg: passing them through the asm statement keeps the compiler from moving
 // loads it takes for invariant ahead of the wait.  Plain loads stay behind it by
-// themselves, so the members of a struct argument that are read that way are
-// not given: the kernel would keep a copy of the struct on its stack (delta-p
-// of 16 batched scenes: 88 bytes a thread and 54.0 us, 32 and 52.1 without).
-// No kernel asks for its
+// themselves; giving delta-p the members of its struct argument, which it reads
+// that way, made it keep a copy of the struct on its stack (16 batched scenes:
+// 88 bytes a thread and 54.0 us, 32 and 52.1 without).  No kernel asks for its
 // successor early: CTAs that wait hold slots which other streams could use
 // (16,384 particles, three handles: 119 us per frame without, 127 to 159 with).
 template <class P>

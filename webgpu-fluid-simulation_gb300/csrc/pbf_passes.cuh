@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256) k_nbr_build_feat(SimParams p, GridParams 
                                                         uint32_t* __restrict__ nbr_count, uint32_t* max_seen,
                                                         uint32_t* err, int have_field,
                                                         const float4* __restrict__ bdata, SolverAux a) {
-  chain_begin(xs, cell_start, bdata);
+  chain_begin(xs, cell_start, bdata, a.pos, a.lam_prev, a.bsdf);
   PBF_TILES(p.n) {
     const uint32_t t = tile0 + threadIdx.x;
     if (t < p.n) {
@@ -1011,7 +1011,7 @@ __global__ void __launch_bounds__(256) k_lambda(SimParams p, int have_field, con
                                                 const uint32_t* __restrict__ nbr_cnt,
                                                 const uint32_t* __restrict__ nbr_list,
                                                 float4* __restrict__ xl, SolverAux a) {
-  chain_begin(bdata, xs, nbr_cnt, nbr_list);
+  chain_begin(bdata, xs, nbr_cnt, nbr_list, a.guard, a.pos, a.lam_prev, a.bsdf, a.lam_sum);
   if (a.guard && *a.guard == 0) return;
   // kMode 2: also the density error at these positions into a.stats (the
   // adaptive iteration's test; the same quantity AttributeUpdate reports)
@@ -1130,7 +1130,7 @@ __global__ void __launch_bounds__(256) k_density_velocity(SimParams p, SolverAux
                                                           const uint32_t* __restrict__ nbr_cnt,
                                                           const uint32_t* __restrict__ nbr_list,
                                                           float4* __restrict__ pos, float4* __restrict__ vel) {
-  chain_begin(xs, nbr_cnt, nbr_list);
+  chain_begin(xs, nbr_cnt, nbr_list, a.guard);
   if (a.guard && *a.guard == 0) return;
   unsigned cmax = 0u, csum = 0u, ccnt = 0u;
   PBF_SLOTS(t, p.n) {
@@ -1334,7 +1334,7 @@ __global__ void __launch_bounds__(256) k_lambda_lanes(SimParams p, int have_fiel
                                                       const uint32_t* __restrict__ nbr_cnt,
                                                       const uint32_t* __restrict__ nbr_list, float4* __restrict__ xl,
                                                       SolverAux a) {
-  chain_begin(bdata, xs, nbr_cnt, nbr_list);
+  chain_begin(bdata, xs, nbr_cnt, nbr_list, a.lam_sum);
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, t = g / kL;
   if (t >= p.n) return;
   uint32_t b, e;
