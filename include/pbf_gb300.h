@@ -324,6 +324,11 @@ typedef enum pbf_search_array {
 int pbf_copy_search_state(pbf_handle* h, int which, uint32_t* host, size_t count);
 /* Keep per-iteration debug fields (PBF_FIELD_DELTA_P); off by default. */
 int pbf_set_capture(pbf_handle* h, int enable);
+/* The handle's stream.  A caller may have it under a capture of its own and
+ * record pbf_run and pbf_step into a graph (whole pairs of substeps: a substep
+ * leaves the state in the other buffers); replays and further steps may follow
+ * in any order.  From the first recorded substep on every substep of the handle
+ * clears its cell counts itself. */
 void* pbf_stream(pbf_handle* h);
 
 /* ---- neighbour search alone: NeighborSearch.execute (src/simulator/neighbor/neighborSearch.ts:270-301).
@@ -350,7 +355,8 @@ int pbf_ns_run(pbf_ns* ns, const float* d_pos4, uint32_t n, uint32_t* d_keys,
  * Fails with PBF_ECAPACITY (writing no list) if the lists need more than
  * `capacity` entries; *total receives the needed size, 0xffffffff if it is
  * larger.  PBF_ETIMEOUT: a scan of this call or of the searches before it gave
- * up its bounded wait, the lists are not valid. */
+ * up its bounded wait, the lists are not valid.  The first call allocates 16
+ * bytes a particle of max_particles, which stay with the context. */
 int pbf_ns_lists(pbf_ns* ns, const float* d_pos4, uint32_t n, float radius,
                  uint32_t* d_nbr_offset, uint32_t* d_nbr_list, uint32_t capacity,
                  uint32_t* total);

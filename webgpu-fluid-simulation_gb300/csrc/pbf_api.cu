@@ -362,7 +362,11 @@ CbArgs cb_args(const pbf_handle* h) {
 // took 2436 us per frame, 1527 us with the small split asked for (14 %: 32 KB;
 // 0, 7 and 28 % measure the same, 44 % is 6 % slower), one handle alone 1663
 // us either way.  The density pass keeps the default: it has a little shared
-// memory of its own and any request slows it down (73 -> 160 us).
+// memory of its own and any request slows it down (73 -> 160 us).  The passes
+// with several lanes a slot gain nothing (an exact scene of 27,000 slots beside
+// two learned-start handles of 2^20: 3,860 us a round either way), the cell-block
+// passes stage records in shared memory and take the split that this needs, and
+// the fallback kernel returns at once in nearly every substep.
 void prefer_l1(const PassSet& ps) {
   for (const void* k :
        {(const void*)ps.predict, (const void*)ps.nbr_build, (const void*)ps.nbr_build2, (const void*)ps.nbr_build_warp,

@@ -30,10 +30,11 @@ cudaError_t launch_chain(bool early, void (*kernel)(P...), dim3 grid, dim3 block
   c.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
-// Slots up to which the step's kernels are launched early.  The gap saved is
-// about a microsecond per kernel: a substep at 68,921 slots goes from 240 to
-// 203 us (exact mode 514 to 447, 2,197 slots 136 to 94); at 2^20 slots it is
-// within the noise (2215, 2208), and 16 batched scenes got 1 % slower.
+// Slots up to which the step's kernels are launched early.  A frame of one
+// graph-replayed substep of 4 iterations, with and without: 2,197 slots 58.5 and
+// 62.7 us (exact mode 82 and 86), 27,000 exact 205 and 209, 68,921 148 and 153
+// (exact 429 and 433), 220,000 667 and 674; at 2^20 slots it is within the noise
+// (2215, 2208), and 16 batched scenes got 1 % slower.
 constexpr uint32_t kEarlyMax = 1u << 18;
 
 // The neighbour passes with several lanes a slot, for small scenes.

@@ -1032,7 +1032,7 @@ int pbf_texture_filter(const pbf_render_options* o, float* d_texture, uint32_t w
   if (cudaMallocAsync(&temp, (size_t)width * height * sizeof(float), st) != cudaSuccess) return PBF_ECUDA;
   cudaError_t e = launch_filter(g, d_texture, temp, (int)width, (int)height, o->filter_size, o->particle_radius, st);
   cudaFreeAsync(temp, st);
-  // the weights table is read from a host array by an asynchronous copy
+  // the texture is filtered when the call returns
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return e == cudaSuccess ? PBF_OK : PBF_ECUDA;
 }
