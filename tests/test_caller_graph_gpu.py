@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from pbf_gb300 import _lib as L
-from pbf_gb300 import PBF, scenes
+from pbf_gb300 import PBF, PBFBatch, mlp_init, scenes
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -138,6 +138,52 @@ def test_recorded_on_the_handles_own_stream():
         replay(stream, g)
         sim.step(1)
         same(state(sim), plain(L.FP_EXACT, 2, 4))
+
+
+@pytest.mark.parametrize("kind", ["learned", "batch", "field", "cellblock"])
+def test_recorded_frames_of_other_routes(kind):
+    """The learned start (side stream and fallback in the recorded graph), 16
+    small scenes in one batch, a volume map and the cell-block passes."""
+
+    def make(stream):
+        if kind == "batch":
+            cfg, sc, fa = scenes.batch_scenes_spec(count=16, n_min=300, n_max=900, seed=3, field_res=(8, 8, 8))
+            cfg, sc = scenes.build_batch((cfg, sc, fa), quadrature=4)
+            cfg.stream = stream.cuda_stream if stream is not None else None
+            return PBFBatch(cfg, sc)
+        if kind == "cellblock":
+            sim = simulator(L.FP_FAST, 2, stream)
+            sim.set_launch(build=L.BUILD_CELLBLOCK_MASK)
+            return sim
+        sc = scenes.reference_scene("boundary_small")
+        cfg = scenes.copy_config(sc.config)
+        cfg.fp_mode, cfg.substeps = L.FP_FAST, 2
+        cfg.stream = stream.cuda_stream if stream is not None else None
+        sim = PBF(cfg)
+        sim.set_particles(sc.particles)
+        f = sc.field
+        sim.set_boundary_field(f["res"], f["origin"], f["extent"], f["sdf"], f["vol"])
+        if kind == "learned":
+            sim.set_learned(mlp_init(3), iterations=1, fallback_bound=0.02)
+        return sim
+
+    def bits(sim):
+        sim.synchronize()
+        return [np.asarray(sim.copy_field(f)).view(np.uint32) for f in FIELDS]
+
+    stream = torch.cuda.Stream()
+    with make(stream) as sim:
+        g = recorded(stream, lambda: sim.step(1))
+        sim.step(1)
+        replay(stream, g)
+        replay(stream, g)
+        sim.enable_graph(True)
+        sim.step(2)
+        replay(stream, g)
+        got = bits(sim)
+    with make(None) as sim:
+        sim.step(6)
+        same(got, bits(sim))
 
 
 def test_first_captured_frame_is_refused_under_the_callers_capture():
